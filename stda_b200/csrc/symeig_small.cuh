@@ -5,9 +5,9 @@
 //      T = Q^T A Q (LAPACK dsytd2, lower, restated) by a cluster of 4 or 8
 //      CTAs with one cluster barrier per reflector (the scheme is described
 //      at the kernel); d, e, tau and the reflectors go to a global workspace;
-//   2. k_symeig_values (one warp per eigenvalue, any number of CTAs): bisection
-//      on Sturm counts (LAPACK dstebz's principle), each lane evaluating the
-//      count at one of 32 points of the current interval per round;
+//   2. k_symeig_values (one CTA per eigenvalue): multisection on Sturm counts
+//      (LAPACK dstebz's principle), each thread evaluating the count at one of
+//      256 points of the current interval per round;
 //   3. k_symeig_vectors (one warp per cluster of close eigenvalues, its work
 //      arrays in shared memory): inverse iteration with a pivoted tridiagonal
 //      LU (LAPACK dstein's scheme: shifts of equal eigenvalues nudged apart,
@@ -63,37 +63,64 @@ __device__ double symeig_block_sum(double v, double *red) {
   return t;
 }
 
-// number of eigenvalues of T (d, e2 = e^2) below x (Sturm sequence)
-__device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x,
-                                           double pivmin) {
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int cnt = q < 0.0;
-  for (int i = 1; i < n; ++i) {
-    q = d[i] - x - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    cnt += q < 0.0;
+// Number of eigenvalues below x of the scaled T: the sign changes of the
+// leading principal minors p_i of T - x I,
+//   p_{i+1} = (d_i - x) p_i - e_{i-1}^2 p_{i-1},
+// with db[i] = {d_i, e_{i-1}^2}.  Dividing the recurrence by p_i gives the
+// usual Sturm quotients, but puts an FP64 division on the serial chain; here
+// the chain is one fused multiply-add per step.  |d - x| <= 2 and e^2 <= 1
+// (scaled), so a step grows max(|p_i|, |p_{i-1}|) at most threefold, and e^2
+// is kept >= kE2Min, so that 8 steps shrink it by at most 2^-800 and two
+// consecutive minors never vanish: the pair is rescaled by a power of two
+// every 8 steps.  A minor that is exactly zero counts once whatever the sign
+// of the zero, since the next one then has the sign opposite to the last.
+constexpr double kE2Min = 6.223015277861142e-61;   // 2^-200
+__device__ __forceinline__ int sturm_count(const double2 *db, int n, double x) {
+  double pm = 1.0, p = db[0].x - x;
+  int neg = __double2hiint(p), cnt = (unsigned)neg >> 31;
+  auto step = [&](double2 v) {
+    const double t = fma(v.x - x, p, -(v.y * pm));
+    pm = p;
+    p = t;
+    const int h = __double2hiint(t);
+    cnt += (unsigned)(h ^ neg) >> 31;
+    neg = h;
+  };
+  int i = 1;
+  for (; i + 8 <= n; i += 8) {
+    double2 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = db[i + u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) step(v[u]);
+    const int ex = max(__double2hiint(p) & 0x7fffffff, __double2hiint(pm) & 0x7fffffff) >> 20;
+    const double sc = __hiloint2double(min(max(2046 - ex, 1), 2046) << 20, 0);
+    p *= sc;
+    pm *= sc;
   }
+  for (; i < n; ++i) step(db[i]);
   return cnt;
 }
 
-// Gershgorin interval [lo, hi] and ||T|| (max row sum) of T, widened by
-// 2 eps ||T||; the same arithmetic in every caller
-__device__ void tri_bounds(const double *d, const double *e, int n, double *lo, double *hi,
-                           double *nrm, double *pivmin) {
-  double l = 1e300, h = -1e300, t = 0.0, emax2 = 0.0;
-  for (int i = 0; i < n; ++i) {
+// Gershgorin bounds of the rows i, i + stride, ... of T: interval [lo, hi] and
+// largest absolute row sum nrm (reduced over the threads by the callers; min
+// and max do not depend on the order)
+__device__ __forceinline__ void tri_bounds(const double *d, const double *e, int n, int i0,
+                                           int stride, double &lo, double &hi, double &nrm) {
+  lo = 1e300;
+  hi = -1e300;
+  nrm = 0.0;
+  for (int i = i0; i < n; i += stride) {
     const double ei = i + 1 < n ? fabs(e[i]) : 0.0, em = i > 0 ? fabs(e[i - 1]) : 0.0;
-    l = fmin(l, d[i] - ei - em);
-    h = fmax(h, d[i] + ei + em);
-    t = fmax(t, fabs(d[i]) + ei + em);
-    if (i + 1 < n) emax2 = fmax(emax2, e[i] * e[i]);
+    lo = fmin(lo, d[i] - ei - em);
+    hi = fmax(hi, d[i] + ei + em);
+    nrm = fmax(nrm, fabs(d[i]) + ei + em);
   }
-  const double eps = 2.220446049250313e-16;
-  *lo = l - (2.0 * eps * t + 1e-300);
-  *hi = h + (2.0 * eps * t + 1e-300);
-  *nrm = t;
-  *pivmin = fmax(1e-300, 1e-290 * fmax(1.0, emax2));
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    nrm = fmax(nrm, __shfl_xor_sync(0xffffffffu, nrm, o));
+  }
 }
 
 struct SymEigWork {
@@ -282,49 +309,86 @@ k_symeig_tridiag_b(const SymEigJob *__restrict__ jobs) {
   symeig_tridiag_body<C>(j.A, j.lda, j.n, j.work);
 }
 
-// ---- 2. eigenvalues: multisection on Sturm counts, one warp per eigenvalue --
-constexpr int kSymEigWarps = 8;   // warps per CTA of phases 2 and 3
+// ---- 2. eigenvalues: multisection on Sturm counts, one CTA per eigenvalue ---
+// A round evaluates the count at kValThreads points of the interval, so that
+// it shrinks 257-fold: 7 rounds instead of the 11 of one warp's 32 points.
+// Measured for the whole eigensolve (25 / 62 pairs of n = 100 / 300): 457 -> 371 us and
+// 1744 -> 1492 us against one warp per eigenvalue with the quotient recurrence.
+constexpr int kSymEigWarps = 8;   // warps per CTA of phase 3
+constexpr int kValThreads = 256;
+
+__host__ __device__ inline size_t symeig_val_smem_bytes(int n) {
+  return sizeof(double) * 4 * (size_t)n;
+}
+
 __device__ __forceinline__ void
-symeig_values_body(int n, int k, const double *__restrict__ work, double *__restrict__ w) {
-  extern __shared__ double sm[];
-  double *d = sm, *e = sm + n, *e2 = sm + 2 * n;
+symeig_values_body(int j, int n, const double *__restrict__ work, double *__restrict__ w) {
+  extern __shared__ __align__(16) double sm[];
+  double2 *db = (double2 *)sm;                 // scaled {d_i, e_{i-1}^2}
+  double *d = sm + 2 * (size_t)n, *e = d + n;
+  __shared__ double red[3][kValThreads / 32];
+  __shared__ int first[2][kValThreads / 32];
   const SymEigWork g(const_cast<double *>(work), n);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < n; i += kValThreads) {
     d[i] = g.d[i];
     e[i] = g.e[i];
-    e2[i] = i + 1 < n ? g.e[i] * g.e[i] : 0.0;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * kSymEigWarps + (threadIdx.x >> 5);
-  if (j >= k) return;
-  const double eps = 2.220446049250313e-16;
-  double a, b, nrm, pivmin;
-  tri_bounds(d, e, n, &a, &b, &nrm, &pivmin);
+  double a, b, nrm;
+  tri_bounds(d, e, n, tid, kValThreads, a, b, nrm);
+  if (lane == 0) {
+    red[0][warp] = a;
+    red[1][warp] = b;
+    red[2][warp] = nrm;
+  }
+  __syncthreads();
+  for (int q = 0; q < kValThreads / 32; ++q) {
+    a = fmin(a, red[0][q]);
+    b = fmax(b, red[1][q]);
+    nrm = fmax(nrm, red[2][q]);
+  }
+  // scale by a power of two to ||T|| in [1/2, 1) (exact)
+  int ex = 0;
+  if (nrm > 0.0 && nrm < 1e300) frexp(nrm, &ex);
+  const double sc = ldexp(1.0, -ex), eps = 2.220446049250313e-16;
+  a = a * sc - (2.0 * eps * nrm * sc + 1e-300);
+  b = b * sc + (2.0 * eps * nrm * sc + 1e-300);
+  for (int i = tid; i < n; i += kValThreads) {
+    const double em = i > 0 ? e[i - 1] * sc : 0.0;
+    db[i] = make_double2(d[i] * sc, fmax(em * em, kE2Min));
+  }
+  __syncthreads();
   for (int round = 0; round < 64; ++round) {
     if (b - a <= 2.0 * eps * fmax(fabs(a), fabs(b)) + 1e-300) break;
-    const double x = a + (b - a) * (double)(lane + 1) / 33.0;
-    const int cnt = sturm_count(d, e2, n, x, pivmin);
+    const double h = (b - a) * (1.0 / (kValThreads + 1));
+    const int cnt = sturm_count(db, n, fma(h, (double)(tid + 1), a));
     // the first point with more than j eigenvalues below it bounds eigenvalue j
     const unsigned above = __ballot_sync(0xffffffffu, cnt > j);
-    const int l = above ? __ffs(above) - 1 : 32;
-    const double na = l == 0 ? a : a + (b - a) * (double)l / 33.0;
-    const double nb = l == 32 ? b : a + (b - a) * (double)(l + 1) / 33.0;
+    if (lane == 0) first[round & 1][warp] = above ? __ffs(above) - 1 : 32;
+    __syncthreads();
+    int l = kValThreads;
+    for (int q = kValThreads / 32 - 1; q >= 0; --q) {
+      const int f = first[round & 1][q];
+      if (f < 32) l = 32 * q + f;
+    }
+    const double na = l == 0 ? a : fma(h, (double)l, a);
+    const double nb = l == kValThreads ? b : fma(h, (double)(l + 1), a);
     a = na;
     b = nb;
   }
-  if (lane == 0) w[j] = 0.5 * (a + b);
+  if (tid == 0) w[j] = ldexp(0.5 * (a + b), ex);
 }
 
-__global__ void __launch_bounds__(kSymEigWarps * 32)
-k_symeig_values(int n, int k, const double *__restrict__ work, double *__restrict__ w) {
-  symeig_values_body(n, k, work, w);
+__global__ void __launch_bounds__(kValThreads)
+k_symeig_values(int n, const double *__restrict__ work, double *__restrict__ w) {
+  symeig_values_body(blockIdx.x, n, work, w);
 }
 
-__global__ void __launch_bounds__(kSymEigWarps * 32)
+__global__ void __launch_bounds__(kValThreads)
 k_symeig_values_b(const SymEigJob *__restrict__ jobs) {
   const SymEigJob j = jobs[blockIdx.y];
-  symeig_values_body(j.n, j.k, j.work, j.w);
+  if (blockIdx.x < j.k) symeig_values_body(blockIdx.x, j.n, j.work, j.w);
 }
 
 // ---- 3. eigenvectors of T, one warp per cluster of close eigenvalues --------
@@ -350,8 +414,8 @@ symeig_vectors_body(int n, int k, double *__restrict__ work, const double *__res
   const int j0 = blockIdx.x * kSymEigWarps + wl;
   if (j0 >= k) return;
   const double eps = 2.220446049250313e-16;
-  double lo_, hi_, nrm, pivmin_;
-  tri_bounds(d, e, n, &lo_, &hi_, &nrm, &pivmin_);
+  double lo_, hi_, nrm;
+  tri_bounds(d, e, n, lane, 32, lo_, hi_, nrm);
   const double ortol = 1e-5 * nrm, pertol = 10.0 * eps * nrm, tiny = eps * nrm + 1e-300;
   if (j0 > 0 && (w[j0] - w[j0 - 1]) <= ortol) return;   // not the first of its cluster
   int j1 = j0 + 1;
@@ -550,7 +614,7 @@ inline void symeig_small(cudaStream_t s, const double *A, int lda, int n, int k,
   S2G_CUDA(cudaFuncSetAttribute(k_symeig_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)symeig_vec_smem_bytes(kSymEigMaxN)));
   const int nb = (k + kSymEigWarps - 1) / kSymEigWarps;
-  S2G_LAUNCH(k_symeig_values, nb, kSymEigWarps * 32, 3 * n * sizeof(double), s, n, k, work, w);
+  S2G_LAUNCH(k_symeig_values, k, kValThreads, symeig_val_smem_bytes(n), s, n, work, w);
   S2G_LAUNCH(k_symeig_vectors, nb, kSymEigWarps * 32, symeig_vec_smem_bytes(n), s, n, k, work, w);
   S2G_LAUNCH(k_symeig_backtransform, nb, kSymEigWarps * 32, symeig_bt_smem_bytes(n), s, n, k,
              work, w, Z, ldz, info);
@@ -601,7 +665,7 @@ inline void symeig_small_batched(cudaStream_t s, const std::vector<SymEigJob> &j
   S2G_CUDA(cudaFuncSetAttribute(k_symeig_vectors_b, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)symeig_vec_smem_bytes(kSymEigMaxN)));
   const dim3 g((kmax + kSymEigWarps - 1) / kSymEigWarps, nj);
-  S2G_LAUNCH(k_symeig_values_b, g, kSymEigWarps * 32, 3 * nmax * sizeof(double), s, d);
+  S2G_LAUNCH(k_symeig_values_b, dim3(kmax, nj), kValThreads, symeig_val_smem_bytes(nmax), s, d);
   S2G_LAUNCH(k_symeig_vectors_b, g, kSymEigWarps * 32, symeig_vec_smem_bytes(nmax), s, d);
   S2G_LAUNCH(k_symeig_backtransform_b, g, kSymEigWarps * 32, symeig_bt_smem_bytes(nmax), s, d);
 }
