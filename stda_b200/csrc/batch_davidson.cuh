@@ -177,7 +177,7 @@ __global__ void k_bd_scale(const BdJob *__restrict__ jobs) {
 
 // Cholesky factor and inverse of every member's Gram matrix G (nc x nc, one
 // CTA each, chol_inv_body); stat[2 b], stat[2 b + 1] as k_chol_inv's
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kCholThreads)
 k_bd_chol_inv(const BdJob *__restrict__ jobs, double tol, double *__restrict__ stat) {
   const BdJob j = jobs[blockIdx.x];
   chol_inv_body(j.G, j.nc, tol, j.Li, stat + 2 * blockIdx.x);
@@ -684,8 +684,6 @@ inline void BatchDavidson::iterate(std::vector<BatchProblem *> &act) {
     S2G_LAUNCH(k_bd_colnorm_finish, Q, 128, 0, cs_, d, Q, ncap, part, kColSplit);
     S2G_LAUNCH(k_bd_scale, dim3(bd_blocks(mx), (unsigned)Q), 256, 0, cs_, d);
   }
-  S2G_CUDA(cudaFuncSetAttribute(k_bd_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(2 * sizeof(double) * kCholMax * kCholMax)));
   for (int round = 0; round < 2; ++round) {
     std::vector<BatchProblem *> o;
     for (BatchProblem *p : act)
@@ -693,7 +691,6 @@ inline void BatchDavidson::iterate(std::vector<BatchProblem *> &act) {
     if (o.empty()) break;
     std::vector<DgProblem> gp, gt, gg;
     std::vector<BdJob> cj;
-    int ncmax = 0;
     for (BatchProblem *p : o) {
       DavidsonWork &dw = *p->dw;
       const int64_t n = p->n;
@@ -706,15 +703,13 @@ inline void BatchDavidson::iterate(std::vector<BatchProblem *> &act) {
       BdJob j = bd_job(*p);
       j.nc = p->ncur;
       cj.push_back(j);
-      ncmax = std::max(ncmax, p->ncur);
     }
     dg_.grouped(cs_, true, false, gp, &stage_);
     dg_.grouped(cs_, false, false, gt, &stage_);
     dg_.grouped(cs_, true, false, gg, &stage_);
     const BdJob *d = upload(cj);
     double *st = gstat_.ensure(2 * o.size());
-    S2G_LAUNCH(k_bd_chol_inv, (int)o.size(), 256, 2 * sizeof(double) * ncmax * ncmax, cs_, d,
-               1e-8, st);
+    S2G_LAUNCH(k_bd_chol_inv, (int)o.size(), kCholThreads, 0, cs_, d, 1e-8, st);
     back_.reset();
     double *b_st = (double *)back_.take(sizeof(double) * 2 * o.size());
     S2G_CUDA(cudaMemcpyAsync(b_st, st, sizeof(double) * 2 * o.size(), cudaMemcpyDeviceToHost,

@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "dgemm.cuh"
+#include "symeig_seq.cuh"
 #include "symeig_small.cuh"
 
 namespace std2g {
@@ -138,83 +139,124 @@ __global__ void k_diag_matrix(double *__restrict__ H, int ld, int k, const doubl
 // column-major nc x nc, zero below the diagonal) so that T L^-T has
 // orthonormal columns.  stat[0] = 1 when a pivot is not positive or its
 // square root falls below sqrt(tol) (the block is numerically dependent),
-// else 0; stat[1] = the smallest pivot (the diagonal of L).  Right-looking
-// factorisation, then one forward substitution per column of L^-1 (thread j
-// solves L x = e_j); deterministic.
-constexpr int kCholMax = 112;   // 2 nc^2 doubles of shared memory
-__device__ __forceinline__ void chol_inv_body(const double *__restrict__ G, int nc, double tol,
-                                              double *__restrict__ out,
-                                              double *__restrict__ stat) {
-  extern __shared__ double sm[];
-  double *L = sm;               // column-major nc x nc
-  double *X = sm + nc * nc;     // X[j*nc + i] = (L^-1)[i][j]
-  __shared__ int fail;
-  __shared__ double dmin;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int q = tid; q < nc * nc; q += nt) {
-    const int i = q % nc, j = q / nc;
-    L[q] = i >= j ? G[q] : 0.0;
-  }
-  if (tid == 0) {
-    fail = 0;
-    dmin = 1e300;
+// else 0; stat[1] = the smallest pivot (the diagonal of L).  Deterministic.
+// Latency-bound: nc dependent steps.  The elimination runs in place on [G | I]
+// in its square-root-free form G = M D M^T: step j subtracts G_ij / d_j times
+// row j from every row i > j, over the trailing columns of G and over the
+// columns of M^-1 grown so far, which take the places of the eliminated ones.
+// Row i lives in the registers of warp i mod 16 (lane = column mod 32); row j
+// is passed through shared memory, and the multipliers are its own entries
+// (the trailing block is kept whole, hence symmetric), so a step is one read
+// of that row, the row updates, one reciprocal (by the lane that holds the next
+// pivot) and one barrier.  L^-1 =
+// D^-1/2 M^-1 at the end.  10.5 / 21 / 29 / 97 us at nc = 25 / 40 / 62 /
+// 112, where a factorisation followed by one forward substitution per thread
+// took 29 / 51 / 103 / 333 us.
+constexpr int kCholMax = 112;
+constexpr int kCholThreads = 512;
+template <int RT, int CT>   // rows per warp, columns per lane: nc <= 16 RT, 32 CT
+__device__ __forceinline__ void chol_inv_tile(const double *__restrict__ G, int nc, double tol,
+                                              double *__restrict__ out, double *__restrict__ stat,
+                                              double *row, double *inv, double *piv) {
+  constexpr int NW = kCholThreads / 32, LD = 128;   // row: two rows of LD, zero padded
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double w[RT][CT];   // rows i = warp + NW t, columns c = lane + 32 u
+#pragma unroll
+  for (int t = 0; t < RT; ++t)
+#pragma unroll
+    for (int u = 0; u < CT; ++u) {
+      const int i = warp + NW * t, c = lane + 32 * u;
+      w[t][u] = i < nc && c < nc ? G[max(i, c) + nc * min(i, c)] : 0.0;
+    }
+  for (int q = threadIdx.x; q < 2 * LD; q += kCholThreads) row[q] = 0.0;
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int u = 0; u < CT; ++u) row[lane + 32 * u] = w[0][u];
+    if (lane == 0) {
+      inv[0] = 1.0 / w[0][0];
+      piv[0] = w[0][0];
+    }
   }
   __syncthreads();
+  bool fail = false;
+  double dmin = 1e300;
   for (int j = 0; j < nc; ++j) {
-    if (tid == 0) {
-      const double d = L[j + nc * j];
-      if (!(d > 0.0) || !(d * d > 0.0) || !isfinite(d)) {
-        fail = 1;
-      } else {
-        const double r = sqrt(d);
-        L[j + nc * j] = r;
-        dmin = fmin(dmin, r);
-        if (!(r * r > tol)) fail = 1;
+    const double *rj = row + (j & 1) * LD;
+    const double d = rj[j], di = inv[j & 1];
+    double x[CT], m[RT];
+#pragma unroll
+    for (int u = 0; u < CT; ++u) x[u] = rj[lane + 32 * u];
+#pragma unroll
+    for (int t = 0; t < RT; ++t) m[t] = warp + NW * t > j ? rj[warp + NW * t] * -di : 0.0;
+    // dependent or not positive: the same decision in every thread
+    if (!(d > tol) || !(d * d > 0.0) || !isfinite(d)) {
+      if (d > 0.0) dmin = fmin(dmin, d);
+      fail = true;
+      break;
+    }
+    dmin = fmin(dmin, d);
+#pragma unroll
+    for (int t = 0; t < RT; ++t)
+#pragma unroll
+      for (int u = 0; u < CT; ++u) w[t][u] = fma(m[t], x[u], w[t][u]);
+    // column j of the rows below becomes M^-1's
+#pragma unroll
+    for (int u = 0; u < CT; ++u)
+      if (lane + 32 * u == j)
+#pragma unroll
+        for (int t = 0; t < RT; ++t)
+          if (warp + NW * t > j) w[t][u] = m[t];
+    // the next row, and the reciprocal of its pivot
+    if ((j + 1) % NW == warp) {
+      double *nx = row + ((j + 1) & 1) * LD;
+#pragma unroll
+      for (int t = 0; t < RT; ++t)
+        if (warp + NW * t == j + 1)
+#pragma unroll
+          for (int u = 0; u < CT; ++u) {
+            nx[lane + 32 * u] = w[t][u];
+            if (lane + 32 * u == j + 1) {
+              inv[(j + 1) & 1] = 1.0 / w[t][u];
+              piv[j + 1] = w[t][u];
+            }
+          }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    stat[0] = fail ? 1.0 : 0.0;
+    stat[1] = dmin < 1e300 ? sqrt(dmin) : dmin;
+  }
+  if (fail) return;
+  // out[c + nc*i] = (L^-1)[i][c]  (upper triangle: c <= i)
+#pragma unroll
+  for (int t = 0; t < RT; ++t) {
+    const int i = warp + NW * t;
+    if (i < nc) {
+      const double s = 1.0 / sqrt(piv[i]);
+#pragma unroll
+      for (int u = 0; u < CT; ++u) {
+        const int c = lane + 32 * u;
+        if (c < nc) out[c + nc * i] = c < i ? w[t][u] * s : (c == i ? s : 0.0);
       }
     }
-    __syncthreads();
-    if (fail) break;
-    const double r = L[j + nc * j];
-    for (int i = j + 1 + tid; i < nc; i += nt) L[i + nc * j] /= r;
-    __syncthreads();
-    // trailing update of the lower triangle: columns l > j, rows i >= l
-    const int m = nc - j - 1;
-    for (int q = tid; q < m * m; q += nt) {
-      const int l = j + 1 + q / m, i = j + 1 + q % m;
-      if (i >= l) L[i + nc * l] -= L[i + nc * j] * L[l + nc * j];
-    }
-    __syncthreads();
-  }
-  if (fail) {
-    if (tid == 0) {
-      stat[0] = 1.0;
-      stat[1] = dmin;
-    }
-    return;
-  }
-  for (int j = tid; j < nc; j += nt) {
-    double *x = X + (size_t)j * nc;
-    for (int i = 0; i < j; ++i) x[i] = 0.0;
-    x[j] = 1.0 / L[j + nc * j];
-    for (int i = j + 1; i < nc; ++i) {
-      double acc = 0.0;
-      for (int k = j; k < i; ++k) acc += L[i + nc * k] * x[k];
-      x[i] = -acc / L[i + nc * i];
-    }
-  }
-  __syncthreads();
-  // out[r + nc*c] = (L^-1)[c][r] = X[r*nc + c]  (upper: r <= c)
-  for (int q = tid; q < nc * nc; q += nt) {
-    const int r = q % nc, c = q / nc;
-    out[q] = r <= c ? X[(size_t)r * nc + c] : 0.0;
-  }
-  if (tid == 0) {
-    stat[0] = 0.0;
-    stat[1] = dmin;
   }
 }
 
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ void chol_inv_body(const double *__restrict__ G, int nc, double tol,
+                                              double *__restrict__ out,
+                                              double *__restrict__ stat) {
+  __shared__ double row[2 * 128], inv[2], piv[128];
+  if (nc <= 32)
+    chol_inv_tile<2, 1>(G, nc, tol, out, stat, row, inv, piv);
+  else if (nc <= 64)
+    chol_inv_tile<4, 2>(G, nc, tol, out, stat, row, inv, piv);
+  else
+    chol_inv_tile<7, 4>(G, nc, tol, out, stat, row, inv, piv);
+}
+
+__global__ void __launch_bounds__(kCholThreads)
 k_chol_inv(const double *__restrict__ G, int nc, double tol, double *__restrict__ out,
            double *__restrict__ stat) {
   chol_inv_body(G, nc, tol, out, stat);
@@ -274,9 +316,10 @@ constexpr int kRRSmallMax = kSymEigMaxN;
 // matrix is not safely positive definite, orthonormalisation through the Gram
 // matrix's eigen-decomposition that drops dependent directions).  Returns the
 // number of columns appended.  kcap: capacity of the k x k work arrays.
+// fixed_order: the small factorisations by the kernels of symeig_seq.cuh.
 inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t sol,
                               cudaStream_t s, double *V, int n, int m, double *T, int nc,
-                              int kcap) {
+                              int kcap, bool fixed_order = false) {
   const int k = kcap;
   const int grid = 148 * 4;
   const double one = 1.0, zero = 0.0, mone = -1.0;
@@ -303,10 +346,15 @@ inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnH
       if (ncur <= kCholMax) {
         // Cholesky QR: L^-T from the engine's small factorisation kernel
         double *Li = dw.Gc.ensure((size_t)k * k), *st = dw.stat.ensure(2);
-        S2G_CUDA(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(2 * sizeof(double) * kCholMax * kCholMax)));
-        S2G_LAUNCH(k_chol_inv, 1, 256, 2 * sizeof(double) * ncur * ncur, s, G, ncur, 1e-8, Li,
-                   st);
+        if (fixed_order) {
+          S2G_CUDA(cudaFuncSetAttribute(seq::k_chol_inv,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)(2 * sizeof(double) * kCholMax * kCholMax)));
+          S2G_LAUNCH(seq::k_chol_inv, 1, 256, 2 * sizeof(double) * ncur * ncur, s, G, ncur, 1e-8,
+                     Li, st);
+        } else {
+          S2G_LAUNCH(k_chol_inv, 1, kCholThreads, 0, s, G, ncur, 1e-8, Li, st);
+        }
         double h_st[2];
         S2G_CUDA(cudaMemcpyAsync(h_st, st, sizeof(h_st), cudaMemcpyDeviceToHost, s));
         S2G_CUDA(cudaStreamSynchronize(s));
@@ -327,8 +375,12 @@ inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnH
       if (ncur <= kRRSmallMax) {
         double *Z = dw.Gz.ensure((size_t)k * k);
         S2G_CUDA(cudaMemsetAsync(info, 0, sizeof(int), s));
-        symeig_small(s, G, ncur, ncur, ncur, lam, Z, ncur,
-                     dw.eigwork.ensure(symeig_work_doubles(ncur, ncur)), info);
+        if (fixed_order)
+          seq::symeig_small(s, G, ncur, ncur, ncur, lam, Z, ncur,
+                            dw.eigwork.ensure(seq::symeig_work_doubles(ncur, ncur)), info);
+        else
+          symeig_small(s, G, ncur, ncur, ncur, lam, Z, ncur,
+                       dw.eigwork.ensure(symeig_work_doubles(ncur, ncur)), info);
         S2G_CUDA(cudaMemcpyAsync(G, Z, sizeof(double) * ncur * ncur, cudaMemcpyDeviceToDevice,
                                  s));
       } else {

@@ -22,7 +22,7 @@
 #include "common.cuh"
 #include "davidson.cuh"
 #include "kernels_fp64.cuh"
-#include "symeig_small.cuh"
+#include "symeig_seq.cuh"
 
 namespace std2g {
 
@@ -107,7 +107,8 @@ inline void rpa_small_eig(DavidsonWork &dw, DavidsonRpaWork &rw, cusolverDnHandl
                           cudaStream_t s, const double *A, int lda, int m, int k, double *w,
                           double *Z, double *Zfull, int *einfo) {
   if (m <= kSymEigMaxN) {
-    symeig_small(s, A, lda, m, k, w, Z, m, dw.eigwork.ensure(symeig_work_doubles(m, k)), einfo);
+    seq::symeig_small(s, A, lda, m, k, w, Z, m,
+                      dw.eigwork.ensure(seq::symeig_work_doubles(m, k)), einfo);
     return;
   }
   // full decomposition on a copy, the lowest k pairs are its leading columns
@@ -278,7 +279,7 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
       }
       m = nkeep;
     }
-    nb = dav_orthonormalize(dw, blas, sol, s, B, n, m, T, 2 * nc, 2 * k);
+    nb = dav_orthonormalize(dw, blas, sol, s, B, n, m, T, 2 * nc, 2 * k, true);
     if (nb == 0) break;
   }
   S2G_CUDA(cudaMemcpyAsync(omega_out, om, sizeof(double) * kwant, cudaMemcpyDeviceToDevice, s));
