@@ -2,9 +2,9 @@
 // for the Rayleigh-Ritz step of the Davidson solver, in four kernels with no
 // host synchronisation:
 //   1. k_symeig_tridiag: Householder reduction to tridiagonal form
-//      T = Q^T A Q (LAPACK dsytd2, lower, restated) by a cluster of 4 or 8
-//      CTAs with one cluster barrier per reflector (the scheme is described
-//      at the kernel); d, e, tau and the reflectors go to a global workspace;
+//      T = Q^T A Q (LAPACK dsytd2, lower, restated) by one CTA or a cluster of
+//      4 or 8, the matrix in registers (the scheme is described at the
+//      kernel); d, e, tau and the reflectors go to a global workspace;
 //   2. k_symeig_values (one CTA per eigenvalue): multisection on Sturm counts
 //      (LAPACK dstebz's principle), each thread evaluating the count at one of
 //      256 points of the current interval per round;
@@ -31,36 +31,31 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
 
 namespace std2g {
 
-constexpr int kTridiagThreads = 512;
-constexpr int kSymEigMaxN = 320;       // full columns of n/8 per CTA, 119 KB
+constexpr int kTridiagThreads = 256;
+constexpr int kSymEigMaxN = 320;       // 3 columns per warp in a cluster of 8 CTAs
 
-// global workspace (doubles): packed reflectors, d, e, tau, 8 spare, and per
-// eigenvector its final y in T's basis (n)
+constexpr int kBtBlock = 8;   // reflectors applied together by the back-transformation
+__host__ __device__ inline int symeig_bt_blocks(int n) {
+  return n > 2 ? (n - 2 + kBtBlock - 1) / kBtBlock : 0;
+}
+
+// global workspace (doubles): packed reflectors, d, e, tau, the triangular
+// factors of the reflector blocks, and per eigenvector its y in T's basis (n)
 __host__ __device__ inline size_t symeig_work_doubles(int n, int k) {
-  return (size_t)n * (n + 1) / 2 + 3 * (size_t)n + 8 + (size_t)k * n;
+  return (size_t)n * (n + 1) / 2 + 3 * (size_t)n +
+         (size_t)symeig_bt_blocks(n) * kBtBlock * kBtBlock + (size_t)k * n;
 }
 
 // packed lower column-major index of (i, j), i >= j
 __device__ __forceinline__ int pk_idx(int i, int j, int n) {
   return j * (2 * n - j + 1) / 2 + (i - j);
-}
-
-__device__ double symeig_block_sum(double v, double *red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double t = 0.0;
-  const int nw = blockDim.x >> 5;
-  for (int q = 0; q < nw; ++q) t += red[q];   // every thread, same order
-  return t;
 }
 
 // Number of eigenvalues below x of the scaled T: the sign changes of the
@@ -124,14 +119,14 @@ __device__ __forceinline__ void tri_bounds(const double *d, const double *e, int
 }
 
 struct SymEigWork {
-  double *ap, *d, *e, *tau, *spare, *vec;
+  double *ap, *d, *e, *tau, *bt, *vec;
   __host__ __device__ SymEigWork(double *work, int n) {
     ap = work;
     d = ap + (size_t)n * (n + 1) / 2;
     e = d + n;
     tau = e + n;
-    spare = tau + n;
-    vec = spare + 8;
+    bt = tau + n;
+    vec = bt + (size_t)symeig_bt_blocks(n) * kBtBlock * kBtBlock;
   }
 };
 
@@ -148,165 +143,279 @@ struct SymEigJob {
 };
 
 // ---- 1. tridiagonal reduction (Q^T A Q = T, Q = H_0 ... H_{n-3}) ----------
-// A cluster of C CTAs; CTA r holds the full columns j = r (mod C) in shared
-// memory, and every CTA also keeps the current column c (cur) and forms the
-// reflector of step c from it itself, with the same arithmetic in every CTA,
-// so that a step takes one cluster barrier:
-//   phase 1: each CTA forms p_j = tau (A v)_j for its own columns j > c as the
-//            dot product of column j with v (A is symmetric), and the owner of
-//            column c+1 publishes that column;
-//   barrier;
-//   phase 2: each CTA gathers p and column c+1 from the owners (distributed
-//            shared memory), forms w = p - (tau p^T v / 2) v, applies the
-//            rank-2 update A -= v w^T + w v^T to its own columns and to its copy
-//            of column c+1, and forms the next reflector from that copy.
-// The published p pieces and columns alternate between two buffers: a CTA
-// that writes buffer (c+1) % 2 has passed the barrier of step c, so every CTA
-// has finished reading that buffer at step c-1.  Every CTA takes the same
-// barriers (all decisions depend on data the CTAs hold identically).
-__host__ __device__ inline int symeig_cluster_ctas(int n) { return n <= 96 ? 4 : 8; }
+// Latency-bound: n - 2 dependent steps.  The matrix stays in the registers of
+// 8 C warps (C CTAs of one cluster): warp g holds the whole columns
+// j = g, g + 8 C, ... (CPW of them), lane l the rows l, l + 32, ... (RB of
+// them).  Every warp keeps itself informed instead of waiting for a block-wide
+// reduction: each one forms the reflector of the current column (cur, in
+// shared memory) and later p^T v with its own shuffles, all with the same
+// arithmetic, so a step takes two barriers:
+//   v, tau from cur; p_j = tau (A v)_j for the own columns, written to the p
+//   array of every CTA; the owner of column c+1 publishes it;
+//   cluster barrier;
+//   w = p - (tau p^T v / 2) v; thread i updates element i of column c+1 into
+//   the next cur; A -= v w^T + w v^T on the own columns;
+//   CTA barrier.
+// The steps run in phases of 32, so that the row blocks and columns that are
+// done drop out at compile time; eight warps, not more, because each repeats
+// the square root and the divisions of the reflector.
+// p and the published column alternate between two buffers: a CTA that writes
+// buffer (c+1) % 2 has passed the cluster barrier of step c, which every CTA
+// enters only after reading that buffer in step c-1.
+// Measured for the whole eigensolve (n = 100 / 300, 25 / 62 pairs): 347 -> 220 us
+// and 1422 -> 799 us against columns in shared memory with block-wide reductions
+// and 4 / 8 CTAs.
+template <int C_, int RB_, int CPW_>
+struct TridiagShape {
+  static constexpr int C = C_, RB = RB_, CPW = CPW_;
+};
+constexpr int kTridiagWarps = kTridiagThreads / 32;
 
-__host__ __device__ inline size_t symeig_smem_bytes(int n, int C) {
-  const size_t ncol = (size_t)(n + C - 1) / C;
-  // own columns, v, p, w, cur, published p pieces [2][ncol], published column
-  // [2][n], reduction scratch
-  return sizeof(double) * (ncol * n + 4 * (size_t)n + 2 * ncol + 2 * (size_t)n + 64);
+template <int I, int N, class F>
+__device__ __forceinline__ void static_for(F &&f) {
+  if constexpr (I < N) {
+    f(std::integral_constant<int, I>{});
+    static_for<I + 1, N>(f);
+  }
 }
 
-// reflector H_c = I - tau v v^T of the current column c (cur, rows c+1..n-1;
-// LAPACK dlarfg's convention: v[c+1] = 1, beta = -sign(alpha) ||x||);
-// the writer CTA stores v, tau, beta = e[c] and d[c] = cur[c]
-__device__ double symeig_reflector(const double *cur, int c, int n, double *v, double *red,
-                                   const SymEigWork &g, bool writer) {
-  const int r0 = c + 1, tid = threadIdx.x, nt = blockDim.x;
-  const double alpha = cur[r0];
-  double s = 0.0;
-  for (int i = r0 + 1 + tid; i < n; i += nt) s += cur[i] * cur[i];
-  const double xn2 = symeig_block_sum(s, red);
-  double tc = 0.0, beta = alpha, scal = 0.0;
-  if (xn2 != 0.0) {
-    beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-    tc = (beta - alpha) / beta;
-    scal = 1.0 / (alpha - beta);
+// Sums of NQ values over the warp: on return lane l holds in x[0] the sum of
+// value q(l), the top log2 bits of the lane (NQ rounded up to a power of two):
+// the halves of the lanes exchange halves of the values, NQ - 1 shuffles
+// instead of 5 NQ, then the rest reduce one value.
+template <int NQ>
+__device__ __forceinline__ int warp_sums(double (&x)[NQ], int lane) {
+  constexpr int P = NQ <= 1 ? 1 : NQ <= 2 ? 2 : NQ <= 4 ? 4 : NQ <= 8 ? 8 : 16;
+  double y[P];
+#pragma unroll
+  for (int q = 0; q < P; ++q) y[q] = q < NQ ? x[q] : 0.0;
+  int o = 16, q0 = 0;
+#pragma unroll
+  for (int h = P / 2; h > 0; h >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double send = up ? y[q] : y[q + h], keep = up ? y[q + h] : y[q];
+      y[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    q0 += up ? h : 0;
+    o >>= 1;
   }
-  for (int i = r0 + tid; i < n; i += nt) {
-    const double vi = i == r0 ? 1.0 : cur[i] * scal;
-    v[i] = vi;
-    if (writer && i > r0) g.ap[pk_idx(i, c, n)] = vi;   // kept for the back-transformation
-  }
-  if (writer && tid == 0) {
-    g.tau[c] = tc;
-    g.e[c] = beta;
-    g.d[c] = cur[c];
-  }
-  __syncthreads();
-  return tc;
+#pragma unroll
+  for (int b = 16; b > 0; b >>= 1)
+    if (b <= o) y[0] += __shfl_xor_sync(0xffffffffu, y[0], b);
+  x[0] = y[0];
+  return q0;
 }
 
-template <int C>
+template <class Shape>
 __device__ __forceinline__ void
 symeig_tridiag_body(const double *__restrict__ A, int lda, int n, double *__restrict__ work) {
+  constexpr int C = Shape::C, RB = Shape::RB, CPW = Shape::CPW, LD = 32 * RB;
+  constexpr int G = kTridiagWarps * C;
   namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank();
-  extern __shared__ double sm[];
-  const int ncol = (n + C - 1) / C;   // local columns j = rank + C * lj
-  double *Aloc = sm;                  // [lj * n + i]
-  double *v = Aloc + (size_t)ncol * n, *p = v + n, *w = p + n, *cur = w + n;
-  double *pubp = cur + n;             // [2][ncol]
-  double *pubc = pubp + 2 * ncol;     // [2][n]
-  double *red = pubc + 2 * n;         // [64]
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int nw = nt >> 5;
-  const bool writer = rank == 0;
-  SymEigWork g(work, n);
-  for (int lj = 0; lj < ncol; ++lj) {
-    const int j = rank + C * lj;
-    if (j >= n) break;
-    for (int i = tid; i < n; i += nt)
-      Aloc[(size_t)lj * n + i] = i >= j ? A[i + (size_t)lda * j] : A[j + (size_t)lda * i];
+  __shared__ double s_cur[2][LD], s_p[2][LD], s_col[2][LD];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int rank = 0;
+  if constexpr (C > 1) rank = (int)cg::this_cluster().block_rank();
+  const int gw = rank * kTridiagWarps + warp;   // columns gw + G q
+  const SymEigWork g(work, n);
+  double a[CPW][RB];
+#pragma unroll
+  for (int q = 0; q < CPW; ++q)
+#pragma unroll
+    for (int t = 0; t < RB; ++t) {
+      const int j = gw + G * q, i = lane + 32 * t;
+      a[q][t] = i < n && j < n ? A[max(i, j) + (size_t)lda * min(i, j)] : 0.0;
+    }
+  for (int i = tid; i < LD; i += kTridiagThreads) {
+    s_cur[0][i] = i < n ? A[i] : 0.0;   // column 0
+    s_cur[1][i] = 0.0;
+    s_p[0][i] = s_p[1][i] = 0.0;
+    s_col[0][i] = s_col[1][i] = 0.0;
   }
-  for (int i = tid; i < n; i += nt) cur[i] = A[i];   // column 0
-  __syncthreads();
-  double tc = n >= 3 ? symeig_reflector(cur, 0, n, v, red, g, writer) : 0.0;
-  for (int c = 0; c + 2 < n; ++c) {
-    const int r0 = c + 1, nxt = c + 1, own_nxt = nxt % C, buf = c & 1;
-    // first local column with j >= r0
-    const int lj0 = r0 > rank ? (r0 - rank + C - 1) / C : 0;
-    // ---- phase 1
-    if (tc != 0.0) {
-      for (int lj = lj0 + warp; lj < ncol; lj += nw) {
-        const int j = rank + C * lj;
-        if (j >= n) break;
-        const double *col = Aloc + (size_t)lj * n;
-        double sdot = 0.0;
-        for (int i = r0 + lane; i < n; i += 32) sdot += col[i] * v[i];
-        for (int o = 16; o > 0; o >>= 1) sdot += __shfl_xor_sync(0xffffffffu, sdot, o);
-        if (lane == 0) pubp[buf * ncol + lj] = tc * sdot;
+  if constexpr (C > 1) cg::this_cluster().sync();   // buffers cleared before remote writes
+  else __syncthreads();
+  static_for<0, RB>([&](auto phase) {
+    constexpr int T0 = decltype(phase)::value, NT = RB - T0;
+    constexpr int Q0 = 32 * T0 / G, NQ = CPW - Q0;   // columns below G Q0 are done
+    for (int c = max(0, 32 * T0 - 1); c < min(n - 2, 32 * T0 + 31); ++c) {
+      const int r0 = c + 1, buf = c & 1, l0 = lane + 32 * T0;
+      const double *cur = s_cur[buf];
+      // ---- reflector H_c = I - tau v v^T of rows r0..n-1 of cur (LAPACK
+      // dlarfg's convention: v[r0] = 1, beta = -sign(alpha) ||x||)
+      double v[NT], xn2 = 0.0;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        v[t] = l0 + 32 * t > r0 ? cur[l0 + 32 * t] : 0.0;
+        xn2 = fma(v[t], v[t], xn2);
       }
-    }
-    if (rank == own_nxt) {
-      const double *col = Aloc + (size_t)(nxt / C) * n;
-      for (int i = r0 + tid; i < n; i += nt) pubc[buf * n + i] = col[i];
-    }
-    cl.sync();
-    // ---- phase 2
-    const double *rc = cl.map_shared_rank(pubc + buf * n, own_nxt);
-    double pv = 0.0;
-    for (int i = r0 + tid; i < n; i += nt) {
-      cur[i] = rc[i];
-      if (tc != 0.0) {
-        const double *rp = cl.map_shared_rank(pubp + buf * ncol, i % C);
-        const double pi = rp[i / C];
-        p[i] = pi;
-        pv += pi * v[i];
+      const double alpha = cur[r0];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
+      double tc = 0.0, beta = alpha, scal = 0.0;
+      if (xn2 != 0.0) {
+        beta = -copysign(sqrt(fma(alpha, alpha, xn2)), alpha);
+        tc = (beta - alpha) / beta;
+        scal = 1.0 / (alpha - beta);
       }
-    }
-    if (tc != 0.0) {
-      const double K = 0.5 * tc * symeig_block_sum(pv, red);   // same value in every CTA
-      for (int i = r0 + tid; i < n; i += nt) w[i] = p[i] - K * v[i];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) v[t] = l0 + 32 * t == r0 ? 1.0 : v[t] * scal;
+      if (gw == 0) {   // kept for the back-transformation
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int i = l0 + 32 * t;
+          if (i > r0 && i < n) g.ap[pk_idx(i, c, n)] = v[t];
+        }
+        if (lane == 0) {
+          g.tau[c] = tc;
+          g.e[c] = beta;
+          g.d[c] = cur[c];
+        }
+      }
+      // ---- p_j = tau (A v)_j, and column c+1 published by its owner
+      double ps[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        double s = 0.0;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) s = fma(a[Q0 + q][T0 + t], v[t], s);
+        ps[q] = s;
+        if (gw + G * (Q0 + q) == r0)
+#pragma unroll
+          for (int t = 0; t < NT; ++t) s_col[buf][l0 + 32 * t] = a[Q0 + q][T0 + t];
+      }
+      const int qs = warp_sums(ps, lane);
+      {
+        // the lanes of one value q write it, lane (their index) mod C to CTA .. C
+        constexpr int P = NQ <= 1 ? 1 : NQ <= 2 ? 2 : NQ <= 4 ? 4 : NQ <= 8 ? 8 : 16;
+        constexpr int L = 32 / P;   // lanes holding the same sum
+        const int j = gw + G * (Q0 + qs);
+        if (qs < NQ && j >= r0 && j < n) {
+#pragma unroll
+          for (int k = 0; k < (C + L - 1) / L; ++k) {
+            const int to = lane % L + L * k;
+            if (to < C) {
+              if constexpr (C > 1) cg::this_cluster().map_shared_rank(s_p[buf], to)[j] = tc * ps[0];
+              else s_p[buf][j] = tc * ps[0];
+            }
+          }
+        }
+      }
+      const double *rc = s_col[buf];
+      if constexpr (C > 1) {
+        cg::this_cluster().sync();
+        rc = cg::this_cluster().map_shared_rank(s_col[buf], (r0 % G) / kTridiagWarps);
+      } else {
+        __syncthreads();
+      }
+      // ---- w = p - K v, the next column, the rank-2 update
+      constexpr int NE = (LD + kTridiagThreads - 1) / kTridiagThreads;
+      double rci[NE];
+#pragma unroll
+      for (int k = 0; k < NE; ++k) {
+        const int i = tid + kTridiagThreads * k;
+        rci[k] = i >= r0 && i < n ? rc[i] : 0.0;
+      }
+      const double *p = s_p[buf];
+      double w[NT], pv = 0.0;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        w[t] = l0 + 32 * t >= r0 ? p[l0 + 32 * t] : 0.0;
+        pv = fma(w[t], v[t], pv);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) pv += __shfl_xor_sync(0xffffffffu, pv, o);
+      const double K = 0.5 * tc * pv;
+#pragma unroll
+      for (int k = 0; k < NE; ++k) {   // element i of column r0; v[r0] = 1
+        const int i = tid + kTridiagThreads * k;
+        if (i >= r0 && i < n) {
+          const double vi = i == r0 ? 1.0 : cur[i] * scal;
+          s_cur[buf ^ 1][i] = rci[k] - fma(vi, p[r0] - K, p[i] - K * vi);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) w[t] = fma(-K, v[t], w[t]);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const int j = gw + G * (Q0 + q);
+        // columns that are done take a zero update
+        const double vj = j > r0 && j < n ? cur[j] * scal : 0.0;
+        const double wj = j > r0 && j < n ? fma(-K, vj, p[j]) : 0.0;
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          a[Q0 + q][T0 + t] = fma(-v[t], wj, fma(-w[t], vj, a[Q0 + q][T0 + t]));
+      }
       __syncthreads();
-      const double vn = v[nxt], wn = w[nxt];
-      for (int i = r0 + tid; i < n; i += nt) cur[i] -= v[i] * wn + w[i] * vn;
-      for (int lj = lj0 + warp; lj < ncol; lj += nw) {
-        const int j = rank + C * lj;
-        if (j >= n) break;
-        const double vj = v[j], wj = w[j];
-        double *col = Aloc + (size_t)lj * n;
-        for (int i = r0 + lane; i < n; i += 32) col[i] -= v[i] * wj + w[i] * vj;
-      }
     }
-    __syncthreads();
-    if (c + 3 < n) tc = symeig_reflector(cur, nxt, n, v, red, g, writer);
-  }
+  });
   // the trailing 2 x 2 block: cur holds column n-2, column n-1 is on its owner
-  if (writer && tid == 0) {
-    if (n >= 2) {
-      g.d[n - 2] = cur[n - 2];
-      g.e[n - 2] = cur[n - 1];
-      g.tau[n - 2] = 0.0;
-    }
+  const double *cur = s_cur[max(n - 2, 0) & 1];
+  if (gw == 0 && lane == 0 && n >= 2) {
+    g.d[n - 2] = cur[n - 2];
+    g.e[n - 2] = cur[n - 1];
+    g.tau[n - 2] = 0.0;
   }
-  if (rank == (n - 1) % C && tid == 0) {
-    g.d[n - 1] = Aloc[(size_t)((n - 1) / C) * n + (n - 1)];
+  if (gw == (n - 1) % G && lane == (n - 1) % 32) {
+#pragma unroll
+    for (int q = 0; q < CPW; ++q)
+#pragma unroll
+      for (int t = 0; t < RB; ++t)
+        if (gw + G * q == n - 1 && lane + 32 * t == n - 1) g.d[n - 1] = a[q][t];
     g.e[n - 1] = 0.0;
     g.tau[n - 1] = 0.0;
   }
-  cl.sync();   // no CTA leaves while others may still read its shared memory
+  if constexpr (C > 1) cg::this_cluster().sync();   // shared memory still read by other CTAs
 }
 
-template <int C>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kTridiagThreads, 1)
+template <class Shape>
+__global__ void __launch_bounds__(kTridiagThreads, 1)
 k_symeig_tridiag(const double *__restrict__ A, int lda, int n, double *__restrict__ work) {
-  symeig_tridiag_body<C>(A, lda, n, work);
+  symeig_tridiag_body<Shape>(A, lda, n, work);
 }
 
 // batched form: cluster blockIdx.y solves jobs[blockIdx.y]
-template <int C>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kTridiagThreads, 1)
+template <class Shape>
+__global__ void __launch_bounds__(kTridiagThreads, 1)
 k_symeig_tridiag_b(const SymEigJob *__restrict__ jobs) {
   const SymEigJob j = jobs[blockIdx.y];
-  symeig_tridiag_body<C>(j.A, j.lda, j.n, j.work);
+  symeig_tridiag_body<Shape>(j.A, j.lda, j.n, j.work);
+}
+
+// f(shape index, Shape) for the shape that serves size n: the fewest CTAs whose
+// registers hold the matrix, up to where more of them were faster (whole
+// eigensolve: n = 96 188 us with one CTA, 212 / 203 with 2 / 4; n = 128 275
+// against 295 / 279; n = 150 343 with 4 against 372 / 342 with 2 / 8; n = 192
+// 439 with 8 against 453 / 500 with 4 / 2; n = 256 652 with 8 against 684)
+constexpr int kTridiagShapes = 8;
+template <class F>
+inline void symeig_tridiag_shape(int n, F &&f) {
+  if (n <= 32) f(0, TridiagShape<1, 1, 4>{});
+  else if (n <= 64) f(1, TridiagShape<1, 2, 8>{});
+  else if (n <= 96) f(2, TridiagShape<1, 3, 12>{});
+  else if (n <= 128) f(3, TridiagShape<1, 4, 16>{});
+  else if (n <= 160) f(4, TridiagShape<4, 5, 5>{});
+  else if (n <= 192) f(5, TridiagShape<8, 6, 3>{});
+  else if (n <= 256) f(6, TridiagShape<8, 8, 4>{});
+  else f(7, TridiagShape<8, 10, 5>{});
+}
+
+template <class... KArgs, class... Args>
+inline void launch_cluster(void (*kernel)(KArgs...), dim3 grid, int threads, int cluster,
+                           cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  ++g_launches;
 }
 
 // ---- 2. eigenvalues: multisection on Sturm counts, one CTA per eigenvalue ---
@@ -318,7 +427,7 @@ constexpr int kSymEigWarps = 8;   // warps per CTA of phase 3
 constexpr int kValThreads = 256;
 
 __host__ __device__ inline size_t symeig_val_smem_bytes(int n) {
-  return sizeof(double) * 4 * (size_t)n;
+  return sizeof(double) * (size_t)n * kBtBlock;   // values: 4 n, block factors: 8 n
 }
 
 __device__ __forceinline__ void
@@ -380,34 +489,90 @@ symeig_values_body(int j, int n, const double *__restrict__ work, double *__rest
   if (tid == 0) w[j] = ldexp(0.5 * (a + b), ex);
 }
 
+// entry i of the reflector vector of H_c (0 for i <= c, 1 at c + 1)
+__device__ __forceinline__ double symeig_v(const SymEigWork &g, int i, int c, int n) {
+  return c < 0 || i <= c ? 0.0 : (i == c + 1 ? 1.0 : g.ap[pk_idx(i, c, n)]);
+}
+
+// Triangular factor of reflector block b (for phase 4), formed beside the
+// eigenvalues on CTAs that would otherwise idle: the block applies H_c,
+// c = n-3-8b-r, in the order r = 0 .. 7, i.e. y <- y - sum_r f_r v_r with
+// f_r = tau_r (v_r^T y - sum_{q<r} (v_r^T v_q) f_q), so f = F V^T y with
+//   F_rr = tau_r,  F_rq = -tau_r sum_{q<=s<r} (v_r^T v_s) F_sq.
+__device__ __forceinline__ void symeig_block_factor(int b, int n, double *__restrict__ work) {
+  extern __shared__ __align__(16) double sm[];   // V[kBtBlock][n]
+  __shared__ double gram[kBtBlock][kBtBlock];
+  const SymEigWork g(work, n);
+  const int c1 = n - 3 - kBtBlock * b, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int x = threadIdx.x; x < kBtBlock * n; x += kValThreads)
+    sm[x] = symeig_v(g, x % n, c1 - x / n, n);
+  __syncthreads();
+  for (int x = warp; x < kBtBlock * kBtBlock; x += kValThreads / 32) {
+    const int r = x / kBtBlock, q = x % kBtBlock;
+    if (q >= r) continue;
+    double s = 0.0;
+    for (int i = lane; i < n; i += 32) s += sm[r * n + i] * sm[q * n + i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) gram[r][q] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < kBtBlock) {
+    const int q = threadIdx.x;
+    double f[kBtBlock];
+#pragma unroll
+    for (int r = 0; r < kBtBlock; ++r) {
+      const double t = c1 - r >= 0 ? g.tau[c1 - r] : 0.0;
+      double s = 0.0;
+#pragma unroll
+      for (int u = 0; u < r; ++u) s += u >= q ? gram[r][u] * f[u] : 0.0;
+      f[r] = r < q ? 0.0 : (r == q ? t : -t * s);
+      g.bt[((size_t)b * kBtBlock + r) * kBtBlock + q] = f[r];
+    }
+  }
+}
+
+// blocks 0 .. k-1: one eigenvalue each; block k + b: reflector block b
 __global__ void __launch_bounds__(kValThreads)
-k_symeig_values(int n, const double *__restrict__ work, double *__restrict__ w) {
-  symeig_values_body(blockIdx.x, n, work, w);
+k_symeig_values(int n, int k, double *__restrict__ work, double *__restrict__ w) {
+  if (blockIdx.x < k) symeig_values_body(blockIdx.x, n, work, w);
+  else symeig_block_factor(blockIdx.x - k, n, work);
 }
 
 __global__ void __launch_bounds__(kValThreads)
 k_symeig_values_b(const SymEigJob *__restrict__ jobs) {
   const SymEigJob j = jobs[blockIdx.y];
   if (blockIdx.x < j.k) symeig_values_body(blockIdx.x, j.n, j.work, j.w);
+  else if (blockIdx.x - j.k < symeig_bt_blocks(j.n))
+    symeig_block_factor(blockIdx.x - j.k, j.n, j.work);
 }
 
 // ---- 3. eigenvectors of T, one warp per cluster of close eigenvalues --------
 // Cluster threshold: eigenvalues closer than 1e-5 ||T|| are orthogonalised
 // against each other; further apart, inverse iteration alone gives vectors
-// orthogonal to ~eps ||T|| / gap <= 2e-11.  Shared memory: d, e, then per
-// warp y and the rows of U (ua holds 1 / pivot), multipliers, pivot flags.
+// orthogonal to ~eps ||T|| / gap <= 2e-11.  The factorisation and the solves
+// are serial chains in one lane, so they are arranged to carry as little as
+// possible: one reciprocal per row in the factorisation, rows of U divided by
+// their pivots beforehand by all lanes (one multiply-add per row in the back
+// substitution), the running values in registers, the rows' other entries
+// loaded four at a time; the first solve starts at the back substitution (its
+// start vector stands for L^-1 P y).  Whole eigensolve: -25 us at n = 100,
+// -70 us at n = 300 against the plain chains.
+// Shared memory: d, e, then per warp y, 1 / pivot, {u1, u2} (the two
+// super-diagonals of U over the pivot), {multiplier, row-swap flag}.
 __host__ __device__ inline size_t symeig_vec_smem_bytes(int n) {
-  return sizeof(double) * (2 * (size_t)n + (size_t)kSymEigWarps * 6 * n);
+  const size_t np = (size_t)(n + 1) & ~(size_t)1;   // 16-byte rows
+  return sizeof(double) * (2 * np + (size_t)kSymEigWarps * 6 * np);
 }
 
 __device__ __forceinline__ void
 symeig_vectors_body(int n, int k, double *__restrict__ work, const double *__restrict__ w) {
-  extern __shared__ double sm[];
-  double *d = sm, *e = sm + n;
+  extern __shared__ __align__(16) double sm[];
+  const int np = (n + 1) & ~1;
+  double *d = sm, *e = sm + np;
   const SymEigWork g(work, n);
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     d[i] = g.d[i];
-    e[i] = g.e[i];
+    e[i] = g.e[i];   // e[n-1] = 0
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -420,62 +585,97 @@ symeig_vectors_body(int n, int k, double *__restrict__ work, const double *__res
   if (j0 > 0 && (w[j0] - w[j0 - 1]) <= ortol) return;   // not the first of its cluster
   int j1 = j0 + 1;
   while (j1 < k && (w[j1] - w[j1 - 1]) <= ortol) ++j1;
-  double *y = sm + 2 * n + (size_t)wl * 6 * n;
-  double *ua = y + n, *ub = ua + n, *uc = ub + n, *mu = uc + n, *fl = mu + n;
+  double *y = sm + 2 * np + (size_t)wl * 6 * np, *ua = y + np;
+  double2 *ub = (double2 *)(ua + np), *mf = ub + np;
   double lam_prev = 0.0;
   for (int m = j0; m < j1; ++m) {
     double lam = w[m];
     if (m > j0 && lam - lam_prev < pertol) lam = lam_prev + pertol;
     lam_prev = lam;
-    if (lane == 0) {   // T - lam I = P L U, rows of U: (ua, ub, uc)
-      double a0 = d[0] - lam, b0 = n > 1 ? e[0] : 0.0;
+    if (lane == 0) {   // T - lam I = P L U with partial pivoting
+      double a0 = d[0] - lam, b0 = e[0];
       for (int i = 0; i + 1 < n; ++i) {
-        const double sub = e[i], dn = d[i + 1] - lam, en = i + 2 < n ? e[i + 1] : 0.0;
-        double piv;
-        if (fabs(a0) >= fabs(sub)) {
-          const double ml = a0 != 0.0 ? sub / a0 : 0.0;
-          piv = a0;
-          ub[i] = b0;
-          uc[i] = 0.0;
-          mu[i] = ml;
-          fl[i] = 0.0;
-          a0 = dn - ml * b0;
-          b0 = en;
-        } else {   // swap rows i and i+1
-          const double ml = a0 / sub;
-          piv = sub;
-          ub[i] = dn;
-          uc[i] = en;
-          mu[i] = ml;
-          fl[i] = 1.0;
-          a0 = b0 - ml * dn;
-          b0 = -ml * en;
-        }
+        const double sub = e[i], dn = d[i + 1] - lam, en = e[i + 1];
+        const bool sw = fabs(a0) < fabs(sub);   // swap rows i and i+1
+        double piv = sw ? sub : a0;
         if (fabs(piv) < tiny) piv = piv < 0.0 ? -tiny : tiny;
-        ua[i] = 1.0 / piv;
+        const double inv = 1.0 / piv, ml = (sw ? a0 : sub) * inv;
+        const double u1 = sw ? dn : b0, u2 = sw ? en : 0.0;
+        ua[i] = inv;
+        ub[i] = make_double2(u1, u2);
+        mf[i] = make_double2(ml, sw ? 1.0 : 0.0);
+        a0 = fma(-ml, u1, sw ? b0 : dn);
+        b0 = sw ? -ml * en : en;
       }
       double piv = a0;
       if (fabs(piv) < tiny) piv = piv < 0.0 ? -tiny : tiny;
       ua[n - 1] = 1.0 / piv;
+      ub[n - 1] = make_double2(0.0, 0.0);
     }
-    for (int i = lane; i < n; i += 32) y[i] = 1.0 + 0.5 * sin(0.7 * (i + 1) + 0.3 * (m + 1));
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+      const double ia = ua[i];
+      const double2 u = ub[i];
+      ub[i] = make_double2(-u.x * ia, -u.y * ia);
+      // start vector: fixed, positive, no pattern
+      const unsigned h = (unsigned)(i + 1) * 0x9E3779B1u ^ (unsigned)(m + 1) * 0x85EBCA77u;
+      y[i] = (1.0 + 0.5 * (double)((h ^ h >> 15) & 0xffffu) * (1.0 / 65536.0)) * ia;
+    }
     __syncwarp();
     for (int it = 0; it < 2; ++it) {
       if (lane == 0) {
-        for (int i = 0; i + 1 < n; ++i) {   // y <- L^-1 P y
-          if (fl[i] != 0.0) {
-            const double t = y[i];
-            y[i] = y[i + 1];
-            y[i + 1] = t - mu[i] * y[i];
-          } else {
-            y[i + 1] -= mu[i] * y[i];
+        if (it > 0) {   // y <- L^-1 P y, each row over its pivot
+          double c = y[0];
+          int i = 0;
+          for (; i + 4 < n; i += 4) {
+            double yn[4], ia[4];
+            double2 f[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              yn[u] = y[i + 1 + u];
+              f[u] = mf[i + u];
+              ia[u] = ua[i + u];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const bool sw = f[u].y != 0.0;
+              const double top = sw ? yn[u] : c, bot = sw ? c : yn[u];
+              y[i + u] = top * ia[u];
+              c = fma(-f[u].x, top, bot);
+            }
+          }
+          for (; i + 1 < n; ++i) {
+            const double yn = y[i + 1];
+            const bool sw = mf[i].y != 0.0;
+            const double top = sw ? yn : c, bot = sw ? c : yn;
+            y[i] = top * ua[i];
+            c = fma(-mf[i].x, top, bot);
+          }
+          y[n - 1] = c * ua[n - 1];
+        }
+        double x1 = 0.0, x2 = 0.0;   // U x = y
+        int i = n - 1;
+        for (; i >= 3; i -= 4) {
+          double yv[4];
+          double2 f[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            yv[u] = y[i - u];
+            f[u] = ub[i - u];
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const double x = fma(f[u].x, x1, fma(f[u].y, x2, yv[u]));
+            y[i - u] = x;
+            x2 = x1;
+            x1 = x;
           }
         }
-        for (int i = n - 1; i >= 0; --i) {   // U x = y
-          double s2 = y[i];
-          if (i + 1 < n) s2 -= ub[i] * y[i + 1];
-          if (i + 2 < n) s2 -= uc[i] * y[i + 2];
-          y[i] = s2 * ua[i];
+        for (; i >= 0; --i) {
+          const double x = fma(ub[i].x, x1, fma(ub[i].y, x2, y[i]));
+          y[i] = x;
+          x2 = x1;
+          x1 = x;
         }
       }
       __syncwarp();
@@ -512,85 +712,107 @@ k_symeig_vectors_b(const SymEigJob *__restrict__ jobs) {
 }
 
 // ---- 4. back-transformation z = H_0 ... H_{n-3} y ----------------------------
-constexpr int kBtBlock = 16;                        // reflectors staged per round
-constexpr int kBtPerLane = (kSymEigMaxN + 31) / 32;  // vector elements per lane
-
-__host__ __device__ inline size_t symeig_bt_smem_bytes(int n) {
-  return sizeof(double) * ((size_t)kBtBlock * n + kBtBlock);
-}
-
+// One CTA of 128 threads per eigenvector, thread = row mod 128 (RL rows each),
+// the vector in registers.  The reflectors come in blocks of 8: the 8 dot
+// products v_r^T y are independent, the coefficients follow through the
+// block's triangular factor (symeig_block_factor), and the next block is
+// loaded meanwhile, so a block costs one reduction and one barrier where
+// reflector after reflector cost eight reductions.  Whole eigensolve: 220 -> 189 us
+// at n = 100, 799 -> 656 us at n = 300 against one warp per vector with the
+// reflectors in shared memory.
+constexpr int kBtThreads = 128;
+template <int RL>
 __device__ __forceinline__ void
-symeig_backtransform_body(int n, int k, const double *__restrict__ work,
-                       const double *__restrict__ w, double *__restrict__ Z, int ldz,
-                       int *info) {
-  extern __shared__ double sm[];
-  double *R = sm;                      // [kBtBlock][n]: v of H_c, zero above row c+1
-  double *tt = sm + (size_t)kBtBlock * n;
+symeig_backtransform_rows(int m, int n, const double *__restrict__ work,
+                          const double *__restrict__ w, double *__restrict__ Z, int ldz,
+                          int *info) {
+  constexpr int B = kBtBlock, NW = kBtThreads / 32;
+  __shared__ double part[2][NW][B];
   const SymEigWork g(const_cast<double *>(work), n);
-  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int m = blockIdx.x * kSymEigWarps + wl;
-  const bool live = m < k;
-  double y[kBtPerLane];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double y[RL], v[B][RL], nx[B][RL];
 #pragma unroll
-  for (int t = 0; t < kBtPerLane; ++t) {
-    const int i = lane + 32 * t;
-    y[t] = live && i < n ? g.vec[(size_t)m * n + i] : 0.0;
+  for (int t = 0; t < RL; ++t) {
+    const int i = tid + kBtThreads * t;
+    y[t] = i < n ? g.vec[(size_t)m * n + i] : 0.0;
   }
-  // H_{n-3} first, H_0 last
-  for (int c1 = n - 3; c1 >= 0; c1 -= kBtBlock) {
-    const int nr = min(kBtBlock, c1 + 1);   // reflectors c1, c1-1, ..., c1-nr+1
-    __syncthreads();
-    for (int e = threadIdx.x; e < nr * n; e += blockDim.x) {
-      const int r = e / n, i = e - r * n, c = c1 - r;
-      R[e] = i <= c ? 0.0 : (i == c + 1 ? 1.0 : g.ap[pk_idx(i, c, n)]);
+  const int nb = symeig_bt_blocks(n);
+  double frow[B], fnx[B];   // row lane % B of the block's factor
+  auto load = [&](int b, double (&x)[B][RL], double (&f)[B]) {
+    const int c1 = n - 3 - B * b;
+#pragma unroll
+    for (int r = 0; r < B; ++r) {
+#pragma unroll
+      for (int t = 0; t < RL; ++t) {
+        const int i = tid + kBtThreads * t;
+        x[r][t] = i < n ? symeig_v(g, i, c1 - r, n) : 0.0;
+      }
+      f[r] = g.bt[((size_t)b * B + lane % B) * B + r];
     }
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) tt[r] = g.tau[c1 - r];
+  };
+  if (nb > 0) load(0, nx, fnx);
+  for (int b = 0; b < nb; ++b) {
+#pragma unroll
+    for (int r = 0; r < B; ++r) {
+      frow[r] = fnx[r];
+#pragma unroll
+      for (int t = 0; t < RL; ++t) v[r][t] = nx[r][t];
+    }
+    if (b + 1 < nb) load(b + 1, nx, fnx);
+    double s[B];
+#pragma unroll
+    for (int r = 0; r < B; ++r) {
+      s[r] = 0.0;
+#pragma unroll
+      for (int t = 0; t < RL; ++t) s[r] = fma(v[r][t], y[t], s[r]);
+    }
+    const int q = warp_sums(s, lane);
+    if (lane % (32 / B) == 0) part[b & 1][warp][q] = s[0];
     __syncthreads();
-    if (!live) continue;
-    for (int r = 0; r < nr; ++r) {
-      const double tc = tt[r];
-      if (tc == 0.0) continue;
-      const double *vr = R + (size_t)r * n;
-      double dot = 0.0;
+    double dot = 0.0, f = 0.0;   // dot product lane % B, coefficient lane % B
 #pragma unroll
-      for (int t = 0; t < kBtPerLane; ++t) {
-        const int i = lane + 32 * t;
-        if (i < n) dot += vr[i] * y[t];
-      }
-      for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      const double f = tc * dot;
+    for (int u = 0; u < NW; ++u) dot += part[b & 1][u][lane % B];
 #pragma unroll
-      for (int t = 0; t < kBtPerLane; ++t) {
-        const int i = lane + 32 * t;
-        if (i < n) y[t] -= f * vr[i];
-      }
+    for (int r = 0; r < B; ++r) f = fma(frow[r], __shfl_sync(0xffffffffu, dot, r), f);
+#pragma unroll
+    for (int r = 0; r < B; ++r) {
+      const double fr = __shfl_sync(0xffffffffu, f, r);
+#pragma unroll
+      for (int t = 0; t < RL; ++t) y[t] = fma(-fr, v[r][t], y[t]);
     }
   }
-  if (!live) return;
-  bool bad = false;
+  bool bad = !isfinite(w[m]);
 #pragma unroll
-  for (int t = 0; t < kBtPerLane; ++t) {
-    const int i = lane + 32 * t;
+  for (int t = 0; t < RL; ++t) {
+    const int i = tid + kBtThreads * t;
     if (i < n) {
       bad |= !isfinite(y[t]);
       Z[i + (size_t)ldz * m] = y[t];
     }
   }
-  if (lane == 0) bad |= !isfinite(w[m]);
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(info, 1);
 }
 
-__global__ void __launch_bounds__(kSymEigWarps * 32)
-k_symeig_backtransform(int n, int k, const double *__restrict__ work,
-                       const double *__restrict__ w, double *__restrict__ Z, int ldz,
-                       int *info) {
-  symeig_backtransform_body(n, k, work, w, Z, ldz, info);
+__device__ __forceinline__ void
+symeig_backtransform_body(int m, int n, const double *__restrict__ work,
+                          const double *__restrict__ w, double *__restrict__ Z, int ldz,
+                          int *info) {
+  if (n <= kBtThreads) symeig_backtransform_rows<1>(m, n, work, w, Z, ldz, info);
+  else if (n <= 2 * kBtThreads) symeig_backtransform_rows<2>(m, n, work, w, Z, ldz, info);
+  else symeig_backtransform_rows<3>(m, n, work, w, Z, ldz, info);
+}
+static_assert(kSymEigMaxN <= 3 * kBtThreads, "rows per thread");
+
+__global__ void __launch_bounds__(kBtThreads)
+k_symeig_backtransform(int n, const double *__restrict__ work, const double *__restrict__ w,
+                       double *__restrict__ Z, int ldz, int *info) {
+  symeig_backtransform_body(blockIdx.x, n, work, w, Z, ldz, info);
 }
 
-__global__ void __launch_bounds__(kSymEigWarps * 32)
+__global__ void __launch_bounds__(kBtThreads)
 k_symeig_backtransform_b(const SymEigJob *__restrict__ jobs) {
   const SymEigJob j = jobs[blockIdx.y];
-  symeig_backtransform_body(j.n, j.k, j.work, j.w, j.Z, j.ldz, j.info);
+  if (blockIdx.x < j.k) symeig_backtransform_body(blockIdx.x, j.n, j.work, j.w, j.Z, j.ldz, j.info);
 }
 
 // host launcher: n <= kSymEigMaxN, k <= n; work: symeig_work_doubles(n, k)
@@ -598,51 +820,38 @@ inline void symeig_small(cudaStream_t s, const double *A, int lda, int n, int k,
                          double *Z, int ldz, double *work, int *info) {
   if (n < 1 || n > kSymEigMaxN || k < 1 || k > n)
     throw Error{STD2G_EINVAL, "symeig_small: size out of range"};
-  const int C = symeig_cluster_ctas(n);
-  // the attribute is the same for every call (contexts on other host threads
-  // launch the same kernel concurrently), the launch takes what n needs
-  const int tsm = (int)symeig_smem_bytes(n, C);
-  if (C == 4) {
-    S2G_CUDA(cudaFuncSetAttribute(k_symeig_tridiag<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)symeig_smem_bytes(kSymEigMaxN, 4)));
-    S2G_LAUNCH(k_symeig_tridiag<4>, 4, kTridiagThreads, tsm, s, A, lda, n, work);
-  } else {
-    S2G_CUDA(cudaFuncSetAttribute(k_symeig_tridiag<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)symeig_smem_bytes(kSymEigMaxN, 8)));
-    S2G_LAUNCH(k_symeig_tridiag<8>, 8, kTridiagThreads, tsm, s, A, lda, n, work);
-  }
+  symeig_tridiag_shape(n, [&](int, auto shape) {
+    using Shape = decltype(shape);
+    launch_cluster(k_symeig_tridiag<Shape>, dim3(Shape::C), kTridiagThreads, Shape::C, s, A, lda,
+                   n, work);
+  });
   S2G_CUDA(cudaFuncSetAttribute(k_symeig_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)symeig_vec_smem_bytes(kSymEigMaxN)));
   const int nb = (k + kSymEigWarps - 1) / kSymEigWarps;
-  S2G_LAUNCH(k_symeig_values, k, kValThreads, symeig_val_smem_bytes(n), s, n, work, w);
+  S2G_LAUNCH(k_symeig_values, k + symeig_bt_blocks(n), kValThreads, symeig_val_smem_bytes(n), s, n,
+             k, work, w);
   S2G_LAUNCH(k_symeig_vectors, nb, kSymEigWarps * 32, symeig_vec_smem_bytes(n), s, n, k, work, w);
-  S2G_LAUNCH(k_symeig_backtransform, nb, kSymEigWarps * 32, symeig_bt_smem_bytes(n), s, n, k,
-             work, w, Z, ldz, info);
+  S2G_LAUNCH(k_symeig_backtransform, k, kBtThreads, 0, s, n, work, w, Z, ldz, info);
 }
 
 // Batched launcher: the problems of `jobs` (each n <= kSymEigMaxN, 1 <= k <= n)
-// in four launches for all of them, plus one tridiagonalisation launch per
-// cluster size.  The job table goes to `dj` (same stream: a later upload
+// in three launches for all of them, plus one tridiagonalisation launch per
+// shape (symeig_tridiag_shape).  The job table goes to `dj` (same stream: a later upload
 // waits for these kernels), from `stage` when given.
 inline void symeig_small_batched(cudaStream_t s, const std::vector<SymEigJob> &jobs,
                                  DBuf<SymEigJob> &dj, PinnedArena *stage = nullptr) {
   if (jobs.empty()) return;
   std::vector<SymEigJob> ord;
-  int n4 = 0, nmax = 0, kmax = 0;
-  size_t sm4 = 0, sm8 = 0;
-  for (int pass = 0; pass < 2; ++pass)
+  int count[kTridiagShapes] = {0}, nmax = 0, kmax = 0;
+  for (int shape = 0; shape < kTridiagShapes; ++shape)
     for (const SymEigJob &j : jobs) {
       if (j.n < 1 || j.n > kSymEigMaxN || j.k < 1 || j.k > j.n)
         throw Error{STD2G_EINVAL, "symeig_small_batched: size out of range"};
-      const int C = symeig_cluster_ctas(j.n);
-      if ((pass == 0) != (C == 4)) continue;
+      int mine = 0;
+      symeig_tridiag_shape(j.n, [&](int q, auto) { mine = q; });
+      if (mine != shape) continue;
       ord.push_back(j);
-      if (C == 4) {
-        ++n4;
-        sm4 = std::max(sm4, symeig_smem_bytes(j.n, 4));
-      } else {
-        sm8 = std::max(sm8, symeig_smem_bytes(j.n, 8));
-      }
+      ++count[shape];
       nmax = std::max(nmax, j.n);
       kmax = std::max(kmax, j.k);
     }
@@ -650,24 +859,20 @@ inline void symeig_small_batched(cudaStream_t s, const std::vector<SymEigJob> &j
   SymEigJob *d = dj.ensure(ord.size());
   const void *h = stage ? stage->put(ord.data(), sizeof(SymEigJob) * ord.size()) : ord.data();
   S2G_CUDA(cudaMemcpyAsync(d, h, sizeof(SymEigJob) * ord.size(), cudaMemcpyHostToDevice, s));
-  if (n4 > 0) {
-    S2G_CUDA(cudaFuncSetAttribute(k_symeig_tridiag_b<4>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)symeig_smem_bytes(kSymEigMaxN, 4)));
-    S2G_LAUNCH(k_symeig_tridiag_b<4>, dim3(4, n4), kTridiagThreads, sm4, s, d);
-  }
-  if (nj > n4) {
-    S2G_CUDA(cudaFuncSetAttribute(k_symeig_tridiag_b<8>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)symeig_smem_bytes(kSymEigMaxN, 8)));
-    S2G_LAUNCH(k_symeig_tridiag_b<8>, dim3(8, nj - n4), kTridiagThreads, sm8, s, d + n4);
-  }
+  for (int shape = 0, at = 0; shape < kTridiagShapes; at += count[shape++])
+    if (count[shape] > 0)
+      symeig_tridiag_shape(ord[at].n, [&](int, auto sh) {
+        using Shape = decltype(sh);
+        launch_cluster(k_symeig_tridiag_b<Shape>, dim3(Shape::C, count[shape]), kTridiagThreads,
+                       Shape::C, s, (const SymEigJob *)(d + at));
+      });
   S2G_CUDA(cudaFuncSetAttribute(k_symeig_vectors_b, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)symeig_vec_smem_bytes(kSymEigMaxN)));
   const dim3 g((kmax + kSymEigWarps - 1) / kSymEigWarps, nj);
-  S2G_LAUNCH(k_symeig_values_b, dim3(kmax, nj), kValThreads, symeig_val_smem_bytes(nmax), s, d);
+  S2G_LAUNCH(k_symeig_values_b, dim3(kmax + symeig_bt_blocks(nmax), nj), kValThreads,
+             symeig_val_smem_bytes(nmax), s, d);
   S2G_LAUNCH(k_symeig_vectors_b, g, kSymEigWarps * 32, symeig_vec_smem_bytes(nmax), s, d);
-  S2G_LAUNCH(k_symeig_backtransform_b, g, kSymEigWarps * 32, symeig_bt_smem_bytes(nmax), s, d);
+  S2G_LAUNCH(k_symeig_backtransform_b, dim3(kmax, nj), kBtThreads, 0, s, d);
 }
 
 }  // namespace std2g
