@@ -498,9 +498,13 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
                                     m, theta, work, lwork, einfo));
     }
     clk.tick(2);
-    // Ritz vectors X = V Y_k, residuals R = W Y_k - X theta
-    (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, k, m, &one, V, n, Hs, m, &zero, X, n));
-    (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, k, m, &one, W, n, Hs, m, &zero, R, n));
+    // Ritz vectors X = V Y_k, residuals R = W Y_k - X theta: the two products in
+    // one launch (members V, W at a fixed distance)
+    const auto apart = [](const double *a, const double *b) {
+      return (int64_t)((intptr_t)b - (intptr_t)a) / (int64_t)sizeof(double);
+    };
+    dw.dg->run(s, false, false, n, k, m, 1.0, V, n, apart(V, W), Hs, m, 0, 0.0, X, n, apart(X, R),
+               2);
     {
       double *part = dw.part.ensure((size_t)k * kColSplit);
       S2G_LAUNCH(k_dav_resid, dim3(kColSplit, (unsigned)k), 256, 0, s, R, X, theta, n, part);

@@ -54,6 +54,10 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool o
                "r"(ok ? 8 : 0)
                : "memory");
 }
+__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -83,54 +87,56 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
   auto As = [&](int st) { return smem_d + (size_t)st * STAGE; };
   auto Bs = [&](int st) { return smem_d + (size_t)st * STAGE + TILE_A; };
 
-  // issue the copies of the K tile starting at k0 into stage st; element q of
-  // this thread is idx = tid + 128 q, so along the tile's slow dimension it
-  // moves by a fixed stride and one source pointer per operand serves all q
-  auto issue = [&](int st, int k0) {
+  // Copies of one K tile into a stage: element q of this thread is tid + 128 q,
+  // each with its own source pointer that moves on by one K tile per call.  Rows
+  // past M (columns past N) read the last valid one instead: they only reach
+  // outputs that are not stored, so a full K tile needs no test at all; the
+  // last, partial K tile is filled with zeros past ke.  With one CTA on an SM
+  // a K tile costs what its instructions take to issue (272 of them per warp
+  // with tests and addresses formed per copy took 1040 cycles, twice the 512
+  // of the DMMAs).
+  constexpr int QA = TILE_A / THREADS, QB = TILE_B / THREADS, KS = THREADS / BN;
+  const double *pa[QA], *pb[QB];
+  const int ka = TA ? tid & 15 : tid >> 6, kbq = TB ? tid / BN : tid & 15;
+#pragma unroll
+  for (int q = 0; q < QA; ++q)
+    pa[q] = TA ? A + (kb + ka) + (int64_t)min(m0 + (tid >> 4) + 8 * q, M - 1) * lda
+               : A + min(m0 + (tid & 63), M - 1) + (int64_t)(kb + ka + 2 * q) * lda;
+#pragma unroll
+  for (int q = 0; q < QB; ++q)
+    pb[q] = TB ? B + min(n0 + (tid & (BN - 1)), N - 1) + (int64_t)(kb + kbq + KS * q) * ldb
+               : B + (kb + kbq) + (int64_t)min(n0 + (tid >> 4) + 8 * q, N - 1) * ldb;
+  const int64_t sa = TA ? BK : BK * lda, sb = TB ? BK * ldb : BK;
+  auto issue = [&](int st, int left) {   // left: K elements from the tile's start to ke
     double *a = As(st), *b = Bs(st);
-    if (!TA) {   // m fastest: m = tid % 64, k = tid / 64 + 2 q
-      const int m = tid & 63, kq = tid >> 6;
-      const bool okm = m0 + m < M;
-      const double *src = A + (m0 + m) + (int64_t)(k0 + kq) * lda;
+    auto dst_a = [&](int q) {
+      return TA ? a + pos_kfast((tid >> 4) + 8 * q, ka) : a + pos_mfast<BM>(ka + 2 * q, tid & 63);
+    };
+    auto dst_b = [&](int q) {
+      return TB ? b + pos_mfast<BN>(kbq + KS * q, tid & (BN - 1))
+                : b + pos_kfast((tid >> 4) + 8 * q, kbq);
+    };
+    if (left >= BK) {
 #pragma unroll
-      for (int q = 0; q < TILE_A / THREADS; ++q) {
-        const int k = kq + 2 * q;
-        const bool ok = okm && k0 + k < ke;
-        cp_async8(a + pos_mfast<BM>(k, m), ok ? src + (int64_t)(2 * q) * lda : A, ok);
+      for (int q = 0; q < QA; ++q) cp_async8(dst_a(q), pa[q]);
+#pragma unroll
+      for (int q = 0; q < QB; ++q) cp_async8(dst_b(q), pb[q]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < QA; ++q) {
+        const bool ok = ka + (TA ? 0 : 2 * q) < left;
+        cp_async8(dst_a(q), ok ? pa[q] : A, ok);
       }
-    } else {     // k fastest: k = tid % 16, m = tid / 16 + 8 q
-      const int k = tid & 15, mq = tid >> 4;
-      const bool okk = k0 + k < ke;
-      const double *src = A + (k0 + k) + (int64_t)(m0 + mq) * lda;
 #pragma unroll
-      for (int q = 0; q < TILE_A / THREADS; ++q) {
-        const int m = mq + 8 * q;
-        const bool ok = okk && m0 + m < M;
-        cp_async8(a + pos_kfast(m, k), ok ? src + (int64_t)(8 * q) * lda : A, ok);
-      }
-    }
-    if (!TB) {   // k fastest: k = tid % 16, n = tid / 16 + 8 q
-      const int k = tid & 15, nq = tid >> 4;
-      const bool okk = k0 + k < ke;
-      const double *src = B + (k0 + k) + (int64_t)(n0 + nq) * ldb;
-#pragma unroll
-      for (int q = 0; q < TILE_B / THREADS; ++q) {
-        const int n = nq + 8 * q;
-        const bool ok = okk && n0 + n < N;
-        cp_async8(b + pos_kfast(n, k), ok ? src + (int64_t)(8 * q) * ldb : B, ok);
-      }
-    } else {     // n fastest: n = tid % BN, k = tid / BN + (128 / BN) q
-      constexpr int KS = THREADS / BN;
-      const int n = tid & (BN - 1), kq = tid / BN;
-      const bool okn = n0 + n < N;
-      const double *src = B + (n0 + n) + (int64_t)(k0 + kq) * ldb;
-#pragma unroll
-      for (int q = 0; q < TILE_B / THREADS; ++q) {
-        const int k = kq + KS * q;
-        const bool ok = okn && k0 + k < ke;
-        cp_async8(b + pos_mfast<BN>(k, n), ok ? src + (int64_t)(KS * q) * ldb : B, ok);
+      for (int q = 0; q < QB; ++q) {
+        const bool ok = kbq + (TB ? KS * q : 0) < left;
+        cp_async8(dst_b(q), ok ? pb[q] : B, ok);
       }
     }
+#pragma unroll
+    for (int q = 0; q < QA; ++q) pa[q] += sa;
+#pragma unroll
+    for (int q = 0; q < QB; ++q) pb[q] += sb;
   };
 
 #pragma unroll
@@ -141,7 +147,7 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
   const int nt = ke > kb ? (ke - kb + BK - 1) / BK : 0;
 #pragma unroll
   for (int p = 0; p < STAGES - 1; ++p) {
-    if (p < nt) issue(p, kb + p * BK);
+    if (p < nt) issue(p, ke - kb - p * BK);
     cp_async_commit();
   }
   for (int it = 0; it < nt; ++it) {
@@ -149,7 +155,7 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
     __syncthreads();
     {
       const int nx = it + STAGES - 1;
-      if (nx < nt) issue(nx % STAGES, kb + nx * BK);
+      if (nx < nt) issue(nx % STAGES, ke - kb - nx * BK);
       cp_async_commit();
     }
     const double *a = As(it % STAGES), *b = Bs(it % STAGES);
@@ -241,18 +247,38 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : (BN == 64 ? 3 : 2)
   }
 }
 
+// s + w[0] + w[mn] + ... + w[(ks-1) mn], added in that order; the loads go out 16
+// at a time, so that the sum costs a few memory latencies instead of ks / 4
+__device__ __forceinline__ double split_sum(const double *__restrict__ w, int64_t mn, int ks) {
+  double s = 0.0;
+  int q = 0;
+  for (; q + 16 <= ks; q += 16) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = w[(q + u) * mn];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s += v[u];
+  }
+  double v[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) v[u] = q + u < ks ? w[(q + u) * mn] : 0.0;
+#pragma unroll
+  for (int u = 0; u < 16; ++u)
+    if (q + u < ks) s += v[u];
+  return s;
+}
+
 // C = alpha sum_s work[b][s] + beta C, splits added in order 0, 1, ...
-__global__ void k_dgemm_reduce(int M, int N, int batch, int ksplit, double alpha,
-                               const double *__restrict__ work, double beta,
-                               double *__restrict__ C, int64_t ldc, int64_t sC) {
+constexpr int kReduceThreads = 64;   // few outputs: small blocks reach more SMs
+__global__ void __launch_bounds__(kReduceThreads)
+k_dgemm_reduce(int M, int N, int batch, int ksplit, double alpha, const double *__restrict__ work,
+               double beta, double *__restrict__ C, int64_t ldc, int64_t sC) {
   const int64_t mn = (int64_t)M * N, total = mn * batch;
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total;
        x += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = x / mn, r = x - b * mn;
     const int64_t col = r / M, row = r - col * M;
-    const double *w = work + b * ksplit * mn + r;
-    double s = 0.0;
-    for (int q = 0; q < ksplit; ++q) s += w[q * mn];
+    const double s = split_sum(work + b * ksplit * mn + r, mn, ksplit);
     double *p = C + b * sC + row + col * ldc;
     *p = beta == 0.0 ? alpha * s : alpha * s + beta * *p;
   }
@@ -333,9 +359,7 @@ __global__ void k_dgemm_grouped_reduce(const DgProblem *__restrict__ probs,
   const int64_t mn = (int64_t)pr.M * pr.N;
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < mn;
        x += (int64_t)gridDim.x * blockDim.x) {
-    const double *w = work + pr.woff + x;
-    double s = 0.0;
-    for (int q = 0; q < pr.ks; ++q) s += w[q * mn];
+    const double s = split_sum(work + pr.woff + x, mn, pr.ks);
     const int64_t col = x / pr.M, row = x - col * pr.M;
     double *p = pr.C + row + col * pr.ldc;
     *p = pr.beta == 0.0 ? pr.alpha * s : pr.alpha * s + pr.beta * *p;
@@ -444,6 +468,58 @@ struct Dgemm {
     }
   }
 
+  // this instance's launches have set the kernels' shared-memory limits (a
+  // host call per product otherwise; an instance serves one device)
+  bool smem_set[2][2][3] = {};
+  // K splits by wave counts only (see pick_split): the sTD-DFT subspace
+  // iteration, whose results must not depend on the order of these sums
+  bool wave_splits = false;
+
+  // Tile width and split count of one product, from the time of the busiest SM
+  // in cycles.  A CTA's K step of 16 is bound by the DMMA rate (64 FMA per SM
+  // and cycle: 16 BN cycles; measured 570 / 1024 / 2010 for BN = 32 / 64 / 128),
+  // so what counts is the sum over the CTAs that share the busiest SM, not how
+  // many of them are resident: 300 CTAs on 148 SMs take half as long again as
+  // 296.  A CTA alone on its SM has one warp per scheduler, which issues a DMMA
+  // only every ~30 cycles instead of 16 (47 % of the rate in the profile of a
+  // 150 x 25 x 21217 product), so it costs as much as nearly two.
+  // Each batch of resident CTAs adds ~2000 cycles to fill its pipeline and
+  // store; a split adds a second launch (~9000) and its partial tiles' traffic
+  // (~2000 bytes per cycle); each is at least 64 long.
+  // wave_splits: waves of four 64 x 32, three 64 x 64 or two 64 x 128 CTAs per
+  // SM, the fewest K steps of the busiest SM (splits at least 256 long, weighted
+  // 3 %), a step of a full wave taking 0.74 / 1 / 1.31.
+  void pick_split(int m, int n, int k, int batch, int &bn, int &ksplit) const {
+    double best = 0.0;
+    const int64_t kk = std::max(k, 1);
+    const int kmax = wave_splits ? (int)std::max<int64_t>(1, std::min<int64_t>(64, k / 256))
+                                 : (int)std::max<int64_t>(1, std::min<int64_t>(2 * nsm, k / 64));
+    for (int w : {32, 64, 128}) {
+      const int64_t ctas = div_up(m, dg::BM) * div_up(n, w) * (int64_t)batch;
+      const int64_t resident = w == 32 ? 4 : (w == 64 ? 3 : 2), slots = resident * nsm;
+      const double wave_step = w == 32 ? 0.74 : (w == 64 ? 1.0 : 1.31);
+      const double step = w == 32 ? 570.0 : (w == 64 ? 1024.0 : 2010.0);
+      for (int ks = 1; ks <= kmax; ++ks) {
+        const int64_t kt = div_up(div_up(kk, ks), dg::BK);
+        double cost;
+        if (wave_splits) {
+          cost = (double)(div_up(ctas * ks, slots) * kt) * wave_step * (ks > 1 ? 1.03 : 1.0);
+        } else {
+          const int64_t q = div_up(ctas * ks, nsm);   // CTAs on the busiest SM
+          cost = (double)kt * step * (q == 1 ? 1.85 : (double)q) +
+                 2000.0 * (double)div_up(q, resident);
+          if (ks > 1) cost += 9000.0 + (double)ks * batch * m * (double)n * 16.0 / 2000.0;
+          if (ctas >= 4 * slots && ks > 1) continue;   // many waves: nothing to split for
+        }
+        if (best == 0.0 || cost < best) {
+          best = cost;
+          bn = w;
+          ksplit = ks;
+        }
+      }
+    }
+  }
+
   // the argument order of cublasDgemm (alpha / beta by pointer, host values)
   void gemm(cudaStream_t s, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k,
             const double *alpha, const double *A, int64_t lda, const double *B, int64_t ldb,
@@ -479,29 +555,8 @@ struct Dgemm {
                                              (int)ldb, sB, &beta, C, (int)ldc, sC, batch));
       return;
     }
-    // tile width and split-K: CTAs run in waves (four 64 x 32, three 64 x 64
-    // or two 64 x 128 CTAs per SM); for each width pick the split count with
-    // the fewest K steps on the busiest SM (each split at least 256 long; a
-    // split adds its workspace pass, weighted 3 %), then the width with the
-    // lower cost (the time of one K step of a full wave, measured on B200: a
-    // 64 x 32 / 64 x 128 wave step takes 0.74 / 1.31 of a 64 x 64 one)
     int bn = 64, ksplit = 1;
-    double best = 0.0;
-    const int kmax = (int)std::max<int64_t>(1, std::min<int64_t>(64, k / 256));
-    for (int w : {32, 64, 128}) {
-      const int64_t ctas = div_up(m, dg::BM) * div_up(n, w) * (int64_t)batch;
-      const int64_t slots = (w == 32 ? 4 : (w == 64 ? 3 : 2)) * (int64_t)nsm;
-      const double per_step = w == 32 ? 0.74 : (w == 64 ? 1.0 : 1.31);
-      for (int ks = 1; ks <= kmax; ++ks) {
-        const int64_t steps = div_up(ctas * ks, slots) * div_up(div_up(std::max(k, 1), ks), dg::BK);
-        const double cost = (double)steps * per_step * (ks > 1 ? 1.03 : 1.0);
-        if (best == 0.0 || cost < best) {
-          best = cost;
-          bn = w;
-          ksplit = ks;
-        }
-      }
-    }
+    pick_split(m, n, k, batch, bn, ksplit);
     const int tiles = (int)(div_up(m, dg::BM) * div_up(n, bn));
     int kchunk = (int)div_up(div_up(std::max(k, 1), ksplit), dg::BK) * dg::BK;
     ksplit = (int)div_up(std::max(k, 1), kchunk);
@@ -511,9 +566,12 @@ struct Dgemm {
     const dim3 grid(tiles, batch * ksplit);
 #define S2G_DGEMM(TA_, TB_, BN_)                                                              \
   do {                                                                                        \
-    S2G_CUDA(cudaFuncSetAttribute(k_dgemm<TA_, TB_, BN_>,                                     \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                \
-                                  dg::smem_bytes<BN_>()));                                    \
+    bool &ready = smem_set[TA_][TB_][BN_ / 64];                                               \
+    if (!ready)                                                                               \
+      S2G_CUDA(cudaFuncSetAttribute(k_dgemm<TA_, TB_, BN_>,                                   \
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,              \
+                                    dg::smem_bytes<BN_>()));                                  \
+    ready = true;                                                                             \
     S2G_LAUNCH((k_dgemm<TA_, TB_, BN_>), grid, dg::THREADS, dg::smem_bytes<BN_>(), s, m, n, k, \
                alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, ksplit, kchunk, wk, tri);     \
   } while (0)
@@ -537,8 +595,9 @@ struct Dgemm {
     ++launches;
     if (ksplit > 1) {
       const int64_t total = (int64_t)m * n * batch;
-      const int g = (int)std::min<int64_t>(div_up(total, 256), (int64_t)nsm * 8);
-      S2G_LAUNCH(k_dgemm_reduce, g, 256, 0, s, m, n, batch, ksplit, alpha, wk, beta, C, ldc, sC);
+      const int g = (int)std::min<int64_t>(div_up(total, kReduceThreads), (int64_t)nsm * 32);
+      S2G_LAUNCH(k_dgemm_reduce, g, kReduceThreads, 0, s, m, n, batch, ksplit, alpha, wk, beta, C,
+                 ldc, sC);
       ++launches;
     }
   }

@@ -855,6 +855,8 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
   c.tc_launches = 0;
   c.dg.reset();
   c.mftc.side.dg.reset();
+  // iterative sTD-DFT roots keep the products' summation order fixed
+  c.dg.wave_splits = p.rpa && !resp && p.nroots > 0;
   c.mixed.rechecked = 0;
   c.mixed.ed_bound_max = 0.0;   // the FP64 PT path lowers the diagonal in FP64
   c.dav_iters = 0;
