@@ -68,6 +68,26 @@ extern std::atomic<int64_t> g_launches;
     S2G_CUDA(cudaGetLastError());                                                \
   } while (0)
 
+// Launch in thread-block clusters of the given size (1 x 1 x 1: none)
+template <class... KArgs, class... Args>
+inline void launch_cluster(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem,
+                           dim3 cluster, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cluster.x;
+  at.val.clusterDim.y = cluster.y;
+  at.val.clusterDim.z = cluster.z;
+  cfg.attrs = &at;
+  cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 1 : 0;
+  S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  ++g_launches;
+}
+
 // Device buffer that only grows; reused across solves of one context.
 template <typename T>
 struct DBuf {

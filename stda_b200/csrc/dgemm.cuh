@@ -2,20 +2,22 @@
 // column-major, op = N or T, optionally batched with fixed strides.
 //
 // B200 has no FP64 kind of tcgen05; its FP64 tensor path is the warp-level
-// DMMA (mma.sync m8n8k4 .f64).  Each CTA (4 warps) computes a 64 x 128 tile
-// of C over a K range in steps of 16: the A (64 x 16) and B (16 x 128) tiles
+// DMMA (mma.sync m8n8k4 .f64).  Each CTA (4 warps) computes a 64 x BN tile (BN =
+// 32 or 64) of C over a K range in steps of 16: the A (64 x 16) and B (16 x BN) tiles
 // arrive by 8-byte cp.async in a 4-stage shared-memory ring (three tiles in
 // flight while one is multiplied), kept in the global layout's fast order and
 // XOR-swizzled so that the fragment reads are conflict-free, and each warp
-// owns a 32 x 64 sub-tile = 4 x 8 DMMA tiles (64 accumulators per thread, so
-// that an accumulator is reused only every 32 DMMAs).
+// owns a 32 x BN/2 sub-tile = 4 x BN/16 DMMA tiles.
 //
-// Tall-skinny products (the Davidson projections V^T W: 300 x 75 outputs over
-// 5e4-long sums) split K across CTAs.  The partial tiles go to a workspace and
-// a second kernel adds them in a fixed order, so every result is bit-for-bit
-// reproducible from run to run (no atomics).  With beta = 0, C is not read.
+// Small products and tall-skinny ones (the Davidson projections V^T W: 300 x 75
+// outputs over 5e4-long sums) split K across the CTAs of a cluster, which add
+// their tiles through distributed shared memory, and across clusters, whose
+// partial tiles go to a workspace where the last one to arrive adds them.  Both
+// sums run in the order of the splits, so every result is bit-for-bit
+// reproducible from run to run.  With beta = 0, C is not read.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cublas_v2.h>
 
 #include <vector>
@@ -28,7 +30,7 @@ namespace dg {
 constexpr int BM = 64, BK = 16, THREADS = 128, STAGES = 4;
 constexpr int TILE_A = BM * BK;                              // doubles per A tile
 template <int BN> __host__ __device__ constexpr int stage_doubles() { return TILE_A + BN * BK; }
-// 64 x 32 tiles: 48 KB (four CTAs per SM); 64 x 64: 64 KB (three); 64 x 128: 96 KB (two)
+// 64 x 32 tiles: 48 KB (four CTAs per SM); 64 x 64: 64 KB (three)
 template <int BN> __host__ __device__ constexpr int smem_bytes() { return STAGES * stage_doubles<BN>() * 8; }
 // Shared-memory positions, XOR-swizzled so that the fragment reads of a half
 // warp (g = 0..3 along m or n, t = 0..3 along k) hit 16 distinct 8-byte banks:
@@ -72,7 +74,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // A tiles are kept in the global layout's fast order: m fastest for op(A) = A
 // ([k][m]), k fastest for op(A) = A^T ([m][k]); B tiles k fastest for
 // op(B) = B ([n][k]), n fastest for op(B) = B^T ([k][n]); swizzled (pos_*).
-// CTA tile 64 x BN (BN = 32, 64, 128); warp w owns rows 32 (w & 1) .. +32 and
+// CTA tile 64 x BN (BN = 32, 64); warp w owns rows 32 (w & 1) .. +32 and
 // columns (BN / 2)(w >> 1) .. +BN / 2: 4 x BN / 16 DMMA tiles.
 template <bool TA, bool TB, int BN>
 __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__restrict__ A,
@@ -181,25 +183,32 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
   cp_async_wait<0>();
 }
 
-// blockIdx.x: tile of C (m fastest); blockIdx.y: batch * ksplit + split.
+// blockIdx.x: tile of C (m fastest, or n fastest); blockIdx.y: batch * ksplit + split.
 // Each split covers K range [split * kchunk, min(K, (split + 1) * kchunk)).
-// ksplit == 1: C = alpha acc + beta C;  else work[(b * ksplit + split)][m + n M] = acc.
+// ksplit == 1: C = alpha acc + beta C.
+// arrived == NULL: work[(b * ksplit + split)][m + n M] = acc (k_dgemm_reduce).
+// Otherwise the cs consecutive splits of a cluster (cluster 1 x cs) are added
+// through distributed shared memory, CTA r taking slice r of the tile's
+// elements; with more than one cluster per tile each writes its sum to
+// work[tile][cluster][element], and the CTA that arrives last at the slice's
+// counter adds them in order, stores C and resets the counter.
 template <bool TA, bool TB, int BN>
-__global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : (BN == 64 ? 3 : 2))
+__global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
     k_dgemm(int M, int N, int K, double alpha, const double *__restrict__ A, int64_t lda,
             int64_t sA, const double *__restrict__ B, int64_t ldb, int64_t sB, double beta,
             double *__restrict__ C, int64_t ldc, int64_t sC, int ksplit, int kchunk,
-            double *__restrict__ work, int tri) {
+            double *__restrict__ work, int tri, int nfast, int cs, int *__restrict__ arrived) {
   using namespace dg;
   extern __shared__ __align__(16) double smem_d[];
-  const int tiles_m = (M + BM - 1) / BM;
-  const int m0 = (blockIdx.x % tiles_m) * BM, n0 = (blockIdx.x / tiles_m) * BN;
+  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
+  const int m0 = (nfast ? blockIdx.x / tiles_n : blockIdx.x % tiles_m) * BM;
+  const int n0 = (nfast ? blockIdx.x % tiles_n : blockIdx.x / tiles_m) * BN;
   // tri > 0: column n is the pair (i, j) = (n / tri, n % tri) of a symmetric
   // pair array and only j <= i is wanted: a tile whose columns all lie above
   // the diagonal is skipped (the caller mirrors those columns)
   if (tri > 0) {
     const int i0 = n0 / tri, i1 = min(N - 1, n0 + BN - 1) / tri;
-    if (i0 == i1 && n0 - i0 * tri > i0) return;
+    if (i0 == i1 && n0 - i0 * tri > i0) return;   // the same in the whole cluster
   }
   const int batch = blockIdx.y / ksplit, split = blockIdx.y % ksplit;
   const int kb = split * kchunk, ke = min(K, kb + kchunk);
@@ -213,8 +222,13 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : (BN == 64 ? 3 : 2)
   dgemm_mainloop<TA, TB, BN>(M, N, A, lda, B, ldb, m0, n0, kb, ke, smem_d, acc);
 
   // epilogue: element (i, j, e) of this thread is C[m0 + wm + 8 i + g][n0 + wn + 8 j + 2 t + e]
+  C += batch * sC;
+  auto store = [&](int row, int col, double s) {
+    double *p = C + row + (int64_t)col * ldc;
+    const double v = alpha * s;
+    *p = beta == 0.0 ? v : v + beta * *p;
+  };
   if (ksplit == 1) {
-    C += batch * sC;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = m0 + wm + 8 * i + g;
@@ -224,13 +238,10 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : (BN == 64 ? 3 : 2)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int col = n0 + wn + 8 * j + 2 * t + e;
-          if (col >= N) continue;
-          double *p = C + row + (int64_t)col * ldc;
-          const double v = alpha * acc[i][j][e];
-          *p = beta == 0.0 ? v : v + beta * *p;
+          if (col < N) store(row, col, acc[i][j][e]);
         }
     }
-  } else {
+  } else if (!arrived) {
     double *wp = work + (int64_t)blockIdx.y * M * N;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -243,6 +254,68 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : (BN == 64 ? 3 : 2)
           const int col = n0 + wn + 8 * j + 2 * t + e;
           if (col < N) wp[row + (int64_t)col * M] = acc[i][j][e];
         }
+    }
+  } else {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    constexpr int LD = BM + 4;   // the tile in shared memory, column-major
+    static_assert(LD * BN <= STAGES * stage_doubles<BN>(), "tile in the pipeline's memory");
+    __syncthreads();             // the last stage has been read
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          smem_d[(wn + 8 * j + 2 * t + e) * LD + wm + 8 * i + g] = acc[i][j][e];
+    cl.sync();
+    constexpr int E = BM * BN;
+    const int rank = split % cs, ng = ksplit / cs, per = E / cs, tiles = gridDim.x;
+    const int64_t tile = (int64_t)batch * tiles + blockIdx.x;
+    double *wp = work + tile * ng * E;   // [cluster][element]
+    const double *remote[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) remote[r] = r < cs ? cl.map_shared_rank(smem_d, r) : smem_d;
+#pragma unroll 4
+    for (int x = tid; x < per; x += THREADS) {
+      const int el = rank * per + x, at = (el / BM) * LD + el % BM;
+      double v[8], s = 0.0;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) v[r] = r < cs ? remote[r][at] : 0.0;
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (r < cs) s += v[r];
+      if (ng == 1) {
+        const int row = m0 + el % BM, col = n0 + el / BM;
+        if (row < M && col < N) store(row, col, s);
+      } else {
+        wp[(int64_t)(split / cs) * E + el] = s;
+      }
+    }
+    cl.sync();   // no CTA leaves while others may still read its tile
+    if (ng > 1) {
+      __shared__ int last;
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) last = atomicAdd(arrived + tile * cs + rank, 1) == ng - 1;
+      __syncthreads();
+      if (last) {
+        __threadfence();
+        for (int x = tid; x < per; x += THREADS) {
+          const int el = rank * per + x, row = m0 + el % BM, col = n0 + el / BM;
+          double s = 0.0;
+          for (int q = 0; q < ng; q += 8) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = q + u < ng ? __ldcg(wp + (int64_t)(q + u) * E + el) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (q + u < ng) s += v[u];
+          }
+          if (row < M && col < N) store(row, col, s);
+        }
+        if (tid == 0) arrived[tile * cs + rank] = 0;
+      }
     }
   }
 }
@@ -303,7 +376,7 @@ struct DgProblem {
 // splits K into ks ranges whose partial tiles go to work + woff and are added
 // in split order by k_dgemm_grouped_reduce (deterministic, no atomics).
 template <bool TA, bool TB, int BN>
-__global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : (BN == 64 ? 3 : 2))
+__global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
     k_dgemm_grouped(const DgProblem *__restrict__ probs, const int *__restrict__ tile0,
                     int nprob, double *__restrict__ work) {
   using namespace dg;
@@ -369,6 +442,7 @@ __global__ void k_dgemm_grouped_reduce(const DgProblem *__restrict__ probs,
 // Launch wrapper with the split-K workspace.
 struct Dgemm {
   DBuf<double> work;
+  DBuf<int> arrived;   // arrival counters of the split tiles (one stream per instance)
   int nsm = 148;
   int64_t launches = 0;
   // set: the products go to cuBLAS on this handle instead (the library
@@ -470,53 +544,75 @@ struct Dgemm {
 
   // this instance's launches have set the kernels' shared-memory limits (a
   // host call per product otherwise; an instance serves one device)
-  bool smem_set[2][2][3] = {};
+  bool smem_set[2][2][2] = {};
   // K splits by wave counts only (see pick_split): the sTD-DFT subspace
   // iteration, whose results must not depend on the order of these sums
   bool wave_splits = false;
 
-  // Tile width and split count of one product, from the time of the busiest SM
-  // in cycles.  A CTA's K step of 16 is bound by the DMMA rate (64 FMA per SM
-  // and cycle: 16 BN cycles; measured 570 / 1024 / 2010 for BN = 32 / 64 / 128),
-  // so what counts is the sum over the CTAs that share the busiest SM, not how
-  // many of them are resident: 300 CTAs on 148 SMs take half as long again as
-  // 296.  A CTA alone on its SM has one warp per scheduler, which issues a DMMA
-  // only every ~30 cycles instead of 16 (47 % of the rate in the profile of a
-  // 150 x 25 x 21217 product), so it costs as much as nearly two.
-  // Each batch of resident CTAs adds ~2000 cycles to fill its pipeline and
-  // store; a split adds a second launch (~9000) and its partial tiles' traffic
-  // (~2000 bytes per cycle); each is at least 64 long.
-  // wave_splits: waves of four 64 x 32, three 64 x 64 or two 64 x 128 CTAs per
-  // SM, the fewest K steps of the busiest SM (splits at least 256 long, weighted
-  // 3 %), a step of a full wave taking 0.74 / 1 / 1.31.
-  void pick_split(int m, int n, int k, int batch, int &bn, int &ksplit) const {
+  // Tile width, cluster size and clusters per tile of one product, by the time
+  // (us) of the busiest SM: every product starts and stores in ~3.9; a K step of
+  // 16 is bound by the DMMA rate (64 FMA per SM and cycle) and takes 0.31 / 0.54
+  // for BN = 32 / 64, counted over the CTAs that share the busiest SM and not over
+  // those that fit on it (300 CTAs on 148 SMs take half as long again as 296).  A
+  // CTA alone on its SM has one warp per scheduler, which issues a DMMA only every
+  // ~30 cycles instead of 16, so it counts for two.  Adding the tiles of a cluster
+  // takes 1.6 + 5.5 / cs, adding g clusters 1 + 0.23 g more (per 32 columns);
+  // several clusters are full ones, so that eight CTAs share the last sum, and
+  // about 0.86 of the slots can hold clusters at a time.  Fitted to sweeps of 66
+  // products of the solver, where it picks a shape within 15 % of the best one in
+  // all but three: 220^3 13.5 -> 8.4 us with 8 CTAs per tile, 75 x 25 x 5945
+  // (transposed) 16.6 -> 12.7 us, against one CTA per tile or split sums in a
+  // second launch.  (Tiles of 128 columns were 3 to 8 % slower than 64 wherever
+  // they fill the GPU: 432 x 100000 x 432 1265 against 1181 us.)
+  // wave_splits: the split count by waves of four 64 x 32, three 64 x 64 or two
+  // 64 x 128 CTAs per SM, the fewest K steps of the busiest SM (splits at least
+  // 256 long, weighted 3 %), a step of a full wave taking 0.74 / 1 / 1.31; no
+  // clusters.  The tile's width does not change a sum.
+  void pick_split(int m, int n, int k, int batch, int &bn, int &ksplit, int &cs) const {
     double best = 0.0;
     const int64_t kk = std::max(k, 1);
-    const int kmax = wave_splits ? (int)std::max<int64_t>(1, std::min<int64_t>(64, k / 256))
-                                 : (int)std::max<int64_t>(1, std::min<int64_t>(2 * nsm, k / 64));
-    for (int w : {32, 64, 128}) {
-      const int64_t ctas = div_up(m, dg::BM) * div_up(n, w) * (int64_t)batch;
-      const int64_t resident = w == 32 ? 4 : (w == 64 ? 3 : 2), slots = resident * nsm;
-      const double wave_step = w == 32 ? 0.74 : (w == 64 ? 1.0 : 1.31);
-      const double step = w == 32 ? 570.0 : (w == 64 ? 1024.0 : 2010.0);
-      for (int ks = 1; ks <= kmax; ++ks) {
-        const int64_t kt = div_up(div_up(kk, ks), dg::BK);
-        double cost;
-        if (wave_splits) {
-          cost = (double)(div_up(ctas * ks, slots) * kt) * wave_step * (ks > 1 ? 1.03 : 1.0);
-        } else {
-          const int64_t q = div_up(ctas * ks, nsm);   // CTAs on the busiest SM
-          cost = (double)kt * step * (q == 1 ? 1.85 : (double)q) +
-                 2000.0 * (double)div_up(q, resident);
-          if (ks > 1) cost += 9000.0 + (double)ks * batch * m * (double)n * 16.0 / 2000.0;
-          if (ctas >= 4 * slots && ks > 1) continue;   // many waves: nothing to split for
-        }
-        if (best == 0.0 || cost < best) {
-          best = cost;
-          bn = w;
-          ksplit = ks;
+    auto tiles_of = [&](int w) { return div_up(m, dg::BM) * div_up(n, w) * (int64_t)batch; };
+    if (wave_splits) {
+      const int kmax = (int)std::max<int64_t>(1, std::min<int64_t>(64, k / 256));
+      for (int w : {32, 64, 128}) {
+        const int64_t slots = (w == 32 ? 4 : (w == 64 ? 3 : 2)) * (int64_t)nsm;
+        const double wave_step = w == 32 ? 0.74 : (w == 64 ? 1.0 : 1.31);
+        for (int ks = 1; ks <= kmax; ++ks) {
+          const int64_t steps =
+              div_up(tiles_of(w) * ks, slots) * div_up(div_up(kk, ks), dg::BK);
+          const double cost = (double)steps * wave_step * (ks > 1 ? 1.03 : 1.0);
+          if (best == 0.0 || cost < best) {
+            best = cost;
+            bn = std::min(w, 64);
+            ksplit = ks;
+          }
         }
       }
+      cs = 0;
+      return;
+    }
+    for (int w : {32, 64}) {
+      const int64_t ctas = tiles_of(w), resident = w == 32 ? 4 : 3, slots = resident * nsm;
+      const double step = w == 32 ? 0.31 : 0.54, cols = w / 32.0;
+      for (int c : {1, 2, 4, 8})
+        for (int g : {1, 2, 3, 4, 6, 8, 12, 16, 24}) {
+          const int64_t ks = (int64_t)c * g;
+          // no split shorter than a K step, or of a product that fills the GPU
+          if ((g > 1 && c < 8) || (ks > 1 && ((ks - 1) * dg::BK >= kk || ctas >= slots))) break;
+          const int64_t kt = div_up(div_up(kk, ks), dg::BK);
+          const int64_t room = c > 1 ? slots * 86 / 100 : slots;
+          const int64_t full = (ctas * ks - 1) / room, q = div_up(ctas * ks - full * room, nsm);
+          const double cost =
+              (double)kt * step * (double)(full * resident) +
+              (double)kt * step * (q == 1 ? 2.05 : (double)q) + (c > 1 ? 12.0 : 0.8) * (double)full +
+              (c > 1 ? 1.6 + 5.5 * cols / c : 0.0) + (g > 1 ? 1.0 + 0.23 * g * cols : 0.0);
+          if (best == 0.0 || cost < best) {
+            best = cost;
+            bn = w;
+            ksplit = (int)ks;
+            cs = c;
+          }
+        }
     }
   }
 
@@ -555,45 +651,57 @@ struct Dgemm {
                                              (int)ldb, sB, &beta, C, (int)ldc, sC, batch));
       return;
     }
-    int bn = 64, ksplit = 1;
-    pick_split(m, n, k, batch, bn, ksplit);
+    int bn = 64, ksplit = 1, cs = 1;
+    pick_split(m, n, k, batch, bn, ksplit, cs);
     const int tiles = (int)(div_up(m, dg::BM) * div_up(n, bn));
-    int kchunk = (int)div_up(div_up(std::max(k, 1), ksplit), dg::BK) * dg::BK;
-    ksplit = (int)div_up(std::max(k, 1), kchunk);
+    const int kchunk = (int)div_up(div_up(std::max(k, 1), ksplit), dg::BK) * dg::BK;
+    if (cs == 0) ksplit = (int)div_up(std::max(k, 1), kchunk);
     if (batch * ksplit > 65535) throw Error{STD2G_EINVAL, "dgemm: batch too large"};
     double *wk = nullptr;
-    if (ksplit > 1) wk = work.ensure((size_t)ksplit * batch * m * n);
-    const dim3 grid(tiles, batch * ksplit);
+    int *arr = nullptr;
+    if (ksplit > 1 && cs == 0) wk = work.ensure((size_t)ksplit * batch * m * n);
+    if (ksplit > 1 && cs > 0) {
+      if (ksplit > cs) wk = work.ensure((size_t)(ksplit / cs) * batch * tiles * dg::BM * bn);
+      // counters of the last arrivals: zero between launches
+      const size_t need = (size_t)batch * tiles * cs;
+      if (need > arrived.n) {
+        arr = arrived.ensure(std::max<size_t>(need, 4096));
+        S2G_CUDA(cudaMemsetAsync(arr, 0, sizeof(int) * arrived.n, s));
+      }
+      arr = arrived.get();
+    }
+    const dim3 grid(tiles, batch * ksplit), cluster(1, std::max(cs, 1));
+    // the CTAs of a wave share the operand whose tiles change slowest: along n
+    // first where A is the larger operand and does not stay in the L2 (65000 x
+    // 6000 x 336: with m first A is read anew for every column tile, 11.7 ms in
+    // the PT selection of C294H42 against 10.0 ms)
+    const int nfast = m > n && (double)m * k * sizeof(double) > 64e6;
 #define S2G_DGEMM(TA_, TB_, BN_)                                                              \
   do {                                                                                        \
-    bool &ready = smem_set[TA_][TB_][BN_ / 64];                                               \
+    bool &ready = smem_set[TA_][TB_][BN_ == 64];                                             \
     if (!ready)                                                                               \
       S2G_CUDA(cudaFuncSetAttribute(k_dgemm<TA_, TB_, BN_>,                                   \
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,              \
                                     dg::smem_bytes<BN_>()));                                  \
     ready = true;                                                                             \
-    S2G_LAUNCH((k_dgemm<TA_, TB_, BN_>), grid, dg::THREADS, dg::smem_bytes<BN_>(), s, m, n, k, \
-               alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, ksplit, kchunk, wk, tri);     \
+    launch_cluster(k_dgemm<TA_, TB_, BN_>, grid, dg::THREADS, dg::smem_bytes<BN_>(), cluster, \
+                   s, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, ksplit,       \
+                   kchunk, wk, tri, nfast, cs, arr);                                               \
   } while (0)
     if (bn == 32) {
       if (!ta && !tb) S2G_DGEMM(false, false, 32);
       else if (!ta && tb) S2G_DGEMM(false, true, 32);
       else if (ta && !tb) S2G_DGEMM(true, false, 32);
       else S2G_DGEMM(true, true, 32);
-    } else if (bn == 64) {
+    } else {
       if (!ta && !tb) S2G_DGEMM(false, false, 64);
       else if (!ta && tb) S2G_DGEMM(false, true, 64);
       else if (ta && !tb) S2G_DGEMM(true, false, 64);
       else S2G_DGEMM(true, true, 64);
-    } else {
-      if (!ta && !tb) S2G_DGEMM(false, false, 128);
-      else if (!ta && tb) S2G_DGEMM(false, true, 128);
-      else if (ta && !tb) S2G_DGEMM(true, false, 128);
-      else S2G_DGEMM(true, true, 128);
     }
 #undef S2G_DGEMM
     ++launches;
-    if (ksplit > 1) {
+    if (ksplit > 1 && cs == 0) {
       const int64_t total = (int64_t)m * n * batch;
       const int g = (int)std::min<int64_t>(div_up(total, kReduceThreads), (int64_t)nsm * 32);
       S2G_LAUNCH(k_dgemm_reduce, g, kReduceThreads, 0, s, m, n, batch, ksplit, alpha, wk, beta, C,

@@ -401,23 +401,6 @@ inline void symeig_tridiag_shape(int n, F &&f) {
   else f(7, TridiagShape<8, 10, 5>{});
 }
 
-template <class... KArgs, class... Args>
-inline void launch_cluster(void (*kernel)(KArgs...), dim3 grid, int threads, int cluster,
-                           cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = cluster;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
-  S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
-  ++g_launches;
-}
-
 // ---- 2. eigenvalues: multisection on Sturm counts, one CTA per eigenvalue ---
 // A round evaluates the count at kValThreads points of the interval, so that
 // it shrinks 257-fold: 7 rounds instead of the 11 of one warp's 32 points.
@@ -822,8 +805,8 @@ inline void symeig_small(cudaStream_t s, const double *A, int lda, int n, int k,
     throw Error{STD2G_EINVAL, "symeig_small: size out of range"};
   symeig_tridiag_shape(n, [&](int, auto shape) {
     using Shape = decltype(shape);
-    launch_cluster(k_symeig_tridiag<Shape>, dim3(Shape::C), kTridiagThreads, Shape::C, s, A, lda,
-                   n, work);
+    launch_cluster(k_symeig_tridiag<Shape>, dim3(Shape::C), kTridiagThreads, 0, dim3(Shape::C), s,
+                   A, lda, n, work);
   });
   S2G_CUDA(cudaFuncSetAttribute(k_symeig_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)symeig_vec_smem_bytes(kSymEigMaxN)));
@@ -863,8 +846,8 @@ inline void symeig_small_batched(cudaStream_t s, const std::vector<SymEigJob> &j
     if (count[shape] > 0)
       symeig_tridiag_shape(ord[at].n, [&](int, auto sh) {
         using Shape = decltype(sh);
-        launch_cluster(k_symeig_tridiag_b<Shape>, dim3(Shape::C, count[shape]), kTridiagThreads,
-                       Shape::C, s, (const SymEigJob *)(d + at));
+        launch_cluster(k_symeig_tridiag_b<Shape>, dim3(Shape::C, count[shape]), kTridiagThreads, 0,
+                       dim3(Shape::C), s, (const SymEigJob *)(d + at));
       });
   S2G_CUDA(cudaFuncSetAttribute(k_symeig_vectors_b, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)symeig_vec_smem_bytes(kSymEigMaxN)));
