@@ -80,7 +80,8 @@ template <bool TA, bool TB, int BN>
 __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__restrict__ A,
                                                int64_t lda, const double *__restrict__ B,
                                                int64_t ldb, int m0, int n0, int kb, int ke,
-                                               double *smem_d, double (&acc)[4][BN / 16][2]) {
+                                               double *smem_d, double (&acc)[4][BN / 16][2],
+                                               const int *__restrict__ bcol = nullptr) {
   using namespace dg;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -105,9 +106,14 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
     pa[q] = TA ? A + (kb + ka) + (int64_t)min(m0 + (tid >> 4) + 8 * q, M - 1) * lda
                : A + min(m0 + (tid & 63), M - 1) + (int64_t)(kb + ka + 2 * q) * lda;
 #pragma unroll
-  for (int q = 0; q < QB; ++q)
-    pb[q] = TB ? B + min(n0 + (tid & (BN - 1)), N - 1) + (int64_t)(kb + kbq + KS * q) * ldb
-               : B + (kb + kbq) + (int64_t)min(n0 + (tid >> 4) + 8 * q, N - 1) * ldb;
+  for (int q = 0; q < QB; ++q) {
+    if (TB) {
+      pb[q] = B + min(n0 + (tid & (BN - 1)), N - 1) + (int64_t)(kb + kbq + KS * q) * ldb;
+    } else {   // bcol: column n of op(B) is column bcol[n] of B
+      const int n = min(n0 + (tid >> 4) + 8 * q, N - 1);
+      pb[q] = B + (kb + kbq) + (int64_t)(bcol ? bcol[n] : n) * ldb;
+    }
+  }
   const int64_t sa = TA ? BK : BK * lda, sb = TB ? BK * ldb : BK;
   auto issue = [&](int st, int left) {   // left: K elements from the tile's start to ke
     double *a = As(st), *b = Bs(st);
@@ -365,6 +371,9 @@ struct DgProblem {
   const double *A, *B;
   double *C;
   int64_t lda, ldb, ldc;
+  // columns by index (op(B) = B only): column n of op(B) is column bcol[n] of B,
+  // column n of C is column ccol[n] of the array at C
+  const int *bcol = nullptr, *ccol = nullptr;
   int ks = 1;          // K splits (set by Dgemm::grouped)
   int64_t woff = 0;    // the member's partial tiles in the workspace (ks > 1)
 };
@@ -400,7 +409,7 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
   double acc[4][NJ][2];
   dgemm_mainloop<TA, TB, BN>(pr.M, pr.N, pr.A, pr.lda, pr.B, pr.ldb, m0, n0, kb, ke, smem_d,
-                             acc);
+                             acc, pr.bcol);
   double *wp = work + pr.woff + (int64_t)split * pr.M * pr.N;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -415,7 +424,7 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
         if (pr.ks > 1) {
           wp[row + (int64_t)col * pr.M] = acc[i][j][e];
         } else {
-          double *p = pr.C + row + (int64_t)col * pr.ldc;
+          double *p = pr.C + row + (int64_t)(pr.ccol ? pr.ccol[col] : col) * pr.ldc;
           const double v = pr.alpha * acc[i][j][e];
           *p = pr.beta == 0.0 ? v : v + pr.beta * *p;
         }
@@ -482,9 +491,10 @@ struct Dgemm {
     S2G_CUDA(cudaEventRecord(ev[nev++], s));
   }
 
-  // grouped launch (k_dgemm_grouped, 64 x 32 tiles) of the members with a
-  // non-empty output; the descriptors go to `gdesc` / `gtile0` (same stream:
-  // a later launch's upload waits for this launch), from `stage` when given
+  // grouped launch (k_dgemm_grouped) of the members with a non-empty output, in
+  // tiles of 64 columns where those fill the GPU, else of 32; the descriptors
+  // go to `gdesc` / `gtile0` (same stream: a later launch's upload waits for this
+  // launch), from `stage` when given
   DBuf<DgProblem> gdesc;
   DBuf<int> gtile0;
   DBuf<double> gwork;   // partial tiles of the split members
@@ -494,13 +504,22 @@ struct Dgemm {
     std::vector<int> t0(1, 0);
     int64_t wtot = 0;
     int64_t mnmax = 0;
+    int64_t t64 = 0;
+    bool split = false;
+    for (const DgProblem &q : in) {
+      if (q.M <= 0 || q.N <= 0) continue;
+      t64 += div_up(q.M, dg::BM) * div_up(q.N, 64);
+      split |= !q.ccol && q.K >= 512;
+    }
+    const int bn = !split && t64 >= 3 * (int64_t)nsm ? 64 : 32;
     for (DgProblem q : in) {
       if (q.M <= 0 || q.N <= 0) continue;
       // long sums over few output tiles (the Davidson's projections, A V of
       // a small block) split K: at least 256 per split, about 128 CTAs
-      const int64_t tmn = div_up(q.M, dg::BM) * div_up(q.N, 32);
-      q.ks = (int)std::max<int64_t>(
-          1, std::min<int64_t>({32, q.K / 256, std::max<int64_t>(1, 128 / tmn)}));
+      const int64_t tmn = div_up(q.M, dg::BM) * div_up(q.N, bn);
+      q.ks = q.ccol ? 1
+                    : (int)std::max<int64_t>(1, std::min<int64_t>({32, q.K / 256,
+                                                                   std::max<int64_t>(1, 128 / tmn)}));
       q.woff = wtot;
       if (q.ks > 1) wtot += (int64_t)q.ks * q.M * q.N;
       mnmax = std::max<int64_t>(mnmax, (int64_t)q.M * q.N);
@@ -521,18 +540,25 @@ struct Dgemm {
     }
     S2G_CUDA(cudaMemcpyAsync(d, hp, sizeof(DgProblem) * pr.size(), cudaMemcpyHostToDevice, s));
     S2G_CUDA(cudaMemcpyAsync(dt, ht, sizeof(int) * t0.size(), cudaMemcpyHostToDevice, s));
-#define S2G_DGEMM_G(TA_, TB_)                                                                   \
+#define S2G_DGEMM_G(TA_, TB_, BN_)                                                              \
   do {                                                                                          \
-    S2G_CUDA(cudaFuncSetAttribute(k_dgemm_grouped<TA_, TB_, 32>,                                \
+    S2G_CUDA(cudaFuncSetAttribute(k_dgemm_grouped<TA_, TB_, BN_>,                               \
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
-                                  dg::smem_bytes<32>()));                                       \
-    S2G_LAUNCH((k_dgemm_grouped<TA_, TB_, 32>), t0.back(), dg::THREADS, dg::smem_bytes<32>(), s, \
-               d, dt, np, wk);                                                                  \
+                                  dg::smem_bytes<BN_>()));                                      \
+    S2G_LAUNCH((k_dgemm_grouped<TA_, TB_, BN_>), t0.back(), dg::THREADS, dg::smem_bytes<BN_>(), \
+               s, d, dt, np, wk);                                                               \
   } while (0)
-    if (!ta && !tb) S2G_DGEMM_G(false, false);
-    else if (ta && !tb) S2G_DGEMM_G(true, false);
-    else if (!ta && tb) S2G_DGEMM_G(false, true);
-    else S2G_DGEMM_G(true, true);
+    if (bn == 64) {
+      if (!ta && !tb) S2G_DGEMM_G(false, false, 64);
+      else if (ta && !tb) S2G_DGEMM_G(true, false, 64);
+      else if (!ta && tb) S2G_DGEMM_G(false, true, 64);
+      else S2G_DGEMM_G(true, true, 64);
+    } else {
+      if (!ta && !tb) S2G_DGEMM_G(false, false, 32);
+      else if (ta && !tb) S2G_DGEMM_G(true, false, 32);
+      else if (!ta && tb) S2G_DGEMM_G(false, true, 32);
+      else S2G_DGEMM_G(true, true, 32);
+    }
 #undef S2G_DGEMM_G
     ++launches;
     if (wtot > 0) {

@@ -75,7 +75,7 @@ struct Ctx {
   DBuf<double> w_Qia, w_Pia, w_Qoo, w_Poo, w_Qvv, w_de, w_ek;
   DBuf<int> w_flag, w_act_idx, w_pk, w_ck, w_tmpi, w_pj, w_pb, w_omap, w_vmap, w_OP, w_VP, w_ci,
       w_ca, w_allk, w_status;
-  DBuf<double> w_ed, w_edsorted, w_Qp, w_QvvP, w_W, w_Pc, w_Kbuf, w_Jbuf, w_pert, w_colpart,
+  DBuf<double> w_ed, w_edsorted, w_Qp, w_W, w_Kbuf, w_pert, w_colpart,
       w_pt2, w_edp;
   DBuf<unsigned char> w_sel;
   DBuf<double> w_Qs, w_Ps, w_K, w_J, w_Kx, w_A, w_Apb, w_Amb, w_Bh, w_Ambh, w_M, w_eval, w_X,
@@ -1087,14 +1087,11 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
     unsigned char *sel = c.w_sel.ensure(nexpt);
     double *pert = c.w_pert.ensure(nexpt);
     double *pt2 = c.w_pt2.ensure(nex), *edp = c.w_edp.ensure(nex);
-    // The PT kernels see the primaries in (j,b) enumeration order (FP64 form:
-    // contiguous coupling reads) or (b,j) order (mixed form: the J
-    // contraction grouped by virtual index); pt2 is mapped back to the energy
-    // order afterwards.
+    // The PT kernels see the primaries in (b,j) order (the (ij|ab) products are
+    // grouped by the virtual index); pt2 is mapped back to the energy order
+    // afterwards.
     std::vector<int> pko = pk_unsorted;
-    if (tc_pt)
-      std::stable_sort(pko.begin(), pko.end(),
-                       [&](int x, int y) { return x % nv < y % nv; });   // (b, j)
+    std::stable_sort(pko.begin(), pko.end(), [&](int x, int y) { return x % nv < y % nv; });
     std::vector<double> edo(nex);
     for (int q = 0; q < nex; ++q) edo[q] = ed[kpos[pko[q]]];
     if (tc_pt) {
@@ -1111,43 +1108,36 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       c.tc_flop = c.mixed.flop;
       c.tc_launches = c.mixed.launches;
     } else {
-      // FP64 form: explicit K (candidates x primaries) and the (i,j) x (a,b)
-      // box of J per chunk of candidate occupied indices, FP64 GEMMs
-      std::vector<int> omap(no, -1), vmap(nv, -1), OP, VP, pj(nex), pb(nex);
+      // FP64 form: the couplings of a chunk of candidate occupied indices with all
+      // primaries, two sums over them (kernels_fp64.cuh)
+      std::vector<int> jq(nex), gq(nex), gb, qs, nq;   // per primary / per group (virtual b)
       for (int q = 0; q < nex; ++q) {
-        pj[q] = pko[q] / nv;
-        pb[q] = pko[q] % nv;
-        omap[pj[q]] = 1;
-        vmap[pb[q]] = 1;
+        const int b = pko[q] % nv;
+        jq[q] = pko[q] / nv;
+        if (gb.empty() || gb.back() != b) {
+          gb.push_back(b);
+          qs.push_back(q);
+          nq.push_back(0);
+        }
+        gq[q] = (int)gb.size() - 1;
+        ++nq.back();
       }
-      for (int i = 0; i < no; ++i)
-        if (omap[i] >= 0) { omap[i] = (int)OP.size(); OP.push_back(i); }
-      for (int a = 0; a < nv; ++a)
-        if (vmap[a] >= 0) { vmap[a] = (int)VP.size(); VP.push_back(a); }
-      const int nop = (int)OP.size(), nvp = (int)VP.size();
       auto up = [&](DBuf<int> &b, const std::vector<int> &v) {
         int *d = b.ensure(v.size());
         S2G_CUDA(cudaMemcpyAsync(d, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, s));
         return d;
       };
-      int *d_pk = up(c.w_pk, pko), *d_ck = up(c.w_ck, ck), *d_pj = up(c.w_pj, pj),
-          *d_pb = up(c.w_pb, pb), *d_omap = up(c.w_omap, omap), *d_vmap = up(c.w_vmap, vmap),
-          *d_OP = up(c.w_OP, OP), *d_VP = up(c.w_VP, VP);
+      int *d_pk = up(c.w_pk, pko), *d_ck = up(c.w_ck, ck), *d_jq = up(c.w_pj, jq),
+          *d_gq = up(c.w_pb, gq), *d_qs = up(c.w_omap, qs), *d_nq = up(c.w_vmap, nq);
       double *d_ed = c.w_edsorted.ensure(nex);
       S2G_CUDA(cudaMemcpyAsync(d_ed, edo.data(), sizeof(double) * nex, cudaMemcpyHostToDevice, s));
-      // primaries' charges and the virtual-pair factor
-      double *Qp = c.w_Qp.ensure((size_t)N * nex);
+      double *Qp = c.w_Qp.ensure((size_t)N * nex);   // the primaries' charges
       S2G_LAUNCH(k_gather_cols, grid_for((int64_t)N * nex), 256, 0, s, Qp, Qia, (int64_t)N, d_pk,
                  (int64_t)nex, (int64_t)N);
-      double *QvvP = c.w_QvvP.ensure((size_t)N * nv * nvp);
-      S2G_LAUNCH(k_gather_virt_pairs, grid_for((int64_t)N * nv * nvp), 256, 0, s, QvvP, Qvv, N, nv,
-                 d_VP, nvp);
-      // chunk candidates by occupied index (candidates are in (i,a) order)
-      const int64_t ldj = (int64_t)nv * nvp;
-      const double budget = 6.0e9;   // bytes of K/J buffers per chunk
-      const double per_occ = 8.0 * ((double)nex * nv + (double)ldj * nop) + 8.0 * (double)N * (nv + nop);
-      int occ_chunk = std::max(1, (int)std::min<double>(no, budget / per_occ));
-      std::vector<int> first_of_occ(no + 1, nexpt);
+      const double budget = 6.0e9;   // bytes of the coupling buffer per chunk
+      const double per_occ = 8.0 * (double)nex * (nv + 1.0);
+      const int occ_chunk = std::max(1, (int)std::min<double>(no, budget / per_occ));
+      std::vector<int> first_of_occ(no + 1, nexpt);   // candidates are in (i,a) order
       {
         int q = 0;
         for (int i = 0; i <= no; ++i) {
@@ -1155,9 +1145,15 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
           first_of_occ[i] = q;
         }
       }
-      int nchunk = (int)div_up(no, occ_chunk);
-      // column sums of the PT terms by segments of candidate rows (deterministic order)
-      const int kSeg = 2048;
+      const int nchunk = (int)div_up(no, occ_chunk);
+      // Column sums by segments of candidate rows, added in order: 2048 rows, or
+      // fewer (64 at the least) where that leaves fewer than 4 blocks per SM; the
+      // iterative sTD-DFT roots keep 2048 (wave_splits: a fixed order of every sum)
+      const int64_t qblocks = div_up(nex, kPtColQ);
+      const int64_t rows_fit = (int64_t)nexpt * qblocks / (4 * (int64_t)c.dev_sms);
+      const int kSeg = c.dg.wave_splits
+                           ? 2048
+                           : (int)std::max<int64_t>(64, std::min<int64_t>(2048, rows_fit / 64 * 64));
       std::vector<int> seg_off(nchunk + 1, 0);
       for (int q = 0; q < nchunk; ++q) {
         int a0 = q * occ_chunk, a1 = std::min(no, a0 + occ_chunk);
@@ -1167,28 +1163,47 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       const int nseg_total = std::max(1, seg_off[nchunk]);
       double *colpart = c.w_colpart.ensure((size_t)nseg_total * nex);
       for (int q = 0; q < nchunk; ++q) {
-        int i0 = q * occ_chunk, i1 = std::min(no, i0 + occ_chunk), ni = i1 - i0;
-        int r0 = first_of_occ[i0], r1 = first_of_occ[i1], nr = r1 - r0;
+        const int i0 = q * occ_chunk, i1 = std::min(no, i0 + occ_chunk), ni = i1 - i0;
+        const int r0 = first_of_occ[i0], r1 = first_of_occ[i1], nr = r1 - r0;
         if (nr == 0) continue;
-        const dim3 cgrid((unsigned)div_up(nex, 128), (unsigned)(seg_off[q + 1] - seg_off[q]));
-        double *cpart = colpart + (size_t)seg_off[q] * nex;
-        double *Pc = c.w_Pc.ensure((size_t)N * nr);
-        S2G_LAUNCH(k_gather_cols, grid_for((int64_t)N * nr), 256, 0, s, Pc, Pia, (int64_t)N,
-                   d_ck + r0, (int64_t)nr, (int64_t)N);
-        double *W = c.w_W.ensure((size_t)N * ni * nop);
-        S2G_LAUNCH(k_gather_occ_pairs, grid_for((int64_t)N * ni * nop), 256, 0, s, W, Poo, N, no,
-                   i0, ni, d_OP, nop);
-        double *Kb = c.w_Kbuf.ensure((size_t)nex * nr);
-        double *Jb = c.w_Jbuf.ensure((size_t)ldj * ni * nop);
-        gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, nex, nr, N, 1.0, Qp, N, Pc, N, 0.0, Kb, nex);
-        gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, (int)ldj, ni * nop, N, 1.0, QvvP, N, W, N, 0.0, Jb,
-             (int)ldj);
-        S2G_LAUNCH((k_pt_rows<double, double>), nr, 256, 0, s, Kb, Jb, ldj, (int64_t)nex, nex,
-                   nvp, nop, nr, d_ck + r0, nv, i0, de, d_pj, d_pb, d_omap, d_vmap, d_ed, ak,
-                   p.thrp, pert + r0, sel + r0);
-        S2G_LAUNCH((k_pt_cols<double, double>), cgrid, 128, 0, s, Kb, Jb, ldj, (int64_t)nex, nex,
-                   nvp, nop, nr, d_ck + r0, nv, i0, de, d_pj, d_pb, d_omap, d_vmap, d_ed, ak,
-                   sel + r0, cpart, kSeg);
+        double *X = c.w_Kbuf.ensure((size_t)nex * nv * ni);
+        int *bcol = c.w_OP.ensure((size_t)nex * ni), *ccol = c.w_VP.ensure((size_t)nex * ni);
+        S2G_LAUNCH(k_pt_columns, grid_for((int64_t)nex * ni), 256, 0, s, d_jq, d_gq, d_qs, d_nq, nex,
+                   ni, i0, no, bcol, ccol);
+        // ak (ia|jb), then -(ij|ab) group by group (ak = 0, 1, 2: exact, so that the
+        // sum is rounded once, as a difference of the two couplings)
+        gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, nv, nex, N, ak, Pia + (int64_t)i0 * nv * N, N, Qp, N, 0.0,
+             X, nv, ni, (int64_t)nv * N, 0, (int64_t)nv * nex);
+        std::vector<DgProblem> jp(gb.size());
+        for (size_t g = 0; g < gb.size(); ++g) {
+          DgProblem &d = jp[g];
+          d.M = nv;
+          d.N = nq[g] * ni;
+          d.K = N;
+          d.alpha = -1.0;
+          d.beta = 1.0;
+          d.A = Qvv + (int64_t)gb[g] * nv * N;   // q_ba = q_ab
+          d.B = Poo;
+          d.C = X;
+          d.lda = d.ldb = N;
+          d.ldc = nv;
+          d.bcol = bcol + (int64_t)qs[g] * ni;
+          d.ccol = ccol + (int64_t)qs[g] * ni;
+        }
+        c.dg.grouped(s, true, false, jp);
+        const int nab = (int)div_up(nv, kPtRowThreads);
+        const int nz = (int)std::max<int64_t>(
+            1, std::min<int64_t>(div_up(nex, 8), div_up(8 * (int64_t)c.dev_sms, (int64_t)ni * nab)));
+        const int qlen = (int)div_up(nex, nz);
+        double *part = c.w_W.ensure((size_t)nz * ni * nv);
+        S2G_LAUNCH(k_pt_rows, dim3((unsigned)nab, (unsigned)ni, (unsigned)nz), kPtRowThreads, 0, s, X,
+                   nv, nex, qlen, i0, de, d_ed, part);
+        S2G_LAUNCH(k_pt_rows_finish, grid_for(nr, 128), 128, 0, s, part, nz, ni, nv, i0, d_ck + r0,
+                   nr, p.thrp, pert + r0, sel + r0);
+        S2G_LAUNCH(k_pt_cols,
+                   dim3((unsigned)qblocks, (unsigned)(seg_off[q + 1] - seg_off[q])), kPtColThreads,
+                   0, s, X, nv, nex, i0, d_ck + r0, nr, de, d_ed, sel + r0,
+                   colpart + (size_t)seg_off[q] * nex, kSeg);
       }
       if (seg_off[nchunk] == 0) S2G_CUDA(cudaMemsetAsync(colpart, 0, sizeof(double) * nex, s));
       S2G_LAUNCH(k_pt2_finish, (int)div_up(nex, 128), 128, 0, s, colpart, nseg_total, nex, d_ed,

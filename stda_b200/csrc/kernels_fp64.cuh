@@ -431,104 +431,116 @@ __global__ void k_diag_screen(const double *__restrict__ P, const double *__rest
   }
 }
 
-// W[A + N*((i-i0)*nop + s)] = Poo[A + N*(i*no + OP[s])]  for i in [i0, i0+ni)
-__global__ void k_gather_occ_pairs(double *__restrict__ W, const double *__restrict__ Poo, int N,
-                                   int no, int i0, int ni, const int *__restrict__ OP, int nop) {
-  int64_t total = (int64_t)N * ni * nop;
+// ---- PT selection, FP64 form (ptselect, stda.f:1773-1863) ----
+// The couplings of a chunk of candidate occupied indices i in [i0, i0 + ni) with
+// the primaries q = (j, b), taken in (b, j) order, are formed in one buffer
+//   X[((i - i0) * nex + q) * nv + a] = ak (ia|jb) - (ij|ab)
+// by two products: p_ia . q_q for each i, then, for each virtual index b of the
+// primaries (group g, primaries qs[g] .. qs[g] + nq[g]), -q_ab . p_ij added over
+// the columns (i, j_q) of that group, so that only the wanted (ij|ab) are formed.
+// (Forming the box of all (i, j) x (a, b) of the primaries' indices took twice
+// the products, C294H42: 62 of 106 ms, and the sums gathered from it.)
+
+// columns of the second product: entry qs ni + ii nq + (q - qs) of group g names
+// column (i0 + ii) no + j_q of p_oo and column ii nex + q of X
+__global__ void k_pt_columns(const int *__restrict__ jq, const int *__restrict__ gq,
+                             const int *__restrict__ g_qs, const int *__restrict__ g_nq, int nex,
+                             int ni, int i0, int no, int *__restrict__ bcol,
+                             int *__restrict__ ccol) {
+  const int64_t total = (int64_t)nex * ni;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t col = t / N;
-    int A = (int)(t - col * N);
-    int ii = (int)(col / nop), s = (int)(col - (int64_t)ii * nop);
-    W[t] = Poo[A + (int64_t)N * ((int64_t)(i0 + ii) * no + OP[s])];
+    const int ii = (int)(t / nex), q = (int)(t - (int64_t)ii * nex);
+    const int g = gq[q], qs = g_qs[g], nq = g_nq[g];
+    const int64_t at = (int64_t)qs * ni + (int64_t)ii * nq + (q - qs);
+    bcol[at] = (i0 + ii) * no + jq[q];
+    ccol[at] = (int)t;
   }
 }
 
-// V[A + N*(a*nvp + t)] = Qvv[A + N*(a*nv + VP[t])]  for all a < nv
-__global__ void k_gather_virt_pairs(double *__restrict__ V, const double *__restrict__ Qvv, int N,
-                                    int nv, const int *__restrict__ VP, int nvp) {
-  int64_t total = (int64_t)N * nv * nvp;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t col = t / N;
-    int A = (int)(t - col * N);
-    int a = (int)(col / nvp), s = (int)(col - (int64_t)a * nvp);
-    V[t] = Qvv[A + (int64_t)N * ((int64_t)a * nv + VP[s])];
-  }
+// one PT term (stda.f:1820-1826): amat^2 / (E_r - E_q + 1e-10)
+__device__ __forceinline__ double pt_term64(double amat, double de_r, double ed) {
+  return amat * amat / (de_r - ed + 1e-10);
 }
 
-// One PT-selection term (ptselect, stda.f:1812-1826):
-//   amat = ak*(ia|jb) - (ij|ab),  pt = amat^2 / (E_k - E_j + 1e-10)
-// K: Kbuf[c + nex*r]; J: Jbuf[(a*nvp + vmap[b]) + ldj*((i-i0)*nop + omap[j])]
-template <typename TK, typename TJ>
-__device__ __forceinline__ double pt_term(const TK *Kbuf, const TJ *Jbuf, int64_t ldj, int64_t ldk,
-                                          int nvp, int nop, int r, int c, int iloc, int a,
-                                          double de_r, const int *pj, const int *pb,
-                                          const int *omap, const int *vmap,
-                                          const double *ed, double ak) {
-  double kv = (double)Kbuf[(int64_t)c + ldk * r];
-  double jv = (double)Jbuf[((int64_t)a * nvp + vmap[pb[c]]) +
-                           ldj * ((int64_t)iloc * nop + omap[pj[c]])];
-  double amat = ak * kv - jv;
-  return amat * amat / (de_r - ed[c] + 1e-10);
-}
-
-// Row pass: pert[r] = sum_j pt(r, j) and the selection pert > thrp.
-template <typename TK, typename TJ>
-__global__ void k_pt_rows(const TK *__restrict__ Kbuf, const TJ *__restrict__ Jbuf, int64_t ldj,
-                          int64_t ldk, int nex, int nvp, int nop, int nrows, const int *__restrict__ cand_k,
-                          int nv, int i0, const double *__restrict__ de_all,
-                          const int *__restrict__ pj, const int *__restrict__ pb,
-                          const int *__restrict__ omap, const int *__restrict__ vmap,
-                          const double *__restrict__ ed, double ak, double thrp,
-                          double *__restrict__ pert_out, unsigned char *__restrict__ sel) {
-  int r = blockIdx.x;
-  if (r >= nrows) return;
-  int k = cand_k[r];
-  int i = k / nv, a = k - i * nv;
-  double de_r = de_all[k];
+// Row pass: part[z][ii nv + a] = sum of the terms of row (i, a) over the
+// primaries [z qlen, (z + 1) qlen); reads X once, consecutive a in consecutive
+// threads (HBM-bound).  Grid (nv / 128, ni, nz).
+constexpr int kPtRowThreads = 128;
+__global__ void __launch_bounds__(kPtRowThreads)
+k_pt_rows(const double *__restrict__ X, int nv, int nex, int qlen, int i0,
+          const double *__restrict__ de_all, const double *__restrict__ ed,
+          double *__restrict__ part) {
+  const int a = blockIdx.x * kPtRowThreads + threadIdx.x, ii = blockIdx.y, z = blockIdx.z;
+  if (a >= nv) return;
+  const int q0 = z * qlen, q1 = min(nex, q0 + qlen);
+  const double de_r = de_all[(int64_t)(i0 + ii) * nv + a];
+  const double *x = X + ((int64_t)ii * nex + q0) * nv + a;
   double s = 0.0;
-  for (int c = threadIdx.x; c < nex; c += blockDim.x)
-    s += pt_term(Kbuf, Jbuf, ldj, ldk, nvp, nop, r, c, i - i0, a, de_r, pj, pb, omap, vmap, ed, ak);
-  __shared__ double red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+  int q = q0;
+  for (; q + 8 <= q1; q += 8, x += (int64_t)8 * nv) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = x[(int64_t)u * nv];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += pt_term64(v[u], de_r, ed[q + u]);
+  }
+  for (; q < q1; ++q, x += nv) s += pt_term64(*x, de_r, ed[q]);
+  part[((int64_t)z * gridDim.y + ii) * nv + a] = s;
+}
+
+// pert[r] = sum_z part (in order) and the selection pert > thrp, candidates r
+__global__ void k_pt_rows_finish(const double *__restrict__ part, int nz, int ni, int nv, int i0,
+                                 const int *__restrict__ cand_k, int nrows, double thrp,
+                                 double *__restrict__ pert, unsigned char *__restrict__ sel) {
+  const int64_t n = (int64_t)ni * nv;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x) {
+    const int64_t e = cand_k[r] - (int64_t)i0 * nv;
+    double s = 0.0;
+    for (int z = 0; z < nz; ++z) s += part[z * n + e];
+    pert[r] = s;
+    sel[r] = s > thrp ? 1 : 0;
+  }
+}
+
+// Column pass: colpart[seg][q] = sum over the non-selected candidates r of
+// segment blockIdx.y (seg_rows candidates, in order) of the terms.  A block
+// takes 32 primaries: all threads form the terms of 64 candidates (consecutive
+// candidates in consecutive threads), then lane l of the first warp adds
+// primary l's 64 terms in order while the others form the next 64.
+constexpr int kPtColQ = 32, kPtColR = 64, kPtColThreads = 288;   // a warp that adds, 8 that form
+__global__ void __launch_bounds__(kPtColThreads)
+k_pt_cols(const double *__restrict__ X, int nv, int nex, int i0, const int *__restrict__ cand_k,
+          int nrows, const double *__restrict__ de_all, const double *__restrict__ ed,
+          const unsigned char *__restrict__ sel, double *__restrict__ colpart, int seg_rows) {
+  __shared__ double term[2][kPtColQ][kPtColR + 1];
+  const int q0 = blockIdx.x * kPtColQ, nq = min(kPtColQ, nex - q0);
+  const int r0 = blockIdx.y * seg_rows, r1 = min(nrows, r0 + seg_rows);
+  const int ntile = (r1 - r0 + kPtColR - 1) / kPtColR;
+  double s = 0.0;
+  for (int t = 0; t <= ntile; ++t) {
+    if (threadIdx.x >= 32) {
+      if (t < ntile) {
+        const int f = threadIdx.x - 32, rl = f % kPtColR, r = r0 + t * kPtColR + rl;
+        const bool use = r < r1 && !sel[r];
+        const int k = r < r1 ? cand_k[r] : 0, i = k / nv, a = k - i * nv;
+        const double de_r = use ? de_all[k] : 1.0;
+        const double *x = X + ((int64_t)(use ? i - i0 : 0) * nex + q0) * nv + a;
+#pragma unroll
+        for (int u = 0; u < kPtColQ * kPtColR / 256; ++u) {
+          const int q = f / kPtColR + 4 * u;
+          term[t & 1][q][rl] =
+              use && q < nq ? pt_term64(x[(int64_t)q * nv], de_r, ed[q0 + q]) : 0.0;
+        }
+      }
+    } else if (t > 0) {
+      const double *v = term[(t - 1) & 1][threadIdx.x];
+#pragma unroll 16
+      for (int r = 0; r < kPtColR; ++r) s += v[r];
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    pert_out[r] = red[0];
-    sel[r] = red[0] > thrp ? 1 : 0;
-  }
-}
-
-// Column pass: colpart[c] = sum over non-selected rows r (in order) of pt(r, c).
-template <typename TK, typename TJ>
-__global__ void k_pt_cols(const TK *__restrict__ Kbuf, const TJ *__restrict__ Jbuf, int64_t ldj,
-                          int64_t ldk, int nex, int nvp, int nop, int nrows, const int *__restrict__ cand_k,
-                          int nv, int i0, const double *__restrict__ de_all,
-                          const int *__restrict__ pj, const int *__restrict__ pb,
-                          const int *__restrict__ omap, const int *__restrict__ vmap,
-                          const double *__restrict__ ed, double ak,
-                          const unsigned char *__restrict__ sel, double *__restrict__ colpart,
-                          int seg_rows) {
-  // grid: x over primaries, y over segments of seg_rows candidate rows;
-  // colpart[y*nex + c] holds the segment's sum (reduced in fixed order later)
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nex) return;
-  const int rbeg = blockIdx.y * seg_rows;
-  const int rend = min(nrows, rbeg + seg_rows);
-  colpart += (int64_t)blockIdx.y * nex;
-  double s = 0.0;
-  for (int r = rbeg; r < rend; ++r) {
-    if (sel[r]) continue;
-    int k = cand_k[r];
-    int i = k / nv, a = k - i * nv;
-    s += pt_term(Kbuf, Jbuf, ldj, ldk, nvp, nop, r, c, i - i0, a, de_all[k], pj, pb, omap, vmap,
-                 ed, ak);
-  }
-  colpart[c] = s;
+  if (threadIdx.x < nq) colpart[(int64_t)blockIdx.y * nex + q0 + threadIdx.x] = s;
 }
 
 // pt2[c] = sum_chunks colpart[chunk*nex + c] (fixed order); ed_out[c] = ed[c] - pt2[c]
