@@ -55,7 +55,7 @@ struct Ctx {
   int ncent = 0, nmo = 0, nao = 0;
   std::vector<double> h_eps, h_occ, h_xyz;
   AoIntsWork aoi;   // primitive list of the device AO integrals (ao_ints.cuh)
-  DBuf<double> w_Ares, w_Rres, w_part, w_rn, w_domc;   // dense residuals, dominant CSFs
+  DBuf<double> w_dall, w_Ares, w_Rres, w_part, w_rn, w_domc;   // dense roots, residuals, dominant CSFs
   DBuf<int> w_domi;
   Dgemm dg;         // the engine's FP64 matrix products (dgemm.cuh)
   int dev_sms = 148;   // SMs of the context's device
@@ -140,6 +140,40 @@ static void record(Ctx &c, int ph) { S2G_CUDA(cudaEventRecord(c.ev[ph], c.stream
 // (ssyevr 'V' range, stda.f:1143-1147) or the lowest k (range 'I').
 // A (n x n) is overwritten by the eigenvectors; returns the number found.
 static void dense_eig_full(Ctx &c, double *A, int n, double *w);
+
+// The same for a TDA matrix of at most kSymEigMaxN CSFs on the engine's own
+// eigensolver (symeig_small.cuh): all eigenvalues, read back to count the window,
+// then the eigenvectors up to its upper end.  syevdx reduces such a matrix in
+// 1.0 ms and synchronises with the host several times (245 CSFs, 14 roots: 1.9 ms
+// against 0.46 here).  The vectors go to `out` (n x k), the window's roots to w.
+static int dense_window_small(Ctx &c, const double *A, int n, double vl, double vu, int kmax,
+                              double *w, DBuf<double> &out, double *&X) {
+  cudaStream_t s = c.stream;
+  const int kv = kmax > 0 ? std::min(kmax, n) : n;
+  double *all = c.w_dall.ensure(n), *work = c.w_work.ensure(symeig_work_doubles(n, kv));
+  int *info = c.w_info.ensure(1);
+  S2G_CUDA(cudaMemsetAsync(info, 0, sizeof(int), s));
+  symeig_small_values(s, A, n, n, kv, all, work);
+  int lo = 0, hi = kv;
+  if (kmax <= 0) {   // the eigenvalues in (vl, vu]
+    std::vector<double> h(n);
+    S2G_CUDA(cudaMemcpyAsync(h.data(), all, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+    S2G_CUDA(cudaStreamSynchronize(s));
+    lo = (int)(std::upper_bound(h.begin(), h.end(), vl) - h.begin());
+    hi = (int)(std::upper_bound(h.begin(), h.end(), vu) - h.begin());
+    if (hi <= lo) return 0;
+  }
+  double *Z = out.ensure((size_t)n * hi);
+  symeig_small_vectors(s, n, hi, all, Z, n, work, info);
+  S2G_CUDA(cudaMemcpyAsync(w, all + lo, sizeof(double) * (hi - lo), cudaMemcpyDeviceToDevice, s));
+  int h_info = 0;
+  S2G_CUDA(cudaMemcpyAsync(&h_info, info, sizeof(int), cudaMemcpyDeviceToHost, s));
+  S2G_CUDA(cudaStreamSynchronize(s));
+  if (h_info != 0) throw Error{STD2G_ECUDA, "eigensolve: non-finite result"};
+  X = Z + (size_t)n * lo;
+  return hi - lo;
+}
+
 static int dense_eig(Ctx &c, double *A, int n, double vl, double vu, int kmax, double *w) {
   if (kmax > 0) {   // lowest kmax roots: full decomposition, eigenvectors in the leading columns
     dense_eig_full(c, A, n, w);
@@ -1549,15 +1583,23 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       root_resid = bp.final_resid;
       root_ritz = bp.final_theta;
     } else {
-      nroot = dense_eig(c, A, nci, 0.0, thr, p.nroots, om);
-      X = A;
+      const bool small = nci <= kSymEigMaxN;
+      if (small) {
+        nroot = dense_window_small(c, A, nci, 0.0, thr, p.nroots, om, c.w_X, X);
+      } else {
+        nroot = dense_eig(c, A, nci, 0.0, thr, p.nroots, om);
+        X = A;
+      }
       c.mixed.lastX = X;
       if (nroot < 1) throw Error{STD2G_ENOROOT, "no root below the energy threshold"};
-      // FP64 residuals ||A x - w x|| of the returned eigenvectors: A rebuilt
-      // from K, J and the diagonal (its storage now holds the eigenvectors)
+      // FP64 residuals ||A x - w x|| of the returned eigenvectors: where the
+      // eigenvectors took A's storage, A rebuilt from K, J and the diagonal
       {
-        double *Ar = c.w_Ares.ensure(n2), *Rr = c.w_Rres.ensure((size_t)nci * nroot);
-        S2G_LAUNCH(k_combine_tda, grid_for(n2), 256, 0, s, Ar, K, J, (int64_t)nci, ak, d_edall);
+        double *Ar = A, *Rr = c.w_Rres.ensure((size_t)nci * nroot);
+        if (!small) {
+          Ar = c.w_Ares.ensure(n2);
+          S2G_LAUNCH(k_combine_tda, grid_for(n2), 256, 0, s, Ar, K, J, (int64_t)nci, ak, d_edall);
+        }
         gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, nci, nroot, nci, 1.0, Ar, nci, X, nci, 0.0, Rr, nci);
         double *part = c.w_part.ensure((size_t)nroot * kColSplit), *rn = c.w_rn.ensure(nroot);
         S2G_LAUNCH(k_dav_resid, dim3(kColSplit, (unsigned)nroot), 256, 0, s, Rr, X, om, nci, part);

@@ -798,9 +798,10 @@ k_symeig_backtransform_b(const SymEigJob *__restrict__ jobs) {
   if (blockIdx.x < j.k) symeig_backtransform_body(blockIdx.x, j.n, j.work, j.w, j.Z, j.ldz, j.info);
 }
 
-// host launcher: n <= kSymEigMaxN, k <= n; work: symeig_work_doubles(n, k)
-inline void symeig_small(cudaStream_t s, const double *A, int lda, int n, int k, double *w,
-                         double *Z, int ldz, double *work, int *info) {
+// host launchers: n <= kSymEigMaxN, k <= n; work: symeig_work_doubles(n, k).
+// Phases 1 and 2 (the lowest k eigenvalues), then 3 and 4 (vectors of the lowest k).
+inline void symeig_small_values(cudaStream_t s, const double *A, int lda, int n, int k, double *w,
+                                double *work) {
   if (n < 1 || n > kSymEigMaxN || k < 1 || k > n)
     throw Error{STD2G_EINVAL, "symeig_small: size out of range"};
   symeig_tridiag_shape(n, [&](int, auto shape) {
@@ -808,13 +809,25 @@ inline void symeig_small(cudaStream_t s, const double *A, int lda, int n, int k,
     launch_cluster(k_symeig_tridiag<Shape>, dim3(Shape::C), kTridiagThreads, 0, dim3(Shape::C), s,
                    A, lda, n, work);
   });
+  S2G_LAUNCH(k_symeig_values, k + symeig_bt_blocks(n), kValThreads, symeig_val_smem_bytes(n), s, n,
+             k, work, w);
+}
+
+inline void symeig_small_vectors(cudaStream_t s, int n, int k, const double *w, double *Z, int ldz,
+                                 double *work, int *info) {
+  // the attribute is the same for every call (contexts on other host threads
+  // launch the same kernel concurrently), the launch takes what n needs
   S2G_CUDA(cudaFuncSetAttribute(k_symeig_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)symeig_vec_smem_bytes(kSymEigMaxN)));
   const int nb = (k + kSymEigWarps - 1) / kSymEigWarps;
-  S2G_LAUNCH(k_symeig_values, k + symeig_bt_blocks(n), kValThreads, symeig_val_smem_bytes(n), s, n,
-             k, work, w);
   S2G_LAUNCH(k_symeig_vectors, nb, kSymEigWarps * 32, symeig_vec_smem_bytes(n), s, n, k, work, w);
   S2G_LAUNCH(k_symeig_backtransform, k, kBtThreads, 0, s, n, work, w, Z, ldz, info);
+}
+
+inline void symeig_small(cudaStream_t s, const double *A, int lda, int n, int k, double *w,
+                         double *Z, int ldz, double *work, int *info) {
+  symeig_small_values(s, A, lda, n, k, w, work);
+  symeig_small_vectors(s, n, k, w, Z, ldz, work, info);
 }
 
 // Batched launcher: the problems of `jobs` (each n <= kSymEigMaxN, 1 <= k <= n)
