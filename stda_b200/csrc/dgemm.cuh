@@ -216,6 +216,9 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
     const int i0 = n0 / tri, i1 = min(N - 1, n0 + BN - 1) / tri;
     if (i0 == i1 && n0 - i0 * tri > i0) return;   // the same in the whole cluster
   }
+  // tri < 0: the product is symmetric; tiles above the diagonal are skipped and
+  // the elements below it written to both places
+  if (tri < 0 && n0 >= m0 + BM) return;
   const int batch = blockIdx.y / ksplit, split = blockIdx.y % ksplit;
   const int kb = split * kchunk, ke = min(K, kb + kchunk);
   A += batch * sA;
@@ -230,9 +233,11 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
   // epilogue: element (i, j, e) of this thread is C[m0 + wm + 8 i + g][n0 + wn + 8 j + 2 t + e]
   C += batch * sC;
   auto store = [&](int row, int col, double s) {
+    if (tri < 0 && row < col) return;
     double *p = C + row + (int64_t)col * ldc;
-    const double v = alpha * s;
-    *p = beta == 0.0 ? v : v + beta * *p;
+    const double v = alpha * s, x = beta == 0.0 ? v : v + beta * *p;
+    *p = x;
+    if (tri < 0) C[col + (int64_t)row * ldc] = x;
   };
   if (ksplit == 1) {
 #pragma unroll
@@ -594,10 +599,13 @@ struct Dgemm {
   // 64 x 128 CTAs per SM, the fewest K steps of the busiest SM (splits at least
   // 256 long, weighted 3 %), a step of a full wave taking 0.74 / 1 / 1.31; no
   // clusters.  The tile's width does not change a sum.
-  void pick_split(int m, int n, int k, int batch, int &bn, int &ksplit, int &cs) const {
+  void pick_split(int m, int n, int k, int batch, bool sym, int &bn, int &ksplit,
+                  int &cs) const {
     double best = 0.0;
-    const int64_t kk = std::max(k, 1);
-    auto tiles_of = [&](int w) { return div_up(m, dg::BM) * div_up(n, w) * (int64_t)batch; };
+    const int64_t kk = std::max(k, 1), tm = div_up(m, dg::BM);
+    auto tiles_of = [&](int w) {
+      return (sym ? tm * (tm + 1) / 2 * (dg::BM / w) : tm * div_up(n, w)) * (int64_t)batch;
+    };
     if (wave_splits) {
       const int kmax = (int)std::max<int64_t>(1, std::min<int64_t>(64, k / 256));
       for (int w : {32, 64, 128}) {
@@ -651,6 +659,7 @@ struct Dgemm {
   }
 
   // op(A) is m x k, op(B) is k x n; strides between batch members (0 for one).
+  // tri > 0: see k_dgemm; tri < 0: a symmetric n x n result (not with wave_splits).
   void run(cudaStream_t s, bool ta, bool tb, int m, int n, int k, double alpha, const double *A,
            int64_t lda, int64_t sA, const double *B, int64_t ldb, int64_t sB, double beta,
            double *C, int64_t ldc, int64_t sC, int batch = 1, int tri = 0) {
@@ -678,7 +687,7 @@ struct Dgemm {
       return;
     }
     int bn = 64, ksplit = 1, cs = 1;
-    pick_split(m, n, k, batch, bn, ksplit, cs);
+    pick_split(m, n, k, batch, tri < 0, bn, ksplit, cs);
     const int tiles = (int)(div_up(m, dg::BM) * div_up(n, bn));
     const int kchunk = (int)div_up(div_up(std::max(k, 1), ksplit), dg::BK) * dg::BK;
     if (cs == 0) ksplit = (int)div_up(std::max(k, 1), kchunk);
