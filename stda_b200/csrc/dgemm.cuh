@@ -68,6 +68,23 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Two-level columns of a product with op(B) = B^T: column n is number n % len of
+// group n / len; its elements of op(B) start at B + n % len + (n / len) sB, and row i
+// of it in C is at C + i ldc + n % len + (n / len) sC (len = 0: plain columns).  The
+// matrix-free products read and write the AOs of one atom in an AO-major array
+// through it.
+struct DgSplitCols {
+  int len = 0;
+  int64_t sB = 0, sC = 0;
+  __host__ __device__ __forceinline__ int64_t b(int n) const {
+    return len > 0 ? n % len + (int64_t)(n / len) * sB : n;
+  }
+  __host__ __device__ __forceinline__ int64_t c(int row, int n, int64_t ldc) const {
+    return len > 0 ? (int64_t)row * ldc + n % len + (int64_t)(n / len) * sC
+                   : row + (int64_t)n * ldc;
+  }
+};
+
 // Main loop of one CTA tile: acc = op(A) op(B) over the K range [kb, ke) for
 // the 64 x BN tile of C at (m0, n0), shared by the strided-batch kernel
 // k_dgemm and the grouped kernel k_dgemm_grouped.
@@ -81,7 +98,8 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
                                                int64_t lda, const double *__restrict__ B,
                                                int64_t ldb, int m0, int n0, int kb, int ke,
                                                double *smem_d, double (&acc)[4][BN / 16][2],
-                                               const int *__restrict__ bcol = nullptr) {
+                                               const int *__restrict__ bcol = nullptr,
+                                               DgSplitCols sc = DgSplitCols{}) {
   using namespace dg;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -108,7 +126,7 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
 #pragma unroll
   for (int q = 0; q < QB; ++q) {
     if (TB) {
-      pb[q] = B + min(n0 + (tid & (BN - 1)), N - 1) + (int64_t)(kb + kbq + KS * q) * ldb;
+      pb[q] = B + sc.b(min(n0 + (tid & (BN - 1)), N - 1)) + (int64_t)(kb + kbq + KS * q) * ldb;
     } else {   // bcol: column n of op(B) is column bcol[n] of B
       const int n = min(n0 + (tid >> 4) + 8 * q, N - 1);
       pb[q] = B + (kb + kbq) + (int64_t)(bcol ? bcol[n] : n) * ldb;
@@ -203,7 +221,8 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
     k_dgemm(int M, int N, int K, double alpha, const double *__restrict__ A, int64_t lda,
             int64_t sA, const double *__restrict__ B, int64_t ldb, int64_t sB, double beta,
             double *__restrict__ C, int64_t ldc, int64_t sC, int ksplit, int kchunk,
-            double *__restrict__ work, int tri, int nfast, int cs, int *__restrict__ arrived) {
+            double *__restrict__ work, int tri, int nfast, int cs, int *__restrict__ arrived,
+            DgSplitCols sc) {
   using namespace dg;
   extern __shared__ __align__(16) double smem_d[];
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
@@ -228,13 +247,13 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
   constexpr int NJ = BN / 16;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
   double acc[4][NJ][2];
-  dgemm_mainloop<TA, TB, BN>(M, N, A, lda, B, ldb, m0, n0, kb, ke, smem_d, acc);
+  dgemm_mainloop<TA, TB, BN>(M, N, A, lda, B, ldb, m0, n0, kb, ke, smem_d, acc, nullptr, sc);
 
   // epilogue: element (i, j, e) of this thread is C[m0 + wm + 8 i + g][n0 + wn + 8 j + 2 t + e]
   C += batch * sC;
   auto store = [&](int row, int col, double s) {
     if (tri < 0 && row < col) return;
-    double *p = C + row + (int64_t)col * ldc;
+    double *p = C + (TB ? sc.c(row, col, ldc) : row + (int64_t)col * ldc);
     const double v = alpha * s, x = beta == 0.0 ? v : v + beta * *p;
     *p = x;
     if (tri < 0) C[col + (int64_t)row * ldc] = x;
@@ -356,14 +375,14 @@ __device__ __forceinline__ double split_sum(const double *__restrict__ w, int64_
 constexpr int kReduceThreads = 64;   // few outputs: small blocks reach more SMs
 __global__ void __launch_bounds__(kReduceThreads)
 k_dgemm_reduce(int M, int N, int batch, int ksplit, double alpha, const double *__restrict__ work,
-               double beta, double *__restrict__ C, int64_t ldc, int64_t sC) {
+               double beta, double *__restrict__ C, int64_t ldc, int64_t sC, DgSplitCols sc) {
   const int64_t mn = (int64_t)M * N, total = mn * batch;
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total;
        x += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = x / mn, r = x - b * mn;
     const int64_t col = r / M, row = r - col * M;
     const double s = split_sum(work + b * ksplit * mn + r, mn, ksplit);
-    double *p = C + b * sC + row + col * ldc;
+    double *p = C + b * sC + sc.c((int)row, (int)col, ldc);
     *p = beta == 0.0 ? alpha * s : alpha * s + beta * *p;
   }
 }
@@ -660,9 +679,12 @@ struct Dgemm {
 
   // op(A) is m x k, op(B) is k x n; strides between batch members (0 for one).
   // tri > 0: see k_dgemm; tri < 0: a symmetric n x n result (not with wave_splits).
+  // sc: two-level columns, op(B) = B^T only (on this kernel also where `lib` is set).
   void run(cudaStream_t s, bool ta, bool tb, int m, int n, int k, double alpha, const double *A,
            int64_t lda, int64_t sA, const double *B, int64_t ldb, int64_t sB, double beta,
-           double *C, int64_t ldc, int64_t sC, int batch = 1, int tri = 0) {
+           double *C, int64_t ldc, int64_t sC, int batch = 1, int tri = 0,
+           DgSplitCols sc = DgSplitCols{}) {
+    if (sc.len > 0 && (!tb || tri != 0)) throw Error{STD2G_EINVAL, "dgemm: split columns"};
     if (m <= 0 || n <= 0 || batch <= 0) return;
     if (k < 0) throw Error{STD2G_EINVAL, "dgemm: negative k"};
     flop += 2.0 * m * n * (double)k * batch;
@@ -675,7 +697,7 @@ struct Dgemm {
         if (g.timed) g.mark(s);
       }
     } end_mark{*this, s};
-    if (lib && tri == 0) {
+    if (lib && tri == 0 && sc.len == 0) {
       const cublasOperation_t oa = ta ? CUBLAS_OP_T : CUBLAS_OP_N, ob = tb ? CUBLAS_OP_T : CUBLAS_OP_N;
       S2G_CUBLAS(cublasSetStream(lib, s));
       if (batch == 1)
@@ -721,7 +743,7 @@ struct Dgemm {
     ready = true;                                                                             \
     launch_cluster(k_dgemm<TA_, TB_, BN_>, grid, dg::THREADS, dg::smem_bytes<BN_>(), cluster, \
                    s, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, ksplit,       \
-                   kchunk, wk, tri, nfast, cs, arr);                                               \
+                   kchunk, wk, tri, nfast, cs, arr, sc);                                      \
   } while (0)
     if (bn == 32) {
       if (!ta && !tb) S2G_DGEMM(false, false, 32);
@@ -740,7 +762,7 @@ struct Dgemm {
       const int64_t total = (int64_t)m * n * batch;
       const int g = (int)std::min<int64_t>(div_up(total, kReduceThreads), (int64_t)nsm * 32);
       S2G_LAUNCH(k_dgemm_reduce, g, kReduceThreads, 0, s, m, n, batch, ksplit, alpha, wk, beta, C,
-                 ldc, sC);
+                 ldc, sC, sc);
       ++launches;
     }
   }

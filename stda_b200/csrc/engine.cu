@@ -767,13 +767,13 @@ static void response_matfree(Ctx &c, int n, const double *musel, const RespReq &
     if (tc)
       mftc_apply(c.mftc, c.blas, s, U, ncol, PU, 2.0 * ak, -1.0, -ax, d);
     else
-      mf_apply(c.mf, c.blas, s, U, ncol, PU, 2.0 * ak, -1.0, -ax, d);
+      mf_apply(c.mf, s, U, ncol, PU, 2.0 * ak, -1.0, -ax, d);
     if (amb_diag)
       S2G_LAUNCH(k_diag_mul, grid_for((int64_t)n * ncol), 256, 0, s, MV, dmd, V, n, ncol);
     else if (tc)
       mftc_apply(c.mftc, c.blas, s, V, ncol, MV, 0.0, -1.0, ax, d);
     else
-      mf_apply(c.mf, c.blas, s, V, ncol, MV, 0.0, -1.0, ax, d);
+      mf_apply(c.mf, s, V, ncol, MV, 0.0, -1.0, ax, d);
   };
   auto fp64 = [&](const double *U, const double *V, double *PU, double *MV) {
     products(U, V, PU, MV, false);
@@ -1485,7 +1485,8 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
     mf.nv = nv;
     mf.nci = nci;
     mf.nao = nao;
-    mf.f32 = false;
+    mf.ci = d_ci;
+    mf.ca = d_ca;
     if (resp_mf || tc_dav) {
       // tensor-core products (mixed form): the first Davidson stage, the
       // velocity correction and the CG products of the refined alpha(w) solve
@@ -1501,18 +1502,16 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       w.ca = d_ca;
     }
     if (resp_mf) {
-      mf_setup_ops<double>(mf, mf.d, s, Clow, c.d_slot_ao.get(), Poo, Pia, Qs, Ps, true);
+      mf_setup_ops(mf, s, Clow, c.d_slot_ao.get(), Poo, Pia, Qs, Ps, true);
       if (tc_resp) mftc_setup(c.mftc, s, Clow, nao, c.d_slot_ao.get(), Poo, Pia);
     } else if (tc_dav) {
       // tensor-core products for the first Davidson stage (and the velocity
       // correction's exchange products)
       mftc_setup(c.mftc, s, Clow, nao, c.d_slot_ao.get(), Poo, p.velcorr ? Pia : nullptr);
     } else {
-      mf_setup_ops<double>(mf, mf.d, s, Clow, c.d_slot_ao.get(), Poo, Pia, Qs, Ps,
-                           p.velcorr || p.rpa);
+      mf_setup_ops(mf, s, Clow, c.d_slot_ao.get(), Poo, Pia, Qs, Ps,
+                   p.velcorr || p.rpa);
     }
-    mf.ci = d_ci;
-    mf.ca = d_ca;
     S2G_LAUNCH(k_mf_diag, (int)div_up(nci, 128), 128, 0, s, mf.dA.ensure(nci), d_edall, ekd, uci,
                d_ci, d_ca, nci, nv, ak);
   }
@@ -1532,13 +1531,13 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
                d_ci, d_ca, nci, nv, ak, p.ax);
     const bool amb_diag = std::fabs(p.ax) < 1e-6;
     MatVec mv_p = [&](const double *V, int nb, double *W) {
-      mf_apply(c.mf, c.blas, s, V, nb, W, 2.0 * ak, -1.0, -p.ax, d);
+      mf_apply(c.mf, s, V, nb, W, 2.0 * ak, -1.0, -p.ax, d);
     };
     MatVec mv_m = [&](const double *V, int nb, double *W) {
       if (amb_diag)   // ax = 0: A-B is its diagonal ed - ak (ia|ia)
         S2G_LAUNCH(k_diag_mul, grid_for((int64_t)nci * nb), 256, 0, s, W, dmd, V, nci, nb);
       else
-        mf_apply(c.mf, c.blas, s, V, nb, W, 0.0, -1.0, p.ax, d);
+        mf_apply(c.mf, s, V, nb, W, 0.0, -1.0, p.ax, d);
     };
     nroot = std::min(p.nroots, nci);
     X = c.w_X.ensure((size_t)nci * nroot);
@@ -1562,7 +1561,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
     const double tol1 = std::max(tol, 1e-6);
     double *Xd = c.w_X.ensure((size_t)nci * p.nroots);
     MatVec mv = [&](const double *V, int nb, double *W) {
-      mf_apply(c.mf, c.blas, s, V, nb, W, ak, -1.0, 0.0, c.mf.dA.get());
+      mf_apply(c.mf, s, V, nb, W, ak, -1.0, 0.0, c.mf.dA.get());
     };
     int conv = 0;
     if (tc_dav) {
@@ -1586,8 +1585,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       SectionClock sc(c.dav, s);
       // (the velocity correction uses the tensor-core exchange products, so the
       // FP64 operators need no P^A_ov)
-      mf_setup_ops<double>(c.mf, c.mf.d, s, Clow, c.d_slot_ao.get(), Poo, Pia, Qs, Ps, false);
-      c.mf.f32 = false;
+      mf_setup_ops(c.mf, s, Clow, c.d_slot_ao.get(), Poo, Pia, Qs, Ps, false);
       sc.tick(0);
       if (c.dav.profile) std::fprintf(stderr, "FP64 operator setup %.2f ms\n", c.dav.sec_ms[0]);
       for (double &v : c.dav.sec_ms) v = 0;
@@ -1851,7 +1849,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       if (use_mf && tc_dav)   // mixed form: tensor-core exchange products
         mftc_apply(c.mftc, c.blas, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);
       else if (use_mf)
-        mf_apply(c.mf, c.blas, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);
+        mf_apply(c.mf, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);
       else
         gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, nci, nroot, nci, 1.0, Bh, nci, X, nci, 0.0, Xn, nci);
       S2G_LAUNCH(k_scale_columns, grid_for((int64_t)nci * nroot), 256, 0, s, Xn, (int64_t)nci,

@@ -1,0 +1,28 @@
+"""FP64 matrix-free products, whose atoms' products read and write the AO slots
+of one atom inside AO-major arrays: iterative roots against the oracle's dense
+diagonalisation, at sizes that put the occupied block and the slots times
+vectors across the edges of the 64 x 32 tiles.  A residual norm of 1e-9 bounds the
+error of a TDA root by 1e-9 Eh; sTD-DFT roots (w^2 is the eigenvalue, of an
+operator of norm below 10 Eh, and w > 0.1 Eh) by 1e-7."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rpa", [False, True])
+@pytest.mark.parametrize("natoms,ethr,nroots,ax", [(3, 20.0, 3, 0.5), (7, 11.0, 5, 0.2), (12, 9.0, 17, 0.5),
+                                                   (18, 8.0, 9, 0.0), (30, 7.0, 25, 0.5)])
+def test_roots(natoms, ethr, nroots, ax, rpa):
+    from oracle.stda_fp64 import Params, stda as oracle_stda
+    from stda_b200 import synth
+    from stda_b200.engine import Engine, Keywords, boundary_inputs
+    mol, ints = synth.random_molecule(natoms, seed=61 + natoms, with_ints=True)
+    kw = dict(ax=ax, e_thr_ev=ethr, rpa=rpa)
+    ref = oracle_stda(mol.xyz4(), mol.C, mol.eps, mol.occ, mol.iaoat(), *ints, Params(**kw))
+    eng = Engine(0, 0)
+    eng.load(boundary_inputs(mol, ints))
+    n = min(nroots, len(ref.iconf), len(ref.omega))
+    sol = eng.solve(Keywords(nroots=n, solver=2, conv_tol=1e-9, **kw))
+    eng.close()
+    assert np.abs(sol.omega[:n] - np.sort(ref.omega)[:n]).max() < (1e-7 if rpa else 1e-9)
