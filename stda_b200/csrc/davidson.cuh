@@ -13,6 +13,8 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
+#include <cstring>
 #include <functional>
 #include <numeric>
 #include <vector>
@@ -24,25 +26,9 @@
 
 namespace std2g {
 
-// T[:, j] = R[:, cols[j]] / (theta - diag), guarded away from zero
-__global__ void k_dav_precond(double *__restrict__ T, const double *__restrict__ R,
-                              const double *__restrict__ diag, const double *__restrict__ theta,
-                              const int *__restrict__ cols, int n, int nc) {
-  int64_t total = (int64_t)n * nc;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    int j = (int)(t / n), i = (int)(t - (int64_t)j * n);
-    int c = cols[j];
-    double d = theta[c] - diag[i];
-    if (fabs(d) < 1e-4) d = d < 0 ? -1e-4 : 1e-4;
-    T[t] = R[i + (int64_t)n * c] / d;
-  }
-}
-
-// R[:, j] -= theta_j X[:, j]; rnorm[j] = ||R[:, j]||  (one block per column)
-// Column norms are reduced in two fixed-order stages so that a block of
-// columns spreads over the whole GPU: grid (kColSplit, ncol) writes partial
-// sums of squares, k_colnorm_finish adds them in order and takes the root.
+// Column norms are reduced in two fixed-order stages so that a block of columns
+// spreads over the whole GPU: grid (kColSplit, ncol) writes partial sums of squares,
+// which their reader (a kernel, or the host for the residuals) adds in order.
 constexpr int kColSplit = 16;
 
 __device__ __forceinline__ double block_sum256(double s, double *red) {
@@ -74,17 +60,40 @@ __global__ void k_dav_resid(double *__restrict__ R, const double *__restrict__ X
   if (threadIdx.x == 0) part[(int64_t)j * gridDim.x + blockIdx.x] = s;
 }
 
-// part[j*gridDim.x + b] = partial |T[:, j]|^2
-__global__ void k_colnorm_part(const double *__restrict__ T, int n, double *__restrict__ part) {
-  const int j = blockIdx.y;
+// T[:, j] = R[:, cols[j]] / (theta - diag), guarded away from zero;
+// part[j*gridDim.x + b] = partial |T[:, j]|^2 (grid (kColSplit, nc))
+__global__ void k_dav_precond(double *__restrict__ T, const double *__restrict__ R,
+                              const double *__restrict__ diag, const double *__restrict__ theta,
+                              const int *__restrict__ cols, int n, double *__restrict__ part) {
+  const int j = blockIdx.y, c = cols[j];
+  const double th = theta[c];
   const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
   const int64_t i0 = chunk * blockIdx.x, i1 = min((int64_t)n, i0 + chunk);
-  const double *t = T + (int64_t)n * j;
   double s = 0.0;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) s += t[i] * t[i];
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    double d = th - diag[i];
+    if (fabs(d) < 1e-4) d = d < 0 ? -1e-4 : 1e-4;
+    const double t = R[i + (int64_t)n * c] / d;
+    T[i + (int64_t)n * j] = t;
+    s += t * t;
+  }
   __shared__ double red[256];
   s = block_sum256(s, red);
   if (threadIdx.x == 0) part[(int64_t)j * gridDim.x + blockIdx.x] = s;
+}
+
+// T[:, j] /= |T[:, j]| from its partial sums of squares (a zero column stays zero);
+// grid (any, ncol)
+__global__ void k_colnorm_scale(double *__restrict__ T, int n, const double *__restrict__ part,
+                                int nsplit) {
+  const int j = blockIdx.y;
+  double s = 0.0;
+  for (int b = 0; b < nsplit; ++b) s += part[(int64_t)j * nsplit + b];
+  const double v = sqrt(s), f = v > 0 ? 1.0 / v : 0.0;
+  double *t = T + (int64_t)n * j;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    t[i] *= f;
 }
 
 // out[j] = sqrt(sum_b part[j*nsplit + b]), in order
@@ -106,15 +115,14 @@ __global__ void k_unit_vectors(double *__restrict__ V, int n, const int *__restr
   }
 }
 
-// column norms of T (one block per column)
-// T[:, j] *= f(s[j]) with mode 0: 1/s, mode 1: 1/sqrt(s)
-__global__ void k_scale_by(double *__restrict__ T, int n, int ncol, const double *__restrict__ sv,
-                           int mode) {
+// T[:, j] *= 1/sqrt(s[j])
+__global__ void k_scale_rsqrt(double *__restrict__ T, int n, int ncol,
+                              const double *__restrict__ sv) {
   int64_t total = (int64_t)n * ncol;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
     double v = sv[t / n];
-    T[t] *= mode == 0 ? (v > 0 ? 1.0 / v : 0.0) : (v > 0 ? 1.0 / sqrt(v) : 0.0);
+    T[t] *= v > 0 ? 1.0 / sqrt(v) : 0.0;
   }
 }
 
@@ -266,7 +274,8 @@ k_chol_inv(const double *__restrict__ G, int nc, double tol, double *__restrict_
 struct DavidsonWork {
   DBuf<double> V, W, H, Hs, theta, X, R, T, tmp, rn, proj, G, Gc, Gz, lam, work2, part, eigwork,
       stat;
-  DBuf<int> cols, idx, info, einfo;
+  DBuf<int> cols, idx, info, einfo;   // einfo: of the batched form
+  PinnedArena pin;   // small copies from and to the host
   DBuf<double> work;
   int iters = 0;
   int64_t matvecs = 0;
@@ -309,13 +318,35 @@ using MatVec = std::function<void(const double *V, int nb, double *W)>;
 // 300 against 1.1 / 2.3 / 3.2 ms for syevd); larger ones to cuSOLVER syevd.
 constexpr int kRRSmallMax = kSymEigMaxN;
 
+// the norm of a column from its kColSplit partial sums of squares
+inline double colnorm(const double *part) {
+  double s = 0.0;
+  for (int b = 0; b < kColSplit; ++b) s += part[b];
+  return std::sqrt(s);
+}
+
+// order[0..k): the k smallest of n values ascending, ties by index
+template <typename Less>
+inline std::vector<int> lowest_indices(int n, int k, const Less &less) {
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  std::partial_sort(order.begin(), order.begin() + k, order.end(), [&](int a, int b) {
+    return less(a, b) || (!less(b, a) && a < b);
+  });
+  return order;
+}
+
 // Orthonormalises the nc columns of T (n x nc) against the m orthonormal
 // columns of V and among themselves, and appends the result to V after column
 // m (BCGS2: normalise, then two rounds of one block classical Gram-Schmidt
 // projection against V followed by Cholesky QR of the block, or, when its Gram
 // matrix is not safely positive definite, orthonormalisation through the Gram
-// matrix's eigen-decomposition that drops dependent directions).  Returns the
+// matrix's eigen-decomposition that drops dependent directions).  dw.part holds
+// the partial squared norms of T's columns (kColSplit each).  Returns the
 // number of columns appended.  kcap: capacity of the k x k work arrays.
+// Both rounds of the Cholesky form are issued before the host looks at either's
+// status (a failed factor only spoils buffers that the fallback writes anew): one
+// wait per block instead of two, each of which left the GPU idle for ~10 us.
 // fixed_order: the small factorisations by the kernels of symeig_seq.cuh.
 inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t sol,
                               cudaStream_t s, double *V, int n, int m, double *T, int nc,
@@ -323,100 +354,108 @@ inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnH
   const int k = kcap;
   const int grid = 148 * 4;
   const double one = 1.0, zero = 0.0, mone = -1.0;
+  if (nc <= 0) return 0;
   double *tmp = dw.tmp.ensure((size_t)n * k);
   double *proj = dw.proj.ensure((size_t)(m + k) * k + 4);
+  double *G = dw.G.ensure((size_t)k * k), *lam = dw.lam.ensure(k);
+  double *Li = dw.Gc.ensure((size_t)k * k), *st = dw.stat.ensure(4);
   int *info = dw.info.ensure(1);
-  int nb = 0;
-  {
-    double *G = dw.G.ensure((size_t)k * k), *lam = dw.lam.ensure(k);
-    double *part = dw.part.ensure((size_t)k * kColSplit);
-    S2G_LAUNCH(k_colnorm_part, dim3(kColSplit, (unsigned)nc), 256, 0, s, T, n, part);
-    S2G_LAUNCH(k_colnorm_finish, (int)div_up(nc, 128), 128, 0, s, part, kColSplit, nc, lam);
-    S2G_LAUNCH(k_scale_by, grid, 256, 0, s, T, n, nc, lam, 0);
-    double *Tb = T;
-    int ncur = nc;
-    for (int round = 0; round < 2 && ncur > 0; ++round) {
-      (dw.dg->gemm(s, CUBLAS_OP_T, CUBLAS_OP_N, m, ncur, n, &one, V, n, Tb, n,
-                             &zero, proj, m));
-      (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, ncur, m, &mone, V, n, proj, m,
-                             &one, Tb, n));
-      // G = Tb^T Tb; Cholesky QR when G is safely positive definite
-      (dw.dg->gemm(s, CUBLAS_OP_T, CUBLAS_OP_N, ncur, ncur, n, &one, Tb, n, Tb, n,
-                             &zero, G, ncur));
-      if (ncur <= kCholMax) {
-        // Cholesky QR: L^-T from the engine's small factorisation kernel
-        double *Li = dw.Gc.ensure((size_t)k * k), *st = dw.stat.ensure(2);
-        if (fixed_order) {
-          S2G_CUDA(cudaFuncSetAttribute(seq::k_chol_inv,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(2 * sizeof(double) * kCholMax * kCholMax)));
-          S2G_LAUNCH(seq::k_chol_inv, 1, 256, 2 * sizeof(double) * ncur * ncur, s, G, ncur, 1e-8,
-                     Li, st);
-        } else {
-          S2G_LAUNCH(k_chol_inv, 1, kCholThreads, 0, s, G, ncur, 1e-8, Li, st);
-        }
-        double h_st[2];
-        S2G_CUDA(cudaMemcpyAsync(h_st, st, sizeof(h_st), cudaMemcpyDeviceToHost, s));
-        S2G_CUDA(cudaStreamSynchronize(s));
-        if (h_st[0] == 0.0) {
-          // dst <- Tb L^-T (through tmp when Tb already is dst)
-          double *dst = V + (size_t)n * m;
-          double *o = Tb == dst ? tmp : dst;
-          (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, ncur, ncur, &one, Tb, n, Li,
-                                 ncur, &zero, o, n));
-          if (o != dst)
-            S2G_CUDA(cudaMemcpyAsync(dst, o, sizeof(double) * n * ncur,
-                                     cudaMemcpyDeviceToDevice, s));
-          Tb = dst;
-          continue;
-        }
-      }
-      // eigenpairs of G ascending: drop dependent directions
-      if (ncur <= kRRSmallMax) {
-        double *Z = dw.Gz.ensure((size_t)k * k);
-        S2G_CUDA(cudaMemsetAsync(info, 0, sizeof(int), s));
-        if (fixed_order)
-          seq::symeig_small(s, G, ncur, ncur, ncur, lam, Z, ncur,
-                            dw.eigwork.ensure(seq::symeig_work_doubles(ncur, ncur)), info);
-        else
-          symeig_small(s, G, ncur, ncur, ncur, lam, Z, ncur,
-                       dw.eigwork.ensure(symeig_work_doubles(ncur, ncur)), info);
-        S2G_CUDA(cudaMemcpyAsync(G, Z, sizeof(double) * ncur * ncur, cudaMemcpyDeviceToDevice,
-                                 s));
-      } else {
-        int lw2 = 0;
-        S2G_CUSOLVER(cusolverDnDsyevd_bufferSize(sol, CUSOLVER_EIG_MODE_VECTOR,
-                                                 CUBLAS_FILL_MODE_LOWER, ncur, G, ncur, lam,
-                                                 &lw2));
-        double *work2 = dw.work2.ensure((size_t)lw2 + 1);
-        S2G_CUSOLVER(cusolverDnDsyevd(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER,
-                                      ncur, G, ncur, lam, work2, lw2, info));
-      }
-      std::vector<double> h_lam(ncur);
-      S2G_CUDA(cudaMemcpyAsync(h_lam.data(), lam, sizeof(double) * ncur, cudaMemcpyDeviceToHost,
-                               s));
-      S2G_CUDA(cudaStreamSynchronize(s));
-      int first = 0;   // keep eigenvalues above the dependence threshold
-      const double cut = round == 0 ? 1e-10 : 1e-14;
-      while (first < ncur && !(h_lam[first] > cut)) ++first;
-      int nkeep = ncur - first;
-      if (nkeep == 0) {
-        ncur = 0;
-        break;
-      }
-      // new block = Tb U_keep diag(lam_keep)^-1/2, written into V after column m
-      double *dst = V + (size_t)n * m;
-      (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, nkeep, ncur, &one, Tb, n,
-                             G + (size_t)ncur * first, ncur, &zero, tmp, n));
-      S2G_LAUNCH(k_scale_by, grid, 256, 0, s, tmp, n, nkeep, lam + first, 1);
-      S2G_CUDA(cudaMemcpyAsync(dst, tmp, sizeof(double) * n * nkeep, cudaMemcpyDeviceToDevice,
-                               s));
-      Tb = dst;   // second round re-orthogonalises the appended block in place
-      ncur = nkeep;
+  double *dst = V + (size_t)n * m;
+  S2G_LAUNCH(k_colnorm_scale, dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(div_up(n, 512), 2 * kColSplit)), (unsigned)nc),
+             256, 0, s, T, n, dw.part.get(), kColSplit);
+  auto project = [&](double *Tb, int nb) {
+    dw.dg->gemm(s, CUBLAS_OP_T, CUBLAS_OP_N, m, nb, n, &one, V, n, Tb, n, &zero, proj, m);
+    dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, nb, m, &mone, V, n, proj, m, &one, Tb, n);
+  };
+  auto gram = [&](const double *Tb, int nb) {
+    dw.dg->gemm(s, CUBLAS_OP_T, CUBLAS_OP_N, nb, nb, n, &one, Tb, n, Tb, n, &zero, G, nb);
+  };
+  // Cholesky QR: out = Tb L^-T, its factor from the engine's small factorisation
+  auto cholesky = [&](const double *Tb, int nb, double *out, double *stat) {
+    if (fixed_order) {
+      S2G_CUDA(cudaFuncSetAttribute(seq::k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(2 * sizeof(double) * kCholMax * kCholMax)));
+      S2G_LAUNCH(seq::k_chol_inv, 1, 256, 2 * sizeof(double) * nb * nb, s, G, nb, 1e-8, Li, stat);
+    } else {
+      S2G_LAUNCH(k_chol_inv, 1, kCholThreads, 0, s, G, nb, 1e-8, Li, stat);
     }
-    nb = ncur;
+    dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, nb, nb, &one, Tb, n, Li, nb, &zero, out, n);
+  };
+  auto statuses = [&](int count) {   // host copy of st[0 .. 2 count)
+    double *h = (double *)dw.pin.take(sizeof(double) * 2 * count);
+    S2G_CUDA(cudaMemcpyAsync(h, st, sizeof(double) * 2 * count, cudaMemcpyDeviceToHost, s));
+    S2G_CUDA(cudaStreamSynchronize(s));
+    dw.pin.reset();
+    return h;
+  };
+  double *Tb = T;
+  int ncur = nc, round = 0;
+  bool failed = false;   // Tb is projected, and its Gram matrix has no Cholesky factor
+  if (nc <= kCholMax) {
+    for (int r = 0; r < 2; ++r) {
+      double *in = r == 0 ? T : tmp, *out = r == 0 ? tmp : dst;
+      project(in, nc);
+      gram(in, nc);
+      cholesky(in, nc, out, st + 2 * r);
+    }
+    const double *h = statuses(2);
+    if (h[0] == 0.0 && h[2] == 0.0) return nc;
+    failed = true;
+    round = h[0] != 0.0 ? 0 : 1;
+    if (round == 1) Tb = tmp;
   }
-  return nb;
+  for (; round < 2; ++round) {
+    if (!failed) project(Tb, ncur);
+    gram(Tb, ncur);
+    if (!failed && ncur <= kCholMax) {
+      double *o = Tb == dst ? tmp : dst;
+      cholesky(Tb, ncur, o, st);
+      if (statuses(1)[0] == 0.0) {
+        if (o != dst)
+          S2G_CUDA(cudaMemcpyAsync(dst, o, sizeof(double) * n * ncur, cudaMemcpyDeviceToDevice, s));
+        Tb = dst;
+        continue;
+      }
+    }
+    failed = false;
+    // eigenpairs of G ascending: drop dependent directions
+    if (ncur <= kRRSmallMax) {
+      double *Z = dw.Gz.ensure((size_t)k * k);
+      S2G_CUDA(cudaMemsetAsync(info, 0, sizeof(int), s));
+      if (fixed_order)
+        seq::symeig_small(s, G, ncur, ncur, ncur, lam, Z, ncur,
+                          dw.eigwork.ensure(seq::symeig_work_doubles(ncur, ncur)), info);
+      else
+        symeig_small(s, G, ncur, ncur, ncur, lam, Z, ncur,
+                     dw.eigwork.ensure(symeig_work_doubles(ncur, ncur)), info);
+      S2G_CUDA(cudaMemcpyAsync(G, Z, sizeof(double) * ncur * ncur, cudaMemcpyDeviceToDevice, s));
+    } else {
+      int lw2 = 0;
+      S2G_CUSOLVER(cusolverDnDsyevd_bufferSize(sol, CUSOLVER_EIG_MODE_VECTOR,
+                                               CUBLAS_FILL_MODE_LOWER, ncur, G, ncur, lam, &lw2));
+      double *work2 = dw.work2.ensure((size_t)lw2 + 1);
+      S2G_CUSOLVER(cusolverDnDsyevd(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, ncur,
+                                    G, ncur, lam, work2, lw2, info));
+    }
+    std::vector<double> h_lam(ncur);
+    S2G_CUDA(cudaMemcpyAsync(h_lam.data(), lam, sizeof(double) * ncur, cudaMemcpyDeviceToHost, s));
+    S2G_CUDA(cudaStreamSynchronize(s));
+    int first = 0;   // keep eigenvalues above the dependence threshold
+    const double cut = round == 0 ? 1e-10 : 1e-14;
+    while (first < ncur && !(h_lam[first] > cut)) ++first;
+    const int nkeep = ncur - first;
+    if (nkeep == 0) return 0;
+    // new block = Tb U_keep diag(lam_keep)^-1/2, written into V after column m
+    double *o = Tb == dst ? tmp : dst;
+    dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, nkeep, ncur, &one, Tb, n, G + (size_t)ncur * first,
+                ncur, &zero, o, n);
+    S2G_LAUNCH(k_scale_rsqrt, grid, 256, 0, s, o, n, nkeep, lam + first);
+    if (o != dst)
+      S2G_CUDA(cudaMemcpyAsync(dst, o, sizeof(double) * n * nkeep, cudaMemcpyDeviceToDevice, s));
+    Tb = dst;   // second round re-orthogonalises the appended block in place
+    ncur = nkeep;
+  }
+  return ncur;
 }
 
 // Returns the number of converged wanted roots (== k on success).  `mv` forms
@@ -443,20 +482,22 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
   double *H = dw.H.ensure((size_t)mmax * mmax);   // V^T W, kept across iterations (ld mmax)
   double *theta = dw.theta.ensure(mmax), *X = dw.X.ensure((size_t)n * k);
   double *R = dw.R.ensure((size_t)n * k), *T = dw.T.ensure((size_t)n * k);
-  double *tmp = dw.tmp.ensure((size_t)n * k), *rn = dw.rn.ensure(k + 2);
-  double *proj = dw.proj.ensure((size_t)mmax * k + 4);
-  int *cols = dw.cols.ensure(k), *info = dw.info.ensure(1);
-  int *einfo = dw.einfo.ensure(1);   // status of the Rayleigh-Ritz eigensolves
+  double *tmp = dw.tmp.ensure((size_t)n * k);
+  int *cols = dw.cols.ensure(k);
+  // partial squared norms of the residuals, the status of the Rayleigh-Ritz
+  // eigensolves behind them: one copy to the host
+  double *rpart = dw.rn.ensure((size_t)k * kColSplit + 1);
+  int *einfo = (int *)(rpart + (size_t)k * kColSplit);
+  dw.part.ensure((size_t)k * kColSplit);
   S2G_CUDA(cudaMemsetAsync(einfo, 0, sizeof(int), s));
-  const double one = 1.0, zero = 0.0, mone = -1.0;
+  const double one = 1.0, zero = 0.0;
 
   // initial guess: unit vectors on the k lowest diagonal elements
   std::vector<double> h_diag(n);
   S2G_CUDA(cudaMemcpyAsync(h_diag.data(), diag, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   S2G_CUDA(cudaStreamSynchronize(s));
-  std::vector<int> order(n);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h_diag[a] < h_diag[b]; });
+  const std::vector<int> order =
+      lowest_indices(n, k, [&](int a, int b) { return h_diag[a] < h_diag[b]; });
   int *idx = dw.idx.ensure(k);
   if (warm) {
     S2G_CUDA(cudaMemcpyAsync(V, X, sizeof(double) * n * k, cudaMemcpyDeviceToDevice, s));
@@ -466,9 +507,11 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
   }
   int m = 0, nb = k;
   int lwork = 0;
-  S2G_CUSOLVER(cusolverDnDsyevd_bufferSize(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER,
-                                           mmax, Hs, mmax, theta, &lwork));
+  if (mmax > kRRSmallMax)
+    S2G_CUSOLVER(cusolverDnDsyevd_bufferSize(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER,
+                                             mmax, Hs, mmax, theta, &lwork));
   double *work = dw.work.ensure((size_t)lwork + 1);
+  dw.pin.reset();
   std::vector<double> h_rn(k);
   int nconv = 0;
   dw.iters = 0;
@@ -505,15 +548,15 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
     };
     dw.dg->run(s, false, false, n, k, m, 1.0, V, n, apart(V, W), Hs, m, 0, 0.0, X, n, apart(X, R),
                2);
-    {
-      double *part = dw.part.ensure((size_t)k * kColSplit);
-      S2G_LAUNCH(k_dav_resid, dim3(kColSplit, (unsigned)k), 256, 0, s, R, X, theta, n, part);
-      S2G_LAUNCH(k_colnorm_finish, (int)div_up(k, 128), 128, 0, s, part, kColSplit, k, rn);
-    }
-    S2G_CUDA(cudaMemcpyAsync(h_rn.data(), rn, sizeof(double) * k, cudaMemcpyDeviceToHost, s));
-    int h_einfo = 0;
-    S2G_CUDA(cudaMemcpyAsync(&h_einfo, einfo, sizeof(int), cudaMemcpyDeviceToHost, s));
+    S2G_LAUNCH(k_dav_resid, dim3(kColSplit, (unsigned)k), 256, 0, s, R, X, theta, n, rpart);
+    const size_t rbytes = sizeof(double) * ((size_t)k * kColSplit + 1);
+    const double *h_part = (const double *)dw.pin.take(rbytes);
+    S2G_CUDA(cudaMemcpyAsync((void *)h_part, rpart, rbytes, cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
+    for (int j = 0; j < k; ++j) h_rn[j] = colnorm(h_part + (size_t)j * kColSplit);
+    int h_einfo = 0;
+    std::memcpy(&h_einfo, h_part + (size_t)k * kColSplit, sizeof(int));
+    dw.pin.reset();
     if (h_einfo != 0)
       throw Error{STD2G_ENOCONV, "Davidson: Rayleigh-Ritz eigensolve failed (" +
                                      std::to_string(h_einfo) + ")"};
@@ -532,8 +575,10 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
     clk.tick(3);
     if (nunc_wanted == 0) break;
     int nc = (int)unc.size();
-    S2G_CUDA(cudaMemcpyAsync(cols, unc.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, s));
-    S2G_LAUNCH(k_dav_precond, grid, 256, 0, s, T, R, diag, theta, cols, n, nc);
+    S2G_CUDA(cudaMemcpyAsync(cols, dw.pin.put(unc.data(), sizeof(int) * nc), sizeof(int) * nc,
+                             cudaMemcpyHostToDevice, s));
+    S2G_LAUNCH(k_dav_precond, dim3(kColSplit, (unsigned)nc), 256, 0, s, T, R, diag, theta, cols, n,
+               dw.part.get());
     if (m + nc > mmax) {
       // restart with the current Ritz vectors: V <- X, W <- W Y_k
       (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, k, m, &one, W, n, Hs, m, &zero,

@@ -71,29 +71,42 @@ __global__ void k_rpa_resid(double *__restrict__ Rp, double *__restrict__ Rm,
 
 // corrections of the unconverged roots cols[0..nc): from the diagonal 2 x 2
 // blocks, T[:, j] = (d- R+ + w R-) / det, T[:, nc + j] = (w R+ + d+ R-) / det,
-// det = d+ d- - w^2 (kept away from zero)
+// det = d+ d- - w^2 (kept away from zero); part[c*gridDim.x + b] = partial
+// |T[:, c]|^2 (grid (kColSplit, nc))
 __global__ void k_rpa_precond(double *__restrict__ T, const double *__restrict__ Rp,
                               const double *__restrict__ Rm, const double *__restrict__ dp,
                               const double *__restrict__ dm, const double *__restrict__ w,
-                              const int *__restrict__ cols, int n, int nc) {
-  const int64_t total = (int64_t)n * nc;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(t / n), i = (int)(t - (int64_t)j * n);
-    const int c = cols[j];
-    const double om = w[c], a = dp[i], b = dm[i];
+                              const int *__restrict__ cols, int n, double *__restrict__ part) {
+  const int j = blockIdx.y, nc = gridDim.y, c = cols[j];
+  const double om = w[c];
+  const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
+  const int64_t i0 = chunk * blockIdx.x, i1 = min((int64_t)n, i0 + chunk);
+  double s0 = 0.0, s1 = 0.0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    const int64_t t = i + (int64_t)n * j;
+    const double a = dp[i], b = dm[i];
     double det = a * b - om * om;
     if (fabs(det) < 1e-8) det = det < 0 ? -1e-8 : 1e-8;
     const double rp = Rp[i + (int64_t)n * c], rm = Rm[i + (int64_t)n * c];
-    T[t] = (b * rp + om * rm) / det;
-    T[t + (int64_t)n * nc] = (om * rp + a * rm) / det;
+    const double t0 = (b * rp + om * rm) / det, t1 = (om * rp + a * rm) / det;
+    T[t] = t0;
+    T[t + (int64_t)n * nc] = t1;
+    s0 += t0 * t0;
+    s1 += t1 * t1;
+  }
+  __shared__ double red[2][256];
+  s0 = block_sum256(s0, red[0]);
+  s1 = block_sum256(s1, red[1]);
+  if (threadIdx.x == 0) {
+    part[(int64_t)j * gridDim.x + blockIdx.x] = s0;
+    part[(int64_t)(nc + j) * gridDim.x + blockIdx.x] = s1;
   }
 }
 
 struct DavidsonRpaWork {
   DBuf<double> Q, Am, Amc, Ap2, S, T1, Mr, lam, ev, Z, Xp, Xm, Rp, Rm, C, Qc, tmpn, rn, part, om,
       wf, XpY, XmY;
-  DBuf<int> cols, einfo;
+  DBuf<int> cols;
   int iters = 0;
   int64_t matvecs = 0;
   // residual norms and roots of the last subspace step (all tracked pairs)
@@ -151,23 +164,25 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
   double *XpY = rw.XpY.ensure((size_t)n * k), *XmY = rw.XmY.ensure((size_t)n * k);
   double *Rp = rw.Rp.ensure((size_t)n * k), *Rm = rw.Rm.ensure((size_t)n * k);
   double *T = dw.T.ensure((size_t)n * 2 * k), *om = rw.om.ensure(k);
-  double *rn = rw.rn.ensure(k), *part = rw.part.ensure((size_t)k * kColSplit);
-  int *cols = rw.cols.ensure(k), *einfo = rw.einfo.ensure(1);
+  // partial squared norms of the residuals, the lowest eigenvalue of A-B in the
+  // subspace and the status of the small eigensolves: one copy to the host
+  double *part = rw.part.ensure((size_t)k * kColSplit + 2), *lam0 = part + (size_t)k * kColSplit;
+  int *cols = rw.cols.ensure(k), *einfo = (int *)(lam0 + 1);
+  dw.part.ensure((size_t)2 * k * kColSplit);
   S2G_CUDA(cudaMemsetAsync(einfo, 0, sizeof(int), s));
   // initial block: unit vectors on the k lowest diagonal elements of A
   std::vector<double> h_dp(n), h_dm(n);
   S2G_CUDA(cudaMemcpyAsync(h_dp.data(), dp, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   S2G_CUDA(cudaMemcpyAsync(h_dm.data(), dm, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   S2G_CUDA(cudaStreamSynchronize(s));
-  std::vector<int> order(n);
-  for (int i = 0; i < n; ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(),
-                   [&](int a, int b) { return h_dp[a] + h_dm[a] < h_dp[b] + h_dm[b]; });
+  const std::vector<int> order = lowest_indices(
+      n, k, [&](int a, int b) { return h_dp[a] + h_dm[a] < h_dp[b] + h_dm[b]; });
   int *idx = dw.idx.ensure(k);
   S2G_CUDA(cudaMemcpyAsync(idx, order.data(), sizeof(int) * k, cudaMemcpyHostToDevice, s));
   S2G_LAUNCH(k_unit_vectors, grid, 256, 0, s, B, n, idx, k);
   int m = 0, nb = k, nconv = 0, last_kk = 0;
-  std::vector<double> h_rn(k), h_lam(1);
+  std::vector<double> h_rn(k);
+  dw.pin.reset();
   rw.iters = 0;
   rw.matvecs = 0;
   auto add_columns = [&](double *H, const double *W, int mnew, int nbn) {
@@ -187,7 +202,7 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
     m += nb;
     // S = Am^1/2
     rpa_small_eig(dw, rw, sol, s, Am, mmax, m, m, lam, U, Zf, einfo);
-    S2G_CUDA(cudaMemcpyAsync(h_lam.data(), lam, sizeof(double), cudaMemcpyDeviceToHost, s));
+    S2G_CUDA(cudaMemcpyAsync(lam0, lam, sizeof(double), cudaMemcpyDeviceToDevice, s));
     S2G_CUDA(cudaMemcpyAsync(T1, U, sizeof(double) * m * m, cudaMemcpyDeviceToDevice, s));
     S2G_LAUNCH(k_cols_times_sqrt, grid, 256, 0, s, T1, lam, m);
     (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_T, m, m, m, &one, T1, m, U, m, &zero, S,
@@ -220,13 +235,18 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
                            n));
     S2G_LAUNCH(k_rpa_resid, dim3(kColSplit, (unsigned)kk), 256, 0, s, Rp, Rm, XpY, XmY, om, n,
                part);
-    S2G_LAUNCH(k_colnorm_finish, (int)div_up(kk, 128), 128, 0, s, part, kColSplit, kk, rn);
-    S2G_CUDA(cudaMemcpyAsync(h_rn.data(), rn, sizeof(double) * kk, cudaMemcpyDeviceToHost, s));
-    int h_einfo = 0;
-    S2G_CUDA(cudaMemcpyAsync(&h_einfo, einfo, sizeof(int), cudaMemcpyDeviceToHost, s));
+    // (kk <= k columns, so lam0 and einfo lie behind the last partial sum)
+    const size_t rbytes = sizeof(double) * ((size_t)k * kColSplit + 2);
+    const double *h_part = (const double *)dw.pin.take(rbytes);
+    S2G_CUDA(cudaMemcpyAsync((void *)h_part, part, rbytes, cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
+    for (int j = 0; j < kk; ++j) h_rn[j] = colnorm(h_part + (size_t)j * kColSplit);
+    const double h_lam = h_part[(size_t)k * kColSplit];
+    int h_einfo = 0;
+    std::memcpy(&h_einfo, h_part + (size_t)k * kColSplit + 1, sizeof(int));
+    dw.pin.reset();
     if (h_einfo != 0) throw Error{STD2G_ENOCONV, "sTD-DFT Davidson: subspace eigensolve failed"};
-    if (!(h_lam[0] > 0.0))
+    if (!(h_lam > 0.0))
       throw Error{STD2G_EAMB_NOT_PD, "matrix power impossible (A-B not positive definite)"};
     std::vector<int> unc;
     int nunc_wanted = 0;
@@ -238,8 +258,10 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
     nconv = std::min(kwant, kk) - nunc_wanted;
     if (nunc_wanted == 0 && kk >= kwant) break;
     const int nc = (int)unc.size();
-    S2G_CUDA(cudaMemcpyAsync(cols, unc.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, s));
-    S2G_LAUNCH(k_rpa_precond, grid, 256, 0, s, T, Rp, Rm, dp, dm, om, cols, n, nc);
+    S2G_CUDA(cudaMemcpyAsync(cols, dw.pin.put(unc.data(), sizeof(int) * nc), sizeof(int) * nc,
+                             cudaMemcpyHostToDevice, s));
+    S2G_LAUNCH(k_rpa_precond, dim3(kColSplit, (unsigned)nc), 256, 0, s, T, Rp, Rm, dp, dm, om, cols,
+               n, dw.part.get());
     if (m + 2 * nc > mmax) {
       // restart on span{X+Y, X-Y} of the kk roots: C = [Xp Xm] (m x 2kk),
       // orthonormalised through its Gram matrix (dependent directions dropped;
@@ -263,7 +285,7 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
       double *Qc = rw.Qc.ensure((size_t)mmax * 2 * k);
       (dw.dg->gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, m, nkeep, nc2, &one, C, m,
                              Gz + (size_t)nc2 * first, nc2, &zero, Qc, m));
-      S2G_LAUNCH(k_scale_by, grid, 256, 0, s, Qc, m, nkeep, gl + first, 1);
+      S2G_LAUNCH(k_scale_rsqrt, grid, 256, 0, s, Qc, m, nkeep, gl + first);
       // b <- b Qc, P <- P Qc, Q <- Q Qc; Ap, Am <- Qc^T (.) Qc
       double *tn = rw.tmpn.ensure((size_t)n * 2 * k);
       for (double *X : {B, P, Q}) {
