@@ -740,8 +740,11 @@ inline void BatchDavidson::iterate(std::vector<BatchProblem *> &act) {
       } else {
         // dependent directions: davidson()'s Gram eigen-decomposition path
         // for this member alone (rare)
+        S2G_LAUNCH(k_colnorm_part, dim3(kColSplit, (unsigned)p->ncur), 256, 0, cs_, p->Tb, p->n,
+                   dw.part.ensure((size_t)p->k * kColSplit));
+        dw.pin.reset();
         p->ncur = dav_orthonormalize(dw, p->blas, p->sol, cs_, dw.V.get(), p->n, p->m, p->Tb,
-                                     p->ncur, p->k);
+                                     p->ncur, p->k, p->mmax - p->m);
         p->ortho_open = false;
       }
     }

@@ -82,6 +82,19 @@ __global__ void k_dav_precond(double *__restrict__ T, const double *__restrict__
   if (threadIdx.x == 0) part[(int64_t)j * gridDim.x + blockIdx.x] = s;
 }
 
+// part[j*gridDim.x + b] = partial |T[:, j]|^2
+__global__ void k_colnorm_part(const double *__restrict__ T, int n, double *__restrict__ part) {
+  const int j = blockIdx.y;
+  const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
+  const int64_t i0 = chunk * blockIdx.x, i1 = min((int64_t)n, i0 + chunk);
+  const double *t = T + (int64_t)n * j;
+  double s = 0.0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) s += t[i] * t[i];
+  __shared__ double red[256];
+  s = block_sum256(s, red);
+  if (threadIdx.x == 0) part[(int64_t)j * gridDim.x + blockIdx.x] = s;
+}
+
 // T[:, j] /= |T[:, j]| from its partial sums of squares (a zero column stays zero);
 // grid (any, ncol)
 __global__ void k_colnorm_scale(double *__restrict__ T, int n, const double *__restrict__ part,
@@ -342,19 +355,22 @@ inline std::vector<int> lowest_indices(int n, int k, const Less &less) {
 // projection against V followed by Cholesky QR of the block, or, when its Gram
 // matrix is not safely positive definite, orthonormalisation through the Gram
 // matrix's eigen-decomposition that drops dependent directions).  dw.part holds
-// the partial squared norms of T's columns (kColSplit each).  Returns the
-// number of columns appended.  kcap: capacity of the k x k work arrays.
+// the partial squared norms of T's columns (kColSplit each).  T may be the place of
+// the new columns itself.  Returns the
+// number of columns appended, at most `room` (the columns that V can still take):
+// a block that is larger goes through the eigen-decomposition, which then keeps its
+// leading directions.  kcap: capacity of the k x k work arrays.
 // Both rounds of the Cholesky form are issued before the host looks at either's
 // status (a failed factor only spoils buffers that the fallback writes anew): one
 // wait per block instead of two, each of which left the GPU idle for ~10 us.
 // fixed_order: the small factorisations by the kernels of symeig_seq.cuh.
 inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t sol,
                               cudaStream_t s, double *V, int n, int m, double *T, int nc,
-                              int kcap, bool fixed_order = false) {
+                              int kcap, int room, bool fixed_order = false) {
   const int k = kcap;
   const int grid = 148 * 4;
   const double one = 1.0, zero = 0.0, mone = -1.0;
-  if (nc <= 0) return 0;
+  if (nc <= 0 || room <= 0) return 0;
   double *tmp = dw.tmp.ensure((size_t)n * k);
   double *proj = dw.proj.ensure((size_t)(m + k) * k + 4);
   double *G = dw.G.ensure((size_t)k * k), *lam = dw.lam.ensure(k);
@@ -391,7 +407,7 @@ inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnH
   double *Tb = T;
   int ncur = nc, round = 0;
   bool failed = false;   // Tb is projected, and its Gram matrix has no Cholesky factor
-  if (nc <= kCholMax) {
+  if (nc <= kCholMax && nc <= room && T != dst) {
     for (int r = 0; r < 2; ++r) {
       double *in = r == 0 ? T : tmp, *out = r == 0 ? tmp : dst;
       project(in, nc);
@@ -407,7 +423,7 @@ inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnH
   for (; round < 2; ++round) {
     if (!failed) project(Tb, ncur);
     gram(Tb, ncur);
-    if (!failed && ncur <= kCholMax) {
+    if (!failed && ncur <= kCholMax && ncur <= room) {
       double *o = Tb == dst ? tmp : dst;
       cholesky(Tb, ncur, o, st);
       if (statuses(1)[0] == 0.0) {
@@ -443,6 +459,7 @@ inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnH
     int first = 0;   // keep eigenvalues above the dependence threshold
     const double cut = round == 0 ? 1e-10 : 1e-14;
     while (first < ncur && !(h_lam[first] > cut)) ++first;
+    first = std::max(first, ncur - room);
     const int nkeep = ncur - first;
     if (nkeep == 0) return 0;
     // new block = Tb U_keep diag(lam_keep)^-1/2, written into V after column m
@@ -590,7 +607,7 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
       S2G_LAUNCH(k_diag_matrix, (int)div_up((int64_t)k * k, 256), 256, 0, s, H, mmax, k, theta);
     }
     // block orthogonalisation of the corrections, appended to V after column m
-    nb = dav_orthonormalize(dw, blas, sol, s, V, n, m, T, nc, k);
+    nb = dav_orthonormalize(dw, blas, sol, s, V, n, m, T, nc, k, mmax - m);
     clk.tick(4);
     if (nb == 0) break;
   }

@@ -301,7 +301,7 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
       }
       m = nkeep;
     }
-    nb = dav_orthonormalize(dw, blas, sol, s, B, n, m, T, 2 * nc, 2 * k, true);
+    nb = dav_orthonormalize(dw, blas, sol, s, B, n, m, T, 2 * nc, 2 * k, mmax - m, true);
     if (nb == 0) break;
   }
   S2G_CUDA(cudaMemcpyAsync(omega_out, om, sizeof(double) * kwant, cudaMemcpyDeviceToDevice, s));

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("natoms,ethr,nroots,rpa", [(3, 20.0, 13, False), (7, 11.0, 70, False),
-                                                    (3, 20.0, 6, True), (7, 11.0, 20, True)])
+                                                    (12, 9.0, 150, False), (3, 20.0, 6, True),
+                                                    (7, 11.0, 20, True)])
 def test_dependent_blocks(natoms, ethr, nroots, rpa):
     from oracle.stda_fp64 import Params, stda as oracle_stda
     from stda_b200 import synth
