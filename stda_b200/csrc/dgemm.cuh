@@ -68,20 +68,25 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Two-level columns of a product with op(B) = B^T: column n is number n % len of
-// group n / len; its elements of op(B) start at B + n % len + (n / len) sB, and row i
-// of it in C is at C + i ldc + n % len + (n / len) sC (len = 0: plain columns).  The
-// matrix-free products read and write the AOs of one atom in an AO-major array
-// through it.
+// Two-level columns of a product: column n is number n % len of group n / len
+// (len = 0: plain columns).  With op(B) = B^T the columns of a group are neighbours: its
+// elements of op(B) start at B + n % len + (n / len) sB, and row i of it in C is at
+// C + i ldc + n % len + (n / len) sC.  With op(B) = B they are leading dimensions apart:
+// B + (n % len) ldb + (n / len) sB and C + i + (n % len) ldc + (n / len) sC.
+// The matrix-free products read and write the AOs of one atom in an array over all
+// AOs through it.
 struct DgSplitCols {
   int len = 0;
   int64_t sB = 0, sC = 0;
-  __host__ __device__ __forceinline__ int64_t b(int n) const {
-    return len > 0 ? n % len + (int64_t)(n / len) * sB : n;
+  template <bool TB>
+  __host__ __device__ __forceinline__ int64_t b(int n, int64_t ldb) const {
+    if (len <= 0) return TB ? n : (int64_t)n * ldb;
+    return (int64_t)(n % len) * (TB ? 1 : ldb) + (int64_t)(n / len) * sB;
   }
-  __host__ __device__ __forceinline__ int64_t c(int row, int n, int64_t ldc) const {
-    return len > 0 ? (int64_t)row * ldc + n % len + (int64_t)(n / len) * sC
-                   : row + (int64_t)n * ldc;
+  __host__ __device__ __forceinline__ int64_t c(bool tb, int row, int n, int64_t ldc) const {
+    if (len <= 0) return row + (int64_t)n * ldc;
+    return (tb ? (int64_t)row * ldc + n % len : row + (int64_t)(n % len) * ldc) +
+           (int64_t)(n / len) * sC;
   }
 };
 
@@ -126,10 +131,10 @@ __device__ __forceinline__ void dgemm_mainloop(int M, int N, const double *__res
 #pragma unroll
   for (int q = 0; q < QB; ++q) {
     if (TB) {
-      pb[q] = B + sc.b(min(n0 + (tid & (BN - 1)), N - 1)) + (int64_t)(kb + kbq + KS * q) * ldb;
+      pb[q] = B + sc.b<true>(min(n0 + (tid & (BN - 1)), N - 1), ldb) + (int64_t)(kb + kbq + KS * q) * ldb;
     } else {   // bcol: column n of op(B) is column bcol[n] of B
       const int n = min(n0 + (tid >> 4) + 8 * q, N - 1);
-      pb[q] = B + (kb + kbq) + (int64_t)(bcol ? bcol[n] : n) * ldb;
+      pb[q] = B + (kb + kbq) + sc.b<false>(bcol ? bcol[n] : n, ldb);
     }
   }
   const int64_t sa = TA ? BK : BK * lda, sb = TB ? BK * ldb : BK;
@@ -253,7 +258,7 @@ __global__ void __launch_bounds__(dg::THREADS, BN == 32 ? 4 : 3)
   C += batch * sC;
   auto store = [&](int row, int col, double s) {
     if (tri < 0 && row < col) return;
-    double *p = C + (TB ? sc.c(row, col, ldc) : row + (int64_t)col * ldc);
+    double *p = C + sc.c(TB, row, col, ldc);
     const double v = alpha * s, x = beta == 0.0 ? v : v + beta * *p;
     *p = x;
     if (tri < 0) C[col + (int64_t)row * ldc] = x;
@@ -375,14 +380,15 @@ __device__ __forceinline__ double split_sum(const double *__restrict__ w, int64_
 constexpr int kReduceThreads = 64;   // few outputs: small blocks reach more SMs
 __global__ void __launch_bounds__(kReduceThreads)
 k_dgemm_reduce(int M, int N, int batch, int ksplit, double alpha, const double *__restrict__ work,
-               double beta, double *__restrict__ C, int64_t ldc, int64_t sC, DgSplitCols sc) {
+               double beta, double *__restrict__ C, int64_t ldc, int64_t sC, DgSplitCols sc,
+               bool tb) {
   const int64_t mn = (int64_t)M * N, total = mn * batch;
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total;
        x += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = x / mn, r = x - b * mn;
     const int64_t col = r / M, row = r - col * M;
     const double s = split_sum(work + b * ksplit * mn + r, mn, ksplit);
-    double *p = C + b * sC + sc.c((int)row, (int)col, ldc);
+    double *p = C + b * sC + sc.c(tb, (int)row, (int)col, ldc);
     *p = beta == 0.0 ? alpha * s : alpha * s + beta * *p;
   }
 }
@@ -679,12 +685,12 @@ struct Dgemm {
 
   // op(A) is m x k, op(B) is k x n; strides between batch members (0 for one).
   // tri > 0: see k_dgemm; tri < 0: a symmetric n x n result (not with wave_splits).
-  // sc: two-level columns, op(B) = B^T only (on this kernel also where `lib` is set).
+  // sc: two-level columns (on this kernel also where `lib` is set).
   void run(cudaStream_t s, bool ta, bool tb, int m, int n, int k, double alpha, const double *A,
            int64_t lda, int64_t sA, const double *B, int64_t ldb, int64_t sB, double beta,
            double *C, int64_t ldc, int64_t sC, int batch = 1, int tri = 0,
            DgSplitCols sc = DgSplitCols{}) {
-    if (sc.len > 0 && (!tb || tri != 0)) throw Error{STD2G_EINVAL, "dgemm: split columns"};
+    if (sc.len > 0 && tri != 0) throw Error{STD2G_EINVAL, "dgemm: split columns"};
     if (m <= 0 || n <= 0 || batch <= 0) return;
     if (k < 0) throw Error{STD2G_EINVAL, "dgemm: negative k"};
     flop += 2.0 * m * n * (double)k * batch;
@@ -762,7 +768,7 @@ struct Dgemm {
       const int64_t total = (int64_t)m * n * batch;
       const int g = (int)std::min<int64_t>(div_up(total, kReduceThreads), (int64_t)nsm * 32);
       S2G_LAUNCH(k_dgemm_reduce, g, kReduceThreads, 0, s, m, n, batch, ksplit, alpha, wk, beta, C,
-                 ldc, sC, sc);
+                 ldc, sC, sc, tb);
       ++launches;
     }
   }

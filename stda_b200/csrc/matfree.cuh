@@ -179,9 +179,14 @@ inline void mf_setup_ops(MatFree &mf, cudaStream_t s, const double *Clow, const 
 
 // out (nci x m) = cK (K X) + cJ (J X) + cX (Kx X) + diag o X  (diag may be NULL).
 // Seven launches for A X: a block of 25 vectors of a 60-atom molecule is bound by
-// their latency.  The atoms' products read the rows of their AOs from Z and write
-// them to Tacc in place (DgSplitCols), where two transposes moved both arrays
-// (61 / 141 atoms: 19 / 34 us of a 140 / 350 us product).
+// their latency.  The atoms' products work in place in an array over all AOs
+// (DgSplitCols), where two transposes moved both arrays.  For large molecules that
+// array is [AO][orbital] with one product per vector: every load and store of the
+// atoms' products is contiguous (336 products 432 x 248 x 432: 2.10 -> 1.2 ms; 50
+// vectors of C294H42 7 % faster, alpha(w) of a 200-atom chain 5 %).  That needs `no`
+// (and `nv`) to fill the 64-row tiles to 87 %.  Below 160 occupied orbitals (112:
+// no difference), and where the sums are to be split as before (wave_splits), it is
+// [orbital][AO] over all vectors at once, whose runs are the 4 to 9 AOs of an atom.
 inline void mf_apply(MatFree &mf, cudaStream_t s, const double *X, int m, double *out, double cK,
                      double cJ, double cX, const double *diag) {
   const int N = mf.N, maxa = mf.maxa, no = mf.no, nv = mf.nv, nci = mf.nci;
@@ -199,30 +204,59 @@ inline void mf_apply(MatFree &mf, cudaStream_t s, const double *X, int m, double
   }
   if (box_part) {
     double *box = mf.box.ensure((size_t)(std::max((int64_t)lv * no, (int64_t)lo * nv) * m));
-    double *Z = mf.Z.ensure((size_t)lr * std::max(no, nv) * m);
-    double *Tacc = mf.Tacc.ensure((size_t)lr * no * m);
-    const int64_t so = (int64_t)lr * no, sv = (int64_t)lr * nv;   // one vector of Z / Tacc
+    double *Z = mf.Z.ensure((size_t)std::max((int64_t)lr * std::max(no, nv),
+                                             (int64_t)rows * std::max(lo, lv)) * m);
+    double *Tacc = mf.Tacc.ensure((size_t)std::max((int64_t)lr * no, (int64_t)rows * lo) * m);
+    const auto fills = [](int n) { return div_up(n, dg::BM) * dg::BM * 87 <= 100 * (int64_t)n; };
+    const bool by_ao =
+        !dg.wave_splits && no >= 160 && fills(no) && (cX == 0.0 || fills(nv));
+    const int64_t so = (int64_t)(by_ao ? rows : lr) * (by_ao ? lo : no);   // one vector of Tacc
     double beta = 0.0;
     if (cJ != 0.0) {
-      // Z = CvP (rows x nv) * XbT (nv x no*m), XbT[b + lv*(j + no*r)]
       S2G_LAUNCH(k_mf_box, grid, 256, 0, s, box, X, mf.pos.get(), nci, nv, no, lv, m);
-      dg.run(s, false, false, rows, no * m, nv, 1.0, mf.CvP.get(), lr, 0, box, lv, 0, 0.0, Z, lr, 0);
-      // atom A: Tacc[(s,i,r)] = cJ sum_j P^A_oo[i,j] Z[(s,j,r)], AO slots s of A
-      dg.run(s, false, true, no, maxa * m, no, cJ, mf.PooA.get(), lo, (int64_t)lo * no, Z, lr, maxa,
-             0.0, Tacc, lr, maxa, N, 0, DgSplitCols{maxa, so, so});
+      if (by_ao) {
+        // Z[j + lo*(R + rows*r)] = sum_b X[(j,b),r] CvP[R,b], R = (A, s)
+        dg.run(s, true, true, no, rows, nv, 1.0, box, lv, (int64_t)lv * no, mf.CvP.get(), lr, 0, 0.0,
+               Z, lo, so, m);
+        // atom A: Tacc[i,(s,r)] = cJ sum_j P^A_oo[i,j] Z[j,(s,r)]
+        dg.run(s, false, false, no, maxa * m, no, cJ, mf.PooA.get(), lo, (int64_t)lo * no, Z, lo,
+               (int64_t)lo * maxa, 0.0, Tacc, lo, (int64_t)lo * maxa, N, 0,
+               DgSplitCols{maxa, so, so});
+      } else {
+        // Z = CvP (rows x nv) * XbT (nv x no*m), XbT[b + lv*(j + no*r)]
+        dg.run(s, false, false, rows, no * m, nv, 1.0, mf.CvP.get(), lr, 0, box, lv, 0, 0.0, Z, lr, 0);
+        // atom A: Tacc[(s,i,r)] = cJ sum_j P^A_oo[i,j] Z[(s,j,r)], AO slots s of A
+        dg.run(s, false, true, no, maxa * m, no, cJ, mf.PooA.get(), lo, (int64_t)lo * no, Z, lr, maxa,
+               0.0, Tacc, lr, maxa, N, 0, DgSplitCols{maxa, so, so});
+      }
       beta = 1.0;
     }
     if (cX != 0.0) {
-      // Z = CoP (rows x no) * Xb (no x nv*m), Xb[j + lo*(b + nv*r)]
-      S2G_LAUNCH(k_mf_box, grid, 256, 0, s, box, X,
-                 mf.pos.get() + (int64_t)no * nv, nci, no, nv, lo, m);
-      dg.run(s, false, false, rows, nv * m, no, 1.0, mf.CoP.get(), lr, 0, box, lo, 0, 0.0, Z, lr, 0);
-      // atom A: Tacc[(s,i,r)] += cX sum_b P^A_ov[i,b] Z[(s,b,r)]
-      dg.run(s, false, true, no, maxa * m, nv, cX, mf.PovA.get(), lo, (int64_t)lo * nv, Z, lr, maxa,
-             beta, Tacc, lr, maxa, N, 0, DgSplitCols{maxa, sv, so});
+      S2G_LAUNCH(k_mf_box, grid, 256, 0, s, box, X, mf.pos.get() + (int64_t)no * nv, nci, no, nv, lo,
+                 m);
+      if (by_ao) {
+        // Z[b + lv*(R + rows*r)] = sum_j X[(j,b),r] CoP[R,j]
+        const int64_t sv = (int64_t)rows * lv;
+        dg.run(s, true, true, nv, rows, no, 1.0, box, lo, (int64_t)lo * nv, mf.CoP.get(), lr, 0, 0.0,
+               Z, lv, sv, m);
+        // atom A: Tacc[i,(s,r)] += cX sum_b P^A_ov[i,b] Z[b,(s,r)]
+        dg.run(s, false, false, no, maxa * m, nv, cX, mf.PovA.get(), lo, (int64_t)lo * nv, Z, lv,
+               (int64_t)lv * maxa, beta, Tacc, lo, (int64_t)lo * maxa, N, 0,
+               DgSplitCols{maxa, sv, so});
+      } else {
+        // Z = CoP (rows x no) * Xb (no x nv*m), Xb[j + lo*(b + nv*r)]
+        dg.run(s, false, false, rows, nv * m, no, 1.0, mf.CoP.get(), lr, 0, box, lo, 0, 0.0, Z, lr, 0);
+        // atom A: Tacc[(s,i,r)] += cX sum_b P^A_ov[i,b] Z[(s,b,r)]
+        dg.run(s, false, true, no, maxa * m, nv, cX, mf.PovA.get(), lo, (int64_t)lo * nv, Z, lr, maxa,
+               beta, Tacc, lr, maxa, N, 0, DgSplitCols{maxa, (int64_t)lr * nv, so});
+      }
     }
     // box[a + lv*(i + no*r)] = CvP^T (nv x rows) * Tacc (rows x no*m)
-    dg.run(s, true, false, nv, no * m, rows, 1.0, mf.CvP.get(), lr, 0, Tacc, lr, 0, 0.0, box, lv, 0);
+    if (by_ao)
+      dg.run(s, true, true, nv, no, rows, 1.0, mf.CvP.get(), lr, 0, Tacc, lo, so, 0.0, box, lv,
+             (int64_t)lv * no, m);
+    else
+      dg.run(s, true, false, nv, no * m, rows, 1.0, mf.CvP.get(), lr, 0, Tacc, lr, 0, 0.0, box, lv, 0);
     S2G_LAUNCH(k_mf_gather, grid, 256, 0, s, out, box, mf.ci, mf.ca, nci, no, lv, m, cK != 0.0, X,
                diag);
   } else if (diag) {

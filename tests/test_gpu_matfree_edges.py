@@ -26,3 +26,25 @@ def test_roots(natoms, ethr, nroots, ax, rpa):
     sol = eng.solve(Keywords(nroots=n, solver=2, conv_tol=1e-9, **kw))
     eng.close()
     assert np.abs(sol.omega[:n] - np.sort(ref.omega)[:n]).max() < (1e-7 if rpa else 1e-9)
+
+
+@pytest.mark.parametrize("natoms,ethr", [(99, 6.5), (108, 6.5)])
+def test_by_ao_form(natoms, ethr):
+    """More than 160 occupied orbitals that fill the tiles (189 and 187; 109 and 116
+    virtual ones, of which only the latter fill theirs): roots and alpha(w) against the
+    engine's explicit matrices.  Roots to the residual bound, alpha as the other
+    matrix-free tests."""
+    from stda_b200 import synth
+    from stda_b200.engine import Engine, Keywords, boundary_inputs
+    mol, ints = synth.random_molecule(natoms, seed=61 + natoms, with_ints=True)
+    eng = Engine(0, 0)
+    eng.load(boundary_inputs(mol, ints))
+    kw = dict(ax=0.5, e_thr_ev=ethr)
+    dense = eng.solve(Keywords(nroots=12, solver=1, **kw)).omega
+    it = eng.solve(Keywords(nroots=12, solver=2, conv_tol=1e-9, **kw)).omega
+    assert np.abs(it - dense[:12]).max() < 1.1e-9
+    om = np.array([0.0, 0.05])
+    a1, _ = eng.polarizability(Keywords(solver=1, rpa=True, **kw), om)
+    a2, _ = eng.polarizability(Keywords(solver=2, rpa=True, **kw), om)
+    eng.close()
+    assert np.allclose(a1, a2, rtol=1e-8, atol=1e-8)
