@@ -782,6 +782,7 @@ static void response_matfree(Ctx &c, int n, const double *musel, const RespReq &
     products(pu, pv, qu, qv, mixed);
   };
   response_ir<double, double>(c, n, musel, rq, fallback, dpd, dmd, fp64, inner);
+  if (mixed) c.mftc.tc.check(s);
 }
 
 // --------------------------------------------------------------------------
@@ -1573,6 +1574,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       c.dav.profile = c.opts.verbose >= 2;
       for (double &v : c.dav.sec_ms) v = 0;
       davidson(c.dav, c.blas, c.solver, s, mv_tc, d_edall, nci, p.nroots, tol1, 300, om, Xd);
+      c.mftc.tc.check(s);
       c.dav_iters = c.dav.iters;
       c.dav_matvecs = c.dav.matvecs;
       if (c.dav.profile)
@@ -1846,9 +1848,10 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
     if (p.velcorr) {
       // X_new = (B/2) X / w (apbtrafo.f:51-65)
       double *Xn = c.w_Y.ensure((size_t)nci * nroot);
-      if (use_mf && tc_dav)   // mixed form: tensor-core exchange products
+      if (use_mf && tc_dav) {   // mixed form: tensor-core exchange products
         mftc_apply(c.mftc, c.blas, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);
-      else if (use_mf)
+        c.mftc.tc.check(s);
+      } else if (use_mf)
         mf_apply(c.mf, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);
       else
         gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, nci, nroot, nci, 1.0, Bh, nci, X, nci, 0.0, Xn, nci);

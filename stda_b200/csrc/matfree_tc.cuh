@@ -2,16 +2,18 @@
 //
 // Same factorisation as matfree.cuh (J X = C_v^T P^A_oo (C_v X^T), per atom A),
 // but every GEMM is the split-BF16 tcgen05 contraction of tc_gemm.cuh:
-//   G1: Z[(j,r), R]      = sum_b  XbT[(j,r), b] * Cv[R, b]        (one launch)
-//   G2: T_A[(s,r), i]    = sum_j  Zt_A[(s,r), j] * P^A[i, j]      (batched over atoms)
+//   G1: Z[R, (r,j)]      = sum_b  Cv[R, b] * XbT[(r,j), b]        (one launch)
+//   G2: T_A[(s,r), i]    = sum_j  Z_A[(s,r), j] * P^A[i, j]       (batched over atoms)
 //   G3: Y[(i,r), a]      = sum_R  Tt[(i,r), R] * Cv[R, a]^T       (one launch)
 // R runs over the padded AO slots (atom A, slot s), j/i over occupied and a/b
-// over virtual MOs of the active window, r over the vectors of the block.  The
-// layout changes between the GEMMs write the next K-major BF16 hi/lo operand
-// directly (tiled transposes).  The K part (p_u . sum_v q_v X_v) is two thin
+// over virtual MOs of the active window, r over the vectors of the block.  G1's
+// epilogue writes the BF16 pair that G2 reads, row (R, r) after row; a tiled
+// transpose writes G3's operand.  (With G1 the other way round, FP32 Z, a
+// transpose and zeroed paddings between the two cost as much as the product itself:
+// 0.24 + 0.24 ms per 50 vectors of C384H48, 48 of 105 us per 15 of a 200-atom chain.)  The K part (p_u . sum_v q_v X_v) is two thin
 // FP64 GEMMs.  The exchange-type products K_x X ((ib|ja), the velocity
 // correction and A +- B) follow the same pattern with C_o and P^A_ov:
-//   G1x: Z2[(b,r), R] = sum_j X[(b,r), j] Co[R, j],
+//   G1x: Z2[R, (r,b)] = sum_j Co[R, j] X[(r,b), j],
 //   G2x: U_A[(s,r), i] = sum_b Z2_A[(s,r), b] P^A_ov[i, b],
 // and U joins T before G3.
 #pragma once
@@ -56,7 +58,7 @@ __global__ void k_tcs_clow(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__rest
 
 // Atom-major rows of a pair tensor: out[A*n1*K2 + i*K2 + j] = P[A + N*(i*n2 + j)]
 // (i < n1, j < n2; P^A_oo with n1 = n2 = no, P^A_ov with n1 = no, n2 = nv;
-// padding columns must be zeroed by the caller).  Tiled over (atoms, pairs).
+// padding columns are left as they are).  Tiled over (atoms, pairs).
 __global__ void k_tcs_pairs(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
                             const double *__restrict__ P, int N, int n1, int n2, int K2) {
   __shared__ double tile[32][33];
@@ -81,66 +83,42 @@ __global__ void k_tcs_pairs(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__res
   }
 }
 
-// XbT[(j + no*r)*Kv + b] = X[u + nci*r] for the CSF u = (j,b)  (box zeroed first)
-__global__ void k_tcs_scatter(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                              const double *__restrict__ X, const int *__restrict__ ci,
-                              const int *__restrict__ ca, int nci, int no, int Kv, int m) {
-  int64_t total = (int64_t)nci * m;
+// out[(g + ng*r)*Kp + f] = X[u + nci*r] with u = pos[f + nf*g], zero where there is no
+// CSF, for f >= nf and for g >= nrow (ng: rows per vector, Kp a multiple of 8).  Eight
+// elements per thread; one pass instead of two memsets and a scatter.
+__global__ void k_tcs_box(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
+                          const double *__restrict__ X, const int *__restrict__ pos, int nci,
+                          int nf, int nrow, int ng, int Kp, int m) {
+  const int64_t total = (int64_t)(Kp / 8) * ng * m;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    int r = (int)(t / nci), u = (int)(t - (int64_t)r * nci);
-    split_store(hi, lo, ((int64_t)ci[u] + (int64_t)no * r) * Kv + ca[u], X[t]);
-  }
-}
-
-// Xb[(b + nv*r)*Ko + j] = X[u + nci*r] for the CSF u = (j,b)  (box zeroed first)
-__global__ void k_tcs_scatter_v(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                                const double *__restrict__ X, const int *__restrict__ ci,
-                                const int *__restrict__ ca, int nci, int nv, int Ko, int m) {
-  int64_t total = (int64_t)nci * m;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    int r = (int)(t / nci), u = (int)(t - (int64_t)r * nci);
-    split_store(hi, lo, ((int64_t)ca[u] + (int64_t)nv * r) * Ko + ci[u], X[t]);
-  }
-}
-
-// Z[(j + no*r)*ldR + R] -> Zt[A*(maxa*m*Ko) + (s + maxa*r)*Ko + j], R = A*maxa + s.
-// grid (no/32, rows/32, m), block 32x8; padding columns j >= no zeroed by the caller.
-__global__ void k_tcs_to_atom(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                              const float *__restrict__ Z, int ldR, int rows, int maxa, int no,
-                              int Ko, int m) {
-  __shared__ float tile[32][33];
-  const int j0 = blockIdx.x * 32, R0 = blockIdx.y * 32, r = blockIdx.z, tx = threadIdx.x;
-  for (int ty = threadIdx.y; ty < 32; ty += 8) {
-    int j = j0 + ty, R = R0 + tx;
-    if (j < no && R < rows) tile[ty][tx] = Z[((int64_t)j + (int64_t)no * r) * ldR + R];
-  }
-  __syncthreads();
-  for (int ty = threadIdx.y; ty < 32; ty += 8) {
-    int R = R0 + ty, j = j0 + tx;
-    if (j < no && R < rows) {
-      int A = R / maxa, s = R - A * maxa;
-      int64_t o = (int64_t)A * maxa * m * Ko + ((int64_t)s + (int64_t)maxa * r) * Ko + j;
-      split_store(hi, lo, o, (double)tile[tx][ty]);
+    const int64_t c = t / (Kp / 8);
+    const int f0 = (int)(t - c * (Kp / 8)) * 8, r = (int)(c / ng), g = (int)(c - (int64_t)r * ng);
+    __align__(16) __nv_bfloat16 h[8], l[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int f = f0 + e;
+      const int u = f < nf && g < nrow ? pos[f + (int64_t)nf * g] : -1;
+      const double x = u >= 0 ? X[u + (int64_t)nci * r] : 0.0;
+      h[e] = __double2bfloat16(x);
+      l[e] = __double2bfloat16(x - (double)__bfloat162float(h[e]));
     }
+    *reinterpret_cast<uint4 *>(hi + c * Kp + f0) = *reinterpret_cast<const uint4 *>(h);
+    *reinterpret_cast<uint4 *>(lo + c * Kp + f0) = *reinterpret_cast<const uint4 *>(l);
   }
 }
 
-// f T_A + fU U_A, both [(s + maxa*r)*ldo + i] per atom (stride bst, either
-// may be NULL) -> Tt[(i + no*r)*KR + R].
-// grid (no/32, rows/32, m), block 32x8; padding columns R >= rows zeroed by the caller.
+// f T + fU U, both [(R*m + r)*ldo + i] (either may be NULL) -> Tt[(i + no*r)*KR + R].
+// grid (no/32, rows/32, m), block 32x8; columns R >= rows are left as they are.
 __global__ void k_tcs_from_atom(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
                                 const float *__restrict__ T, const float *__restrict__ U,
-                                int64_t bst, int ldo, int rows, int maxa, int no, int KR, int m,
-                                double f, double fU) {
+                                int ldo, int rows, int no, int KR, int m, double f, double fU) {
   __shared__ float tile[32][33];
   const int i0 = blockIdx.x * 32, R0 = blockIdx.y * 32, r = blockIdx.z, tx = threadIdx.x;
   for (int ty = threadIdx.y; ty < 32; ty += 8) {
     int R = R0 + ty, i = i0 + tx;
     if (i < no && R < rows) {
-      int A = R / maxa, s = R - A * maxa;
-      const int64_t o = (int64_t)A * bst + ((int64_t)s + (int64_t)maxa * r) * ldo + i;
+      const int64_t o = ((int64_t)R * m + r) * ldo + i;
       float v = 0.f;
       if (T) v += (float)f * T[o];
       if (U) v += (float)fU * U[o];
@@ -155,15 +133,18 @@ __global__ void k_tcs_from_atom(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *_
   }
 }
 
-// out[u + nci*r] += Y[(i_u + no*r)*ldv + a_u]
+// out[u + nci*r] += Y[(i_u + no*r)*ldv + a_u] + diag[u] X[u + nci*r] (diag may be NULL)
 __global__ void k_tcs_gather(double *__restrict__ out, const float *__restrict__ Y, int ldv,
                              const int *__restrict__ ci, const int *__restrict__ ca, int nci,
-                             int no, int m) {
+                             int no, int m, const double *__restrict__ X,
+                             const double *__restrict__ diag) {
   int64_t total = (int64_t)nci * m;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
     int r = (int)(t / nci), u = (int)(t - (int64_t)r * nci);
-    out[t] += (double)Y[((int64_t)ci[u] + (int64_t)no * r) * ldv + ca[u]];
+    double v = out[t] + (double)Y[((int64_t)ci[u] + (int64_t)no * r) * ldv + ca[u]];
+    if (diag) v = fma(diag[u], X[t], v);
+    out[t] = v;
   }
 }
 
@@ -200,12 +181,13 @@ struct MatFreeTc {
   TcGemm tc;
   DBuf<__nv_bfloat16> cvt_h, cvt_l, cv2_h, cv2_l, poo_h, poo_l;
   DBuf<__nv_bfloat16> xb_h, xb_l, zt_h, zt_l, tt_h, tt_l;
-  DBuf<float> Z, T, Y;
+  DBuf<float> T, Y;
+  DBuf<int> pos;   // positions of the CSFs (k_mf_positions)
   // exchange chain (K_x X, the (ib|ja) products): C_o rows, P^A_ov rows
   bool has_x = false;
   DBuf<__nv_bfloat16> cot_h, cot_l, pov_h, pov_l, xv_h, xv_l, z2t_h, z2t_l;
-  DBuf<float> Z2, U;
-  DBuf<double> G, Kt;
+  DBuf<float> U;
+  DBuf<double> G;
   SideStream side;
 };
 
@@ -225,12 +207,14 @@ inline void mftc_setup(MatFreeTc &w, cudaStream_t s, const double *Clow, int nao
              1);
   const size_t np = (size_t)w.N * w.no * w.Ko;
   __nv_bfloat16 *ph = w.poo_h.ensure(np), *pl = w.poo_l.ensure(np);
-  S2G_CUDA(cudaMemsetAsync(ph, 0, np * 2, s));
-  S2G_CUDA(cudaMemsetAsync(pl, 0, np * 2, s));
   S2G_LAUNCH(k_tcs_pairs,
              dim3((unsigned)div_up(w.N, 32),
                   (unsigned)std::min<int64_t>(div_up((int64_t)w.no * w.no, 32), 65535)),
              dim3(32, 8), 0, s, ph, pl, Poo, w.N, w.no, w.no, w.Ko);
+  int *pos = w.pos.ensure((size_t)2 * w.no * w.nv);
+  S2G_CUDA(cudaMemsetAsync(pos, 0xff, sizeof(int) * 2 * w.no * w.nv, s));
+  S2G_LAUNCH(k_mf_positions, (int)div_up(w.nci, 256), 256, 0, s, pos, w.ci, w.ca, w.nci, w.no,
+             w.nv);
   w.has_x = Pia != nullptr;
   if (w.has_x) {
     S2G_LAUNCH(k_tcs_clow, g, 256, 0, s, w.cot_h.ensure((size_t)w.rows * w.Ko),
@@ -238,8 +222,6 @@ inline void mftc_setup(MatFreeTc &w, cudaStream_t s, const double *Clow, int nao
                w.Ko, 2);
     const size_t nq = (size_t)w.N * w.no * w.Kv;
     __nv_bfloat16 *qh = w.pov_h.ensure(nq), *ql = w.pov_l.ensure(nq);
-    S2G_CUDA(cudaMemsetAsync(qh, 0, nq * 2, s));
-    S2G_CUDA(cudaMemsetAsync(ql, 0, nq * 2, s));
     S2G_LAUNCH(k_tcs_pairs,
                dim3((unsigned)div_up(w.N, 32),
                     (unsigned)std::min<int64_t>(div_up((int64_t)w.no * w.nv, 32), 65535)),
@@ -273,67 +255,51 @@ inline void mftc_apply(MatFreeTc &w, cublasHandle_t h, cudaStream_t s, const dou
   (void)h;
   if (cJ != 0.0 || cX != 0.0) {
     const int64_t mo = (int64_t)no * m, mz = (int64_t)maxa * m;
-    const int ldR = ld4(rows), ldo = ld4(no), ldv = ld4(nv);
-    const int64_t bst = mz * ldo;
+    const int ldo = ld4(no), ldv = ld4(nv), Zo = ld8(no), Zv = ld8(nv);
     const dim3 tb(32, 8);
     float *T = nullptr, *U = nullptr;
     if (cJ != 0.0) {
-      // G1: Z[(j,r), R] = sum_b X_jb^r Cv[R, b]
-      __nv_bfloat16 *xh = w.xb_h.ensure((size_t)mo * w.Kv), *xl = w.xb_l.ensure((size_t)mo * w.Kv);
-      S2G_CUDA(cudaMemsetAsync(xh, 0, (size_t)mo * w.Kv * 2, s));
-      S2G_CUDA(cudaMemsetAsync(xl, 0, (size_t)mo * w.Kv * 2, s));
-      S2G_LAUNCH(k_tcs_scatter, g, 256, 0, s, xh, xl, X, w.ci, w.ca, nci, no, w.Kv, m);
-      float *Z = w.Z.ensure((size_t)mo * ldR);
-      w.tc.run(s, xh, xl, w.cvt_h.get(), w.cvt_l.get(), (int)mo, rows, w.Kv, Z, ldR,
-               2.0 * mo * rows * nv, 1, false, 0, false);
+      // G1: Z[R, (r,j)] = sum_b Cv[R, b] X_jb^r, j padded to Zo
+      const size_t nx = (size_t)m * Zo * w.Kv, nz = (size_t)rows * m * Zo;
+      __nv_bfloat16 *xh = w.xb_h.ensure(nx), *xl = w.xb_l.ensure(nx);
+      S2G_LAUNCH(k_tcs_box, g, 256, 0, s, xh, xl, X, w.pos.get(), nci, nv, no, Zo, w.Kv, m);
+      __nv_bfloat16 *zh = w.zt_h.ensure(nz), *zl = w.zt_l.ensure(nz);
+      w.tc.run(s, w.cvt_h.get(), w.cvt_l.get(), w.Kv, xh, xl, w.Kv, rows, m * Zo, nv, zh, zl,
+               (int64_t)m * Zo, 2.0 * mo * rows * nv);
       // G2: T_A[(s,r), i] = sum_j Z_A[(s,r), j] P^A_oo[i, j], batched over atoms
-      __nv_bfloat16 *zh = w.zt_h.ensure((size_t)N * mz * w.Ko),
-                    *zl = w.zt_l.ensure((size_t)N * mz * w.Ko);
-      S2G_CUDA(cudaMemsetAsync(zh, 0, (size_t)N * mz * w.Ko * 2, s));
-      S2G_CUDA(cudaMemsetAsync(zl, 0, (size_t)N * mz * w.Ko * 2, s));
-      S2G_LAUNCH(k_tcs_to_atom, dim3((unsigned)div_up(no, 32), (unsigned)div_up(rows, 32), (unsigned)m),
-                 tb, 0, s, zh, zl, Z, ldR, rows, maxa, no, w.Ko, m);
-      T = w.T.ensure((size_t)N * bst);
-      w.tc.run(s, zh, zl, w.poo_h.get(), w.poo_l.get(), (int)mz, no, w.Ko, T, ldo,
-               2.0 * mz * no * no, N, true, bst, false);
+      T = w.T.ensure((size_t)N * mz * ldo);
+      w.tc.run(s, zh, zl, Zo, w.poo_h.get(), w.poo_l.get(), w.Ko, (int)mz, no, no, T, nullptr, ldo,
+               2.0 * mz * no * no, N, true, mz * ldo);
     }
     if (cX != 0.0) {
-      // G1x: Z2[(b,r), R] = sum_j X_jb^r Co[R, j]
+      // G1x: Z2[R, (r,b)] = sum_j Co[R, j] X_jb^r, b padded to Zv
       const int64_t mv = (int64_t)nv * m;
-      __nv_bfloat16 *xh = w.xv_h.ensure((size_t)mv * w.Ko), *xl = w.xv_l.ensure((size_t)mv * w.Ko);
-      S2G_CUDA(cudaMemsetAsync(xh, 0, (size_t)mv * w.Ko * 2, s));
-      S2G_CUDA(cudaMemsetAsync(xl, 0, (size_t)mv * w.Ko * 2, s));
-      S2G_LAUNCH(k_tcs_scatter_v, g, 256, 0, s, xh, xl, X, w.ci, w.ca, nci, nv, w.Ko, m);
-      float *Z2 = w.Z2.ensure((size_t)mv * ldR);
-      w.tc.run(s, xh, xl, w.cot_h.get(), w.cot_l.get(), (int)mv, rows, w.Ko, Z2, ldR,
-               2.0 * mv * rows * no, 1, false, 0, false);
+      const size_t nx = (size_t)m * Zv * w.Ko, nz = (size_t)rows * m * Zv;
+      __nv_bfloat16 *xh = w.xv_h.ensure(nx), *xl = w.xv_l.ensure(nx);
+      S2G_LAUNCH(k_tcs_box, g, 256, 0, s, xh, xl, X, w.pos.get() + (int64_t)no * nv, nci, no, nv,
+                 Zv, w.Ko, m);
+      __nv_bfloat16 *zh = w.z2t_h.ensure(nz), *zl = w.z2t_l.ensure(nz);
+      w.tc.run(s, w.cot_h.get(), w.cot_l.get(), w.Ko, xh, xl, w.Ko, rows, m * Zv, no, zh, zl,
+               (int64_t)m * Zv, 2.0 * mv * rows * no);
       // G2x: U_A[(s,r), i] = sum_b Z2_A[(s,r), b] P^A_ov[i, b], batched over atoms
-      __nv_bfloat16 *zh = w.z2t_h.ensure((size_t)N * mz * w.Kv),
-                    *zl = w.z2t_l.ensure((size_t)N * mz * w.Kv);
-      S2G_CUDA(cudaMemsetAsync(zh, 0, (size_t)N * mz * w.Kv * 2, s));
-      S2G_CUDA(cudaMemsetAsync(zl, 0, (size_t)N * mz * w.Kv * 2, s));
-      S2G_LAUNCH(k_tcs_to_atom, dim3((unsigned)div_up(nv, 32), (unsigned)div_up(rows, 32), (unsigned)m),
-                 tb, 0, s, zh, zl, Z2, ldR, rows, maxa, nv, w.Kv, m);
-      U = w.U.ensure((size_t)N * bst);
-      w.tc.run(s, zh, zl, w.pov_h.get(), w.pov_l.get(), (int)mz, no, w.Kv, U, ldo,
-               2.0 * mz * no * nv, N, true, bst, false);
+      U = w.U.ensure((size_t)N * mz * ldo);
+      w.tc.run(s, zh, zl, Zv, w.pov_h.get(), w.pov_l.get(), w.Kv, (int)mz, no, nv, U, nullptr, ldo,
+               2.0 * mz * no * nv, N, true, mz * ldo);
     }
     // G3 operand: cJ T + cX U back to (i, r) rows; G3: Y[(i,r), a] = sum_R Tt Cv[R, a]
     __nv_bfloat16 *th = w.tt_h.ensure((size_t)mo * w.KR), *tl = w.tt_l.ensure((size_t)mo * w.KR);
-    S2G_CUDA(cudaMemsetAsync(th, 0, (size_t)mo * w.KR * 2, s));
-    S2G_CUDA(cudaMemsetAsync(tl, 0, (size_t)mo * w.KR * 2, s));
     S2G_LAUNCH(k_tcs_from_atom, dim3((unsigned)div_up(no, 32), (unsigned)div_up(rows, 32), (unsigned)m),
-               tb, 0, s, th, tl, T, U, bst, ldo, rows, maxa, no, w.KR, m, cJ, cX);
+               tb, 0, s, th, tl, T, U, ldo, rows, no, w.KR, m, cJ, cX);
     float *Y = w.Y.ensure((size_t)mo * ldv);
-    w.tc.run(s, th, tl, w.cv2_h.get(), w.cv2_l.get(), (int)mo, nv, w.KR, Y, ldv,
-             2.0 * mo * nv * rows, 1, false, 0, false);
+    w.tc.run(s, th, tl, w.KR, w.cv2_h.get(), w.cv2_l.get(), w.KR, (int)mo, nv, rows, Y, nullptr,
+             ldv, 2.0 * mo * nv * rows);
     if (side) S2G_CUDA(cudaStreamWaitEvent(s, w.side.join, 0));
-    S2G_LAUNCH(k_tcs_gather, g, 256, 0, s, out, Y, ldv, w.ci, w.ca, nci, no, m);
-    w.tc.check(s);
-  } else if (side) {
-    S2G_CUDA(cudaStreamWaitEvent(s, w.side.join, 0));
+    S2G_LAUNCH(k_tcs_gather, g, 256, 0, s, out, Y, ldv, w.ci, w.ca, nci, no, m, X, diag);
+    w.tc.poll(s);
+  } else {
+    if (side) S2G_CUDA(cudaStreamWaitEvent(s, w.side.join, 0));
+    if (diag) S2G_LAUNCH(k_add_diag, g, 256, 0, s, out, X, diag, nci, m);
   }
-  if (diag) S2G_LAUNCH(k_add_diag, g, 256, 0, s, out, X, diag, nci, m);
 }
 
 }  // namespace std2g

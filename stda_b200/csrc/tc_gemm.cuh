@@ -167,7 +167,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
 }
 
 // 3-D tiled TMA store (x = column, y = row, z = batch) from 128B-swizzled smem;
-// x is a multiple of 32 FP32 elements and never negative
+// x is a multiple of 32 elements (FP32: 128 bytes, BF16: 64) and never negative
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void *src, int x, int y,
                                              int z) {
   asm volatile(
@@ -239,16 +239,19 @@ struct GridTiles {
 // The TMEM accumulator is double-buffered (2 x BN columns) so that the
 // epilogue of one tile overlaps the MMAs of the next; the TMA producer runs
 // ahead across tile boundaries through the 3-stage shared-memory ring.
-// Epilogue: kDirect = false stores D[m][n] through 128B-swizzled shared
-// memory and TMA (map mD); kDirect = true writes D[out_base + n*col_stride + m]
-// from registers (the transposed layout of the PT couplings; a warp's 32 rows
-// are 128 contiguous bytes per column).
-template <class Tiles, bool kDirect, bool kF16 = false>
+// Epilogue: kOut = kOutTma stores D[m][n] through 128B-swizzled shared memory
+// and TMA (map mD); kOutDirect writes D[out_base + n*col_stride + m] from registers
+// (the transposed layout of the PT couplings; a warp's 32 rows are 128 contiguous
+// bytes per column); kOutPair stores D[m][n] as a BF16 pair (maps mD, mD2), the
+// operand form of the next product.
+enum { kOutTma = 0, kOutDirect = 1, kOutPair = 2 };
+template <class Tiles, int kOut, bool kF16 = false>
 __global__ void __launch_bounds__(256, 1)
 k_tc_gemm_bf16x3(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
                  const __grid_constant__ CUtensorMap mBh, const __grid_constant__ CUtensorMap mBl,
-                 const __grid_constant__ CUtensorMap mD, const Tiles tiles, float *D, int Kpad,
-                 int *err) {
+                 const __grid_constant__ CUtensorMap mD, const __grid_constant__ CUtensorMap mD2,
+                 const Tiles tiles, float *D, int Kpad, int *err) {
+  constexpr bool kDirect = kOut == kOutDirect;
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -392,17 +395,41 @@ k_tc_gemm_bf16x3(const __grid_constant__ CUtensorMap mAh, const __grid_constant_
           __syncwarp();
           uint32_t v[32];
           tc::tmem_ld32(tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(ab * BN + c), v);
-          // row `lane`: 16-byte chunk q goes to chunk q ^ (lane % 8) (128B swizzle)
-          unsigned char *rowp = buf + lane * 128;
+          if (kOut == kOutPair) {
+            // 64-byte rows of hi and lo: chunk q goes to q ^ (lane / 2 % 4) (64B swizzle)
+            unsigned char *rowp = buf + lane * 64;
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            uint4 w = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            *reinterpret_cast<uint4 *>(rowp + ((q ^ (lane & 7)) << 4)) = w;
+            for (int q = 0; q < 4; ++q) {
+              uint32_t hw[4], lw[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float x0 = __uint_as_float(v[8 * q + 2 * e]);
+                const float x1 = __uint_as_float(v[8 * q + 2 * e + 1]);
+                const __nv_bfloat162 hh = __floats2bfloat162_rn(x0, x1);
+                const __nv_bfloat162 ll = __floats2bfloat162_rn(x0 - __low2float(hh),
+                                                                x1 - __high2float(hh));
+                hw[e] = *reinterpret_cast<const uint32_t *>(&hh);
+                lw[e] = *reinterpret_cast<const uint32_t *>(&ll);
+              }
+              unsigned char *at = rowp + ((q ^ ((lane >> 1) & 3)) << 4);
+              *reinterpret_cast<uint4 *>(at) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+              *reinterpret_cast<uint4 *>(at + EPI_BUF / 2) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+            }
+          } else {
+            // row `lane`: 16-byte chunk q goes to chunk q ^ (lane % 8) (128B swizzle)
+            unsigned char *rowp = buf + lane * 128;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              uint4 w = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+              *reinterpret_cast<uint4 *>(rowp + ((q ^ (lane & 7)) << 4)) = w;
+            }
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) {
             tc::tma_store_3d(&mD, buf, tl.n0 + c, tl.m0 + wq * 32, tl.z);
+            if (kOut == kOutPair)
+              tc::tma_store_3d(&mD2, buf + EPI_BUF / 2, tl.n0 + c, tl.m0 + wq * 32, tl.z);
             tc::bulk_commit();
           }
         }
@@ -446,12 +473,11 @@ struct TcGemm {
   PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   DBuf<int> err;
   bool ready = false;
-  double ms = 0, flop = 0;
+  double flop = 0;
   int64_t launches = 0;
   bool armed = false;
   int nsm = 148;
   int max_ctas = 0;   // > 0: at most this many persistent CTAs (SMs shared with other work)
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
 
   void init() {
     if (ready) return;
@@ -461,22 +487,23 @@ struct TcGemm {
     if (!fn || q != cudaDriverEntryPointSuccess)
       throw Error{STD2G_ECUDA, "cuTensorMapEncodeTiled unavailable"};
     encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-    S2G_CUDA(cudaFuncSetAttribute(k_tc_gemm_bf16x3<GridTiles, false>,
+    S2G_CUDA(cudaFuncSetAttribute(k_tc_gemm_bf16x3<GridTiles, kOutTma>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES));
-    S2G_CUDA(cudaEventCreate(&e0));
-    S2G_CUDA(cudaEventCreate(&e1));
+    S2G_CUDA(cudaFuncSetAttribute(k_tc_gemm_bf16x3<GridTiles, kOutPair>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES));
     int dev = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     S2G_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     ready = true;
   }
 
-  // rows x Kpad BF16 matrices, `batch` of them `rows*Kpad` elements apart
-  CUtensorMap map(const void *p, int64_t rows, int Kpad, int box_rows, int batch = 1,
+  // rows x K BF16 matrices of row pitch `pitch` (a multiple of 8), `batch` of them
+  // rows*pitch elements apart; elements from K on read as zeros
+  CUtensorMap map(const void *p, int64_t rows, int K, int pitch, int box_rows, int batch = 1,
                   CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16) {
     CUtensorMap m;
-    cuuint64_t dims[3] = {(cuuint64_t)Kpad, (cuuint64_t)rows, (cuuint64_t)batch};
-    cuuint64_t strides[2] = {(cuuint64_t)Kpad * 2, (cuuint64_t)rows * Kpad * 2};
+    cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)batch};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)rows * pitch * 2};
     cuuint32_t box[3] = {(cuuint32_t)tc::BK, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = encode(&m, dt, 3, (void *)p, dims, strides, box,
@@ -504,26 +531,46 @@ struct TcGemm {
     return m;
   }
 
-  // D (M x N, row-major ldd) = A (M x Kpad) B (N x Kpad)^T, split-BF16 operands,
-  // for `batch` independent problems (A, D batched; B batched when b_batched).
-  // nflop: algorithmic FLOPs credited to this launch (2 M N K_true per problem).
-  void run(cudaStream_t s, const __nv_bfloat16 *Ah, const __nv_bfloat16 *Al,
-           const __nv_bfloat16 *Bh, const __nv_bfloat16 *Bl, int M, int N, int Kpad, float *D,
-           int64_t ldd, double nflop, int batch = 1, bool b_batched = false,
-           int64_t bstride_d = 0, bool sync = true) {
+  // BF16 output (rows x cols, pitch a multiple of 8) stored in 32 x 32 blocks from
+  // 64B-swizzled smem
+  CUtensorMap map_pair(__nv_bfloat16 *p, int64_t rows, int64_t cols, int64_t pitch) {
+    CUtensorMap m;
+    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)rows * pitch * 2};
+    cuuint32_t box[3] = {(cuuint32_t)tc::EPI_COLS, 32, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)p, dims, strides, box,
+                        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+      throw Error{STD2G_ECUDA, "cuTensorMapEncodeTiled (pair) failed " + std::to_string((int)r)};
+    return m;
+  }
+
+  // D (M x N, row-major ldd) = A (M x K, pitch pa) B (N x K, pitch pb)^T, split-BF16
+  // operands, for `batch` independent problems (A, D batched; B batched when b_batched).
+  // Dl == NULL: D is FP32; else D and Dl are the BF16 halves of the result (batch 1).
+  // nflop: algorithmic FLOPs credited to this launch (2 M N K per problem).  No
+  // synchronisation: the wait status is read by the next poll() / check().
+  void run(cudaStream_t s, const __nv_bfloat16 *Ah, const __nv_bfloat16 *Al, int pa,
+           const __nv_bfloat16 *Bh, const __nv_bfloat16 *Bl, int pb, int M, int N, int K, void *D,
+           __nv_bfloat16 *Dl, int64_t ldd, double nflop, int batch = 1, bool b_batched = false,
+           int64_t bstride_d = 0) {
     init();
     if (M <= 0 || N <= 0) return;
-    if (Kpad % tc::BK != 0) throw Error{STD2G_EINVAL, "tc_gemm: K not padded to 64"};
+    if (K < 1 || (pa | pb) % 8 != 0 || K > pa || K > pb)
+      throw Error{STD2G_EINVAL, "tc_gemm: operand pitch"};
     if (((uintptr_t)Ah | (uintptr_t)Al | (uintptr_t)Bh | (uintptr_t)Bl) & 15)
       throw Error{STD2G_EINVAL, "tc_gemm: operands not 16-byte aligned"};
-    if ((ldd % 4) != 0 || ((uintptr_t)D & 15))
+    if ((ldd % (Dl ? 8 : 4)) != 0 || (((uintptr_t)D | (uintptr_t)Dl) & 15))
       throw Error{STD2G_EINVAL, "tc_gemm: output not 16-byte aligned"};
     if (batch < 1 || batch > 65535) throw Error{STD2G_EINVAL, "tc_gemm: bad batch"};
-    if (batch > 1 && ((bstride_d % 4) != 0)) throw Error{STD2G_EINVAL, "tc_gemm: batch stride"};
-    CUtensorMap ah = map(Ah, M, Kpad, tc::BM, batch), al = map(Al, M, Kpad, tc::BM, batch);
-    CUtensorMap bh = map(Bh, N, Kpad, tc::BN, b_batched ? batch : 1);
-    CUtensorMap bl = map(Bl, N, Kpad, tc::BN, b_batched ? batch : 1);
-    CUtensorMap dm = map_out(D, M, N, ldd, batch, batch > 1 ? bstride_d : (int64_t)M * ldd);
+    if (batch > 1 && (Dl || (bstride_d % 4) != 0))
+      throw Error{STD2G_EINVAL, "tc_gemm: batch stride"};
+    CUtensorMap ah = map(Ah, M, K, pa, tc::BM, batch), al = map(Al, M, K, pa, tc::BM, batch);
+    CUtensorMap bh = map(Bh, N, K, pb, tc::BN, b_batched ? batch : 1);
+    CUtensorMap bl = map(Bl, N, K, pb, tc::BN, b_batched ? batch : 1);
+    const int Kpad = (int)div_up(K, tc::BK) * tc::BK;
     int *e = err.ensure(1);
     if (!armed) {
       S2G_CUDA(cudaMemsetAsync(e, 0, sizeof(int), s));
@@ -532,19 +579,19 @@ struct TcGemm {
     const int64_t ntiles = div_up(N, tc::BN) * div_up(M, tc::BM) * (int64_t)batch;
     const int cap = max_ctas > 0 ? std::min(max_ctas, nsm) : nsm;
     const int grid = (int)std::min<int64_t>(ntiles, cap);
-    if (sync) S2G_CUDA(cudaEventRecord(e0, s));
     const GridTiles tiles{M, N, batch, b_batched ? 1 : 0};
-    S2G_LAUNCH((k_tc_gemm_bf16x3<GridTiles, false>), grid, 256, tc::SMEM_BYTES, s, ah, al, bh, bl,
-               dm, tiles, (float *)nullptr, Kpad, e);
+    if (Dl) {
+      CUtensorMap dh = map_pair((__nv_bfloat16 *)D, M, N, ldd), dl = map_pair(Dl, M, N, ldd);
+      S2G_LAUNCH((k_tc_gemm_bf16x3<GridTiles, kOutPair>), grid, 256, tc::SMEM_BYTES, s, ah, al, bh,
+                 bl, dh, dl, tiles, (float *)nullptr, Kpad, e);
+    } else {
+      CUtensorMap dm =
+          map_out((float *)D, M, N, ldd, batch, batch > 1 ? bstride_d : (int64_t)M * ldd);
+      S2G_LAUNCH((k_tc_gemm_bf16x3<GridTiles, kOutTma>), grid, 256, tc::SMEM_BYTES, s, ah, al, bh,
+                 bl, dm, dm, tiles, (float *)nullptr, Kpad, e);
+    }
     ++launches;
     flop += nflop * batch;
-    if (sync) {
-      S2G_CUDA(cudaEventRecord(e1, s));
-      check(s);
-      float t = 0;
-      S2G_CUDA(cudaEventElapsedTime(&t, e0, e1));
-      ms += t;
-    }
   }
 
   // D[tile.out_base + n*tile.col_stride + m] for the tiles of `tiles` (a
@@ -565,12 +612,14 @@ struct TcGemm {
     if (a_rows >= (int64_t)1 << 31 || b_rows >= (int64_t)1 << 31)
       throw Error{STD2G_EINVAL, "tc_gemm: operand rows beyond the TMA coordinate range"};
     // per device and instantiation; a cheap host call, made every time
-    S2G_CUDA(cudaFuncSetAttribute(k_tc_gemm_bf16x3<Tiles, true, kF16>,
+    S2G_CUDA(cudaFuncSetAttribute(k_tc_gemm_bf16x3<Tiles, kOutDirect, kF16>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES));
     const CUtensorMapDataType dt =
         kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    CUtensorMap ah = map(Ah, a_rows, Kpad, tc::BM, 1, dt), al = map(Al, a_rows, Kpad, tc::BM, 1, dt);
-    CUtensorMap bh = map(Bh, b_rows, Kpad, tc::BN, 1, dt), bl = map(Bl, b_rows, Kpad, tc::BN, 1, dt);
+    CUtensorMap ah = map(Ah, a_rows, Kpad, Kpad, tc::BM, 1, dt),
+                al = map(Al, a_rows, Kpad, Kpad, tc::BM, 1, dt);
+    CUtensorMap bh = map(Bh, b_rows, Kpad, Kpad, tc::BN, 1, dt),
+                bl = map(Bl, b_rows, Kpad, Kpad, tc::BN, 1, dt);
     int *e = err.ensure(1);
     if (!armed) {
       S2G_CUDA(cudaMemsetAsync(e, 0, sizeof(int), s));
@@ -578,21 +627,44 @@ struct TcGemm {
     }
     const int cap = max_ctas > 0 ? std::min(max_ctas, nsm) : nsm;
     const int grid = (int)std::min<int64_t>(ntiles, cap);
-    S2G_LAUNCH((k_tc_gemm_bf16x3<Tiles, true, kF16>), grid, 256, tc::SMEM_BYTES, s, ah, al, bh,
-               bl, ah, tiles, D, Kpad, e);
+    S2G_LAUNCH((k_tc_gemm_bf16x3<Tiles, kOutDirect, kF16>), grid, 256, tc::SMEM_BYTES, s, ah, al, bh,
+               bl, ah, ah, tiles, D, Kpad, e);
     ++launches;
     flop += nflop;
+  }
+
+  // error flag as of the last poll() of this stream that the GPU has passed; no wait
+  int *h_err = nullptr;
+  TcGemm() = default;
+  TcGemm(const TcGemm &) = delete;
+  TcGemm &operator=(const TcGemm &) = delete;
+  ~TcGemm() {
+    if (h_err) cudaFreeHost(h_err);
+  }
+  [[noreturn]] void expired(int code) {
+    throw Error{STD2G_ETIMEOUT, "tc_gemm: bounded wait expired (" + std::to_string(code) + ")"};
+  }
+  // between products of an iteration: reports an expired wait of an earlier one as soon
+  // as the host can see it; the caller ends with check()
+  void poll(cudaStream_t s) {
+    if (!armed) return;
+    if (!h_err) {
+      S2G_CUDA(cudaMallocHost(&h_err, sizeof(int)));
+      *h_err = 0;
+    }
+    if (*(volatile int *)h_err) check(s);
+    S2G_CUDA(cudaMemcpyAsync(h_err, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
   }
 
   // read the error flag of the launches since the last check (synchronises)
   void check(cudaStream_t s) {
     if (!armed) return;
-    int h_err = 0;
-    S2G_CUDA(cudaMemcpyAsync(&h_err, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    int code = 0;
+    S2G_CUDA(cudaMemcpyAsync(&code, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
     armed = false;
-    if (h_err)
-      throw Error{STD2G_ETIMEOUT, "tc_gemm: bounded wait expired (" + std::to_string(h_err) + ")"};
+    if (h_err) *h_err = 0;
+    if (code) expired(code);
   }
 };
 
