@@ -90,7 +90,7 @@ struct Ctx {
   MixedWork mixed;
   struct RespWork {
     DBuf<float> Apb32, Amb32, dp, dm;
-    DBuf<double> B1, U, V, PU, MV, R1, R2, pa, pb, wcol, rz, alpha, beta, rr, nrm, nrm2, dmf, dpd,
+    DBuf<double> B1, U, V, PU, MV, R1, R2, pa, pb, wcol, rz, pq, rr, nrm, nrm2, dmf, dpd,
         dmd;
     DBuf<char> vecs[12];
     DBuf<unsigned> flag;
@@ -603,6 +603,7 @@ static void response_ir(Ctx &c, int n, const double *musel, const RespReq &rq,
   S2G_CUDA(cudaMemsetAsync(U, 0, sizeof(double) * nc, s));
   S2G_CUDA(cudaMemsetAsync(V, 0, sizeof(double) * nc, s));
   const dim3 rgrid(kRespSplit, (unsigned)ncol);
+  const dim3 dgrid((unsigned)std::min<int64_t>(div_up(n, 512), 128), (unsigned)ncol);
   const int sgrid = (int)div_up(ncol, 32);
   auto coldot64 = [&](const double *a, const double *b, double *out) {
     S2G_LAUNCH(k_resp_dot64, rgrid, 256, 0, s, a, b, n, pa);
@@ -616,25 +617,24 @@ static void response_ir(Ctx &c, int n, const double *musel, const RespReq &rq,
   for (int q = 0; q < 12; ++q) vec[q] = (T *)w.vecs[q].ensure(nc * sizeof(T));
   T *yu = vec[0], *yv = vec[1], *ru = vec[2], *rv = vec[3], *zu = vec[4], *zv = vec[5],
     *pu = vec[6], *pv = vec[7], *qu = vec[8], *qv = vec[9], *cu = vec[10], *cv = vec[11];
-  double *rz = w.rz.ensure(ncol), *al = w.alpha.ensure(ncol), *be = w.beta.ensure(ncol),
-         *rr = w.rr.ensure(ncol);
+  double *rz = w.rz.ensure(2 * ncol), *rr = w.rr.ensure(ncol);
+  double *pq = w.pq.ensure((size_t)ncol * kRespSplit);
   unsigned *flag = w.flag.ensure(1);
   S2G_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), s));
   auto pcg = [&]() {
     S2G_LAUNCH((k_pcg2_init<T, D>), rgrid, 256, 0, s, yu, yv, ru, rv, zu, zv, pu, pv, cu, cv, dp,
                dm, wcol, n, pa, pb);
-    S2G_LAUNCH(k_pcg_beta, sgrid, 32, 0, s, pa, pb, kRespSplit, ncol, rz, be, rr, 1);
+    S2G_LAUNCH(k_pcg_init_sums, sgrid, 32, 0, s, pa, pb, ncol, rz, rr);
     std::vector<double> rr0(ncol), rrn(ncol);
     S2G_CUDA(cudaMemcpyAsync(rr0.data(), rr, sizeof(double) * ncol, cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
     for (int it = 1; it <= kMaxInner; ++it) {
       inner(pu, pv, qu, qv);
-      S2G_LAUNCH(k_pcg2_pq<T>, rgrid, 256, 0, s, qu, qv, pu, pv, wcol, n, pa);
-      S2G_LAUNCH(k_pcg_alpha, sgrid, 32, 0, s, pa, kRespSplit, ncol, rz, al, flag);
+      S2G_LAUNCH(k_pcg2_pq<T>, rgrid, 256, 0, s, qu, qv, pu, pv, wcol, n, pq);
+      double *rz0 = rz + (it - 1) % 2 * ncol, *rz1 = rz + it % 2 * ncol;
       S2G_LAUNCH((k_pcg2_update<T, D>), rgrid, 256, 0, s, yu, yv, ru, rv, zu, zv, pu, pv, qu, qv,
-                 dp, dm, wcol, al, n, pa, pb);
-      S2G_LAUNCH(k_pcg_beta, sgrid, 32, 0, s, pa, pb, kRespSplit, ncol, rz, be, rr, 0);
-      S2G_LAUNCH(k_pcg2_dir<T>, g, 256, 0, s, pu, pv, zu, zv, be, n, ncol);
+                 dp, dm, wcol, rz0, pq, flag, n, pa, pb);
+      S2G_LAUNCH(k_pcg2_dir<T>, dgrid, 256, 0, s, pu, pv, zu, zv, pa, pb, rz0, rz1, rr, n);
       ++w.inner;
       if (it % 8 == 0) {
         S2G_CUDA(cudaMemcpyAsync(rrn.data(), rr, sizeof(double) * ncol, cudaMemcpyDeviceToHost,

@@ -140,7 +140,20 @@ __global__ void k_resp_accum(double *__restrict__ U, double *__restrict__ V,
 // ---- preconditioned CG on the 2n system, ncol independent systems in lockstep ----
 // Vectors (type T: FP32 for the dense mixed form, FP64 for the matrix-free
 // form) come in halves (u, v), each n x ncol column-major.  Scalars per column
-// (FP64): rz, alpha, beta, rr; flag: bit j set on negative curvature.
+// (FP64): rz (two buffers, old and new), rr; flag: bit j set on negative curvature.
+// A step is the products and three kernels: the scalars of a column are formed from the
+// partial sums by every block that needs them (two single-block kernels in between took
+// 5 us each of the 45 us of a step of 900 CSFs).
+
+// part[0] + part[1] + ... of one column, in order; the loads go out together
+__device__ __forceinline__ double resp_part_sum(const double *__restrict__ part) {
+  double v[kRespSplit], s = 0.0;
+#pragma unroll
+  for (int b = 0; b < kRespSplit; ++b) v[b] = part[b];
+#pragma unroll
+  for (int b = 0; b < kRespSplit; ++b) s += v[b];
+  return s;
+}
 
 // z = P r with P the inverse of the 2x2 blocks [[p, -w], [-w, m]]
 template <typename T, typename D>
@@ -214,35 +227,27 @@ __global__ void k_pcg2_pq(T *__restrict__ qu, T *__restrict__ qv, const T *__res
   if (threadIdx.x == 0) part[(int64_t)j * gridDim.x + blockIdx.x] = s;
 }
 
-// alpha_j = rz_j / pq_j; 0 for a finished column, 0 and flag bit j on negative curvature
-__global__ void k_pcg_alpha(const double *__restrict__ part, int nsplit, int ncol,
-                            const double *__restrict__ rz, double *__restrict__ alpha,
-                            unsigned *__restrict__ flag) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ncol) return;
-  double pq = 0.0;
-  for (int b = 0; b < nsplit; ++b) pq += part[(int64_t)j * nsplit + b];
-  if (rz[j] == 0.0 || pq == 0.0) {   // converged (or underflowed) column: frozen
-    alpha[j] = 0.0;
-  } else if (!(pq > 0.0)) {           // negative curvature: not positive definite
-    alpha[j] = 0.0;
-    atomicOr(flag, 1u << j);
-  } else {
-    alpha[j] = rz[j] / pq;
-  }
-}
-
-// y += a p ; r -= a q ; z = P r ; partial r.z and r.r
+// y += a p ; r -= a q ; z = P r ; partial r.z and r.r, with a = rz / p.q from the
+// partial p.q: 0 for a finished column, 0 and flag bit j on negative curvature
 template <typename T, typename D>
 __global__ void k_pcg2_update(T *__restrict__ yu, T *__restrict__ yv, T *__restrict__ ru,
                               T *__restrict__ rv, T *__restrict__ zu, T *__restrict__ zv,
                               const T *__restrict__ pu, const T *__restrict__ pv,
                               const T *__restrict__ qu, const T *__restrict__ qv,
                               const D *__restrict__ dp, const D *__restrict__ dm,
-                              const double *__restrict__ wcol, const double *__restrict__ alpha,
+                              const double *__restrict__ wcol, const double *__restrict__ rz,
+                              const double *__restrict__ part_pq, unsigned *__restrict__ flag,
                               int n, double *__restrict__ part_rz, double *__restrict__ part_rr) {
   const int j = blockIdx.y;
-  const T a = (T)alpha[j], w = (T)wcol[j];
+  const double pq = resp_part_sum(part_pq + (int64_t)j * kRespSplit), rzj = rz[j];
+  double alpha = 0.0;
+  if (rzj == 0.0 || pq == 0.0) {      // converged (or underflowed) column: frozen
+  } else if (!(pq > 0.0)) {           // negative curvature: not positive definite
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(flag, 1u << j);
+  } else {
+    alpha = rzj / pq;
+  }
+  const T a = (T)alpha, w = (T)wcol[j];
   const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
   const int64_t i0 = chunk * blockIdx.x, i1 = min((int64_t)n, i0 + chunk);
   double srz = 0.0, srr = 0.0;
@@ -270,31 +275,32 @@ __global__ void k_pcg2_update(T *__restrict__ yu, T *__restrict__ yv, T *__restr
   }
 }
 
-// rz_new, beta = rz_new / rz, rr; with init != 0 only rz and rr are set
-__global__ void k_pcg_beta(const double *__restrict__ part_rz, const double *__restrict__ part_rr,
-                           int nsplit, int ncol, double *__restrict__ rz, double *__restrict__ beta,
-                           double *__restrict__ rr, int init) {
+// rz, rr of the first residual
+__global__ void k_pcg_init_sums(const double *__restrict__ part_rz,
+                                const double *__restrict__ part_rr, int ncol,
+                                double *__restrict__ rz, double *__restrict__ rr) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ncol) return;
-  double a = 0.0, b = 0.0;
-  for (int q = 0; q < nsplit; ++q) {
-    a += part_rz[(int64_t)j * nsplit + q];
-    b += part_rr[(int64_t)j * nsplit + q];
-  }
-  if (!init) beta[j] = rz[j] != 0.0 ? a / rz[j] : 0.0;
-  rz[j] = a;
-  rr[j] = b;
+  rz[j] = resp_part_sum(part_rz + (int64_t)j * kRespSplit);
+  rr[j] = resp_part_sum(part_rr + (int64_t)j * kRespSplit);
 }
 
-// p = z + beta p, both halves
+// rz_new, rr; p = z + beta p, both halves, beta = rz_new / rz; grid (any, ncol)
 template <typename T>
 __global__ void k_pcg2_dir(T *__restrict__ pu, T *__restrict__ pv, const T *__restrict__ zu,
-                           const T *__restrict__ zv, const double *__restrict__ beta, int n,
-                           int ncol) {
-  const int64_t total = (int64_t)n * ncol;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const T b = (T)beta[t / n];
+                           const T *__restrict__ zv, const double *__restrict__ part_rz,
+                           const double *__restrict__ part_rr, const double *__restrict__ rz,
+                           double *__restrict__ rz_new, double *__restrict__ rr, int n) {
+  const int j = blockIdx.y;
+  const double a = resp_part_sum(part_rz + (int64_t)j * kRespSplit), old = rz[j];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    rz_new[j] = a;
+    rr[j] = resp_part_sum(part_rr + (int64_t)j * kRespSplit);
+  }
+  const T b = (T)(old != 0.0 ? a / old : 0.0);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = i + (int64_t)n * j;
     pu[t] = zu[t] + b * pu[t];
     pv[t] = zv[t] + b * pv[t];
   }
