@@ -180,13 +180,12 @@ inline void mf_setup_ops(MatFree &mf, cudaStream_t s, const double *Clow, const 
 // out (nci x m) = cK (K X) + cJ (J X) + cX (Kx X) + diag o X  (diag may be NULL).
 // Seven launches for A X: a block of 25 vectors of a 60-atom molecule is bound by
 // their latency.  The atoms' products work in place in an array over all AOs
-// (DgSplitCols), where two transposes moved both arrays.  For large molecules that
-// array is [AO][orbital] with one product per vector: every load and store of the
-// atoms' products is contiguous (336 products 432 x 248 x 432: 2.10 -> 1.2 ms; 50
-// vectors of C294H42 7 % faster, alpha(w) of a 200-atom chain 5 %).  That needs `no`
-// (and `nv`) to fill the 64-row tiles to 87 %.  Below 160 occupied orbitals (112:
-// no difference), and where the sums are to be split as before (wave_splits), it is
-// [orbital][AO] over all vectors at once, whose runs are the 4 to 9 AOs of an atom.
+// (DgSplitCols), where two transposes moved both arrays.  That array is [AO][orbital],
+// with one product per vector around it, so that every load and store of the atoms'
+// products is contiguous.  Where the sums are to be split as before (wave_splits) it is
+// [orbital][AO] over all vectors at once, whose runs are the 4 to 9 AOs of an atom: 336
+// products 432 x 248 x 432 take 2.10 ms on those and 1.2 on contiguous ones, alpha(w) of
+// 57 atoms 10.1 and 9.05, of a 200-atom chain 34.3 and 32.9 ms, 20 and 61 atoms the same.
 inline void mf_apply(MatFree &mf, cudaStream_t s, const double *X, int m, double *out, double cK,
                      double cJ, double cX, const double *diag) {
   const int N = mf.N, maxa = mf.maxa, no = mf.no, nv = mf.nv, nci = mf.nci;
@@ -207,9 +206,7 @@ inline void mf_apply(MatFree &mf, cudaStream_t s, const double *X, int m, double
     double *Z = mf.Z.ensure((size_t)std::max((int64_t)lr * std::max(no, nv),
                                              (int64_t)rows * std::max(lo, lv)) * m);
     double *Tacc = mf.Tacc.ensure((size_t)std::max((int64_t)lr * no, (int64_t)rows * lo) * m);
-    const auto fills = [](int n) { return div_up(n, dg::BM) * dg::BM * 87 <= 100 * (int64_t)n; };
-    const bool by_ao =
-        !dg.wave_splits && no >= 160 && fills(no) && (cX == 0.0 || fills(nv));
+    const bool by_ao = !dg.wave_splits;
     const int64_t so = (int64_t)(by_ao ? rows : lr) * (by_ao ? lo : no);   // one vector of Tacc
     double beta = 0.0;
     if (cJ != 0.0) {

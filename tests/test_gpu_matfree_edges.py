@@ -30,10 +30,9 @@ def test_roots(natoms, ethr, nroots, ax, rpa):
 
 @pytest.mark.parametrize("natoms,ethr", [(99, 6.5), (108, 6.5)])
 def test_by_ao_form(natoms, ethr):
-    """More than 160 occupied orbitals that fill the tiles (189 and 187; 109 and 116
-    virtual ones, of which only the latter fill theirs): roots and alpha(w) against the
-    engine's explicit matrices.  Roots to the residual bound, alpha as the other
-    matrix-free tests."""
+    """Several tiles of occupied (189 and 187) and virtual orbitals (109 and 116): roots
+    and alpha(w) against the engine's explicit matrices.  Roots to the residual
+    bound, alpha as the other matrix-free tests."""
     from stda_b200 import synth
     from stda_b200.engine import Engine, Keywords, boundary_inputs
     mol, ints = synth.random_molecule(natoms, seed=61 + natoms, with_ints=True)
