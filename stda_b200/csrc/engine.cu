@@ -320,10 +320,16 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
     double *stat = c.w_ns.ensure(2), h[2];
     S2G_CUDA(cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns_small_smem(kNsSmallMax)));
+    if (c.dg.timed) c.dg.mark(s);
     S2G_LAUNCH(k_ns_small, 1, kNsThreads, ns_small_smem(n), s, S, n, out, stat);
+    if (c.dg.timed) c.dg.mark(s);
     S2G_CUDA(cudaMemcpyAsync(h, stat, sizeof(h), cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
     c.ns_iters = (int)h[1];
+    // the products that the kernel formed: one, then three per step but the last's Z
+    const int products = 3 * (c.ns_iters - 1);
+    c.dg.calls += products;
+    c.dg.flop += 2.0 * n * (double)nn * products;
     fail(h[0]);
     return;
   }
