@@ -379,6 +379,42 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
   S2G_LAUNCH(k_scale_copy, grid_for((int64_t)nn), 256, 0, s, out, Y, (int64_t)nn, std::sqrt(cmax));
 }
 
+// (A-B)^1/2 of a dense sTD-DFT matrix of at most kSymEigMaxN CSFs by the same iteration
+// as S^1/2, instead of all eigenpairs through syevd: with the roots on the engine's
+// eigensolver too, 10 roots of a 12-atom cluster 6.27 -> 2.13 ms per load and solve.  False, with `out` undefined, when the iteration does not converge or Y Y
+// misses A by more than rounding (64 eps of the largest element; this form leaves 4 to 27
+// eps for n = 30 to 320, an eigen-decomposition 8 to 20): near-singular and indefinite
+// matrices, which the caller's eigen-decomposition decides.
+// R: n x n scratch.
+static bool sqrt_small(Ctx &c, const double *A, int n, double *out, double *R) {
+  cudaStream_t s = c.stream;
+  const size_t nn = (size_t)n * n;
+  const int iters = c.ns_iters;
+  const bool waves = c.dg.wave_splits;
+  c.dg.wave_splits = false;   // symmetric products
+  bool ok = true;
+  try {
+    sqrt_overlap(c, A, n, out);
+  } catch (const Error &e) {
+    c.dg.wave_splits = waves;
+    if (e.code != STD2G_ES_NOT_PD) throw;
+    ok = false;
+  }
+  c.dg.wave_splits = waves;
+  c.ns_iters = iters;
+  if (!ok) return false;
+  S2G_CUDA(cudaMemcpyAsync(R, A, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
+  gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, 1.0, out, n, out, n, -1.0, R, n);
+  auto *flags = (unsigned long long *)c.w_ns.ensure(2);
+  S2G_CUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(unsigned long long), s));
+  S2G_LAUNCH(k_abs_max, grid_for((int64_t)nn), 256, 0, s, R, (int64_t)nn, flags);
+  S2G_LAUNCH(k_abs_max, grid_for((int64_t)nn), 256, 0, s, A, (int64_t)nn, flags + 1);
+  double h[2];
+  S2G_CUDA(cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, s));
+  S2G_CUDA(cudaStreamSynchronize(s));
+  return h[0] <= 64 * 2.220446049250313e-16 * h[1];
+}
+
 static uint64_t fnv1a(const std::vector<int> &a, const std::vector<int> &b) {
   uint64_t h = 1469598103934665603ull;
   for (size_t k = 0; k < a.size(); ++k) {
@@ -1788,22 +1824,28 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
     record(c, PH_EIGEN);
     // (A-B)^1/2 (smatpow srpapack.f:201-256)
     double *U = c.w_Ambh.ensure(n2);
-    S2G_CUDA(cudaMemcpyAsync(U, Amb, sizeof(double) * n2, cudaMemcpyDeviceToDevice, s));
-    double *w = c.w_eval.ensure(std::max(nci, nao));
-    dense_eig_full(c, U, nci, w);
-    double wmin = 0;
-    S2G_CUDA(cudaMemcpyAsync(&wmin, w, sizeof(double), cudaMemcpyDeviceToHost, s));
-    S2G_CUDA(cudaStreamSynchronize(s));
-    if (wmin < 0) throw Error{STD2G_EAMB_NOT_PD, "matrix power impossible (A-B)"};
     double *Ambh = c.w_M.ensure(n2);
     double *tmp2 = c.w_Kx.ensure(n2);   // Kx no longer needed
-    sym_sqrt(c, U, w, nci, Ambh, tmp2);
+    const bool small = nci <= kSymEigMaxN;
+    if (!small || !sqrt_small(c, Amb, nci, Ambh, U)) {
+      S2G_CUDA(cudaMemcpyAsync(U, Amb, sizeof(double) * n2, cudaMemcpyDeviceToDevice, s));
+      double *w = c.w_eval.ensure(std::max(nci, nao));
+      dense_eig_full(c, U, nci, w);
+      double wmin = 0;
+      S2G_CUDA(cudaMemcpyAsync(&wmin, w, sizeof(double), cudaMemcpyDeviceToHost, s));
+      S2G_CUDA(cudaStreamSynchronize(s));
+      if (wmin < 0) throw Error{STD2G_EAMB_NOT_PD, "matrix power impossible (A-B)"};
+      sym_sqrt(c, U, w, nci, Ambh, tmp2);
+    }
     // M = (A-B)^1/2 (A+B) (A-B)^1/2 (srpapack.f:58-71)
     gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, nci, nci, nci, 1.0, Apb, nci, Ambh, nci, 0.0, tmp2, nci);
     double *Mm = U;
     gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, nci, nci, nci, 1.0, Ambh, nci, tmp2, nci, 0.0, Mm, nci);
     om = c.w_eval.ensure(std::max(nci, nao));
-    nroot = dense_eig(c, Mm, nci, 0.0, thr * thr, p.nroots, om);
+    if (small)
+      nroot = dense_window_small(c, Mm, nci, 0.0, thr * thr, p.nroots, om, c.w_Ares, Mm);
+    else
+      nroot = dense_eig(c, Mm, nci, 0.0, thr * thr, p.nroots, om);
     if (nroot < 1) throw Error{STD2G_ENOROOT, "RPA diag failed"};
     S2G_LAUNCH(k_sqrt_inplace, (int)div_up(nroot, 128), 128, 0, s, om, nroot);
     // X+Y = (A-B)^1/2 Z / sqrt(w); X-Y = (A+B)(X+Y)/w (srpapack.f:108-143)
