@@ -1,6 +1,6 @@
 """FP64 CPU oracle of std2's sTDA / sTD-DFT path (TEST INFRASTRUCTURE ONLY).
 
-This module is the checker for the CUDA engine.  Only ``tests/``,
+This module is the oracle for the CUDA engine.  Only ``tests/``,
 ``__graft_entry__.smoke()`` and ``bench.py``'s CPU-baseline leg may import
 it; the engine itself never calls it.  It restates, in double precision and
 numpy, what ``SUBROUTINE stda`` (``stda.f:53-1606``) does between the AO
