@@ -547,6 +547,20 @@ __host__ __device__ inline size_t symeig_vec_smem_bytes(int n) {
   return sizeof(double) * (2 * np + (size_t)kSymEigWarps * 6 * np);
 }
 
+// Entry i of member m's start vector: +-[1/2, 1), from a hash of (i, m) that mixes
+// the two through products.  The start vectors of a cluster of equal eigenvalues have
+// to be independent of each other, since the Gram-Schmidt steps keep only what is new
+// in each: exclusive-or and shifts of one function of i and one of m span 17
+// directions, and a 150-fold eigenvalue of 2 x 2 blocks got dependent vectors.
+__device__ __forceinline__ double symeig_start(int i, int m) {
+  unsigned h = (unsigned)(i + 1) * 0x9E3779B1u + (unsigned)(m + 1) * 0x85EBCA77u;
+  h = (h ^ h >> 16) * 0x9E3779B1u;
+  h = (h ^ h >> 15) * 0x85EBCA77u;
+  h ^= h >> 16;
+  const double v = 0.5 + (double)(h >> 1) * 0x1p-32;
+  return h & 1 ? v : -v;
+}
+
 __device__ __forceinline__ void
 symeig_vectors_body(int n, int k, double *__restrict__ work, const double *__restrict__ w) {
   extern __shared__ __align__(16) double sm[];
@@ -600,9 +614,7 @@ symeig_vectors_body(int n, int k, double *__restrict__ work, const double *__res
       const double ia = ua[i];
       const double2 u = ub[i];
       ub[i] = make_double2(-u.x * ia, -u.y * ia);
-      // start vector: fixed, positive, no pattern
-      const unsigned h = (unsigned)(i + 1) * 0x9E3779B1u ^ (unsigned)(m + 1) * 0x85EBCA77u;
-      y[i] = (1.0 + 0.5 * (double)((h ^ h >> 15) & 0xffffu) * (1.0 / 65536.0)) * ia;
+      y[i] = symeig_start(i, m) * ia;
     }
     __syncwarp();
     for (int it = 0; it < 2; ++it) {
