@@ -254,8 +254,25 @@ symeig_tridiag_body(const double *__restrict__ A, int lda, int n, double *__rest
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
       double tc = 0.0, beta = alpha, scal = 0.0;
-      if (xn2 != 0.0) {
-        beta = -copysign(sqrt(fma(alpha, alpha, xn2)), alpha);
+      const double h2 = fma(alpha, alpha, xn2);
+      if (h2 < 1e-280) {
+        // a column below 1e-140, whose squares are lost in part or altogether (the
+        // reflector would not be orthogonal): formed from the column times 2^600;
+        // entries below 1e-300 count as zero
+        double x2 = 0.0;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) x2 = fma(v[t] * 0x1p600, v[t] * 0x1p600, x2);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x2 += __shfl_xor_sync(0xffffffffu, x2, o);
+        const double as = alpha * 0x1p600;
+        if (x2 > 1e-239) {
+          const double bs = -copysign(sqrt(fma(as, as, x2)), as);
+          beta = bs * 0x1p-600;
+          tc = (bs - as) / bs;
+          scal = 0x1p600 / (as - bs);
+        }
+      } else if (xn2 != 0.0) {
+        beta = -copysign(sqrt(h2), alpha);
         tc = (beta - alpha) / beta;
         scal = 1.0 / (alpha - beta);
       }
