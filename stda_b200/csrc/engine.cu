@@ -55,7 +55,7 @@ struct Ctx {
   int ncent = 0, nmo = 0, nao = 0;
   std::vector<double> h_eps, h_occ, h_xyz;
   AoIntsWork aoi;   // primitive list of the device AO integrals (ao_ints.cuh)
-  DBuf<double> w_dall, w_Ares, w_Rres, w_part, w_rn, w_domc;   // dense roots, residuals, dominant CSFs
+  DBuf<double> w_dall, w_zref, w_Ares, w_Rres, w_part, w_rn, w_domc;   // dense roots and vectors, residuals, dominant CSFs
   DBuf<int> w_domi;
   Dgemm dg;         // the engine's FP64 matrix products (dgemm.cuh)
   int dev_sms = 148;   // SMs of the context's device
@@ -141,37 +141,67 @@ static void record(Ctx &c, int ph) { S2G_CUDA(cudaEventRecord(c.ev[ph], c.stream
 // A (n x n) is overwritten by the eigenvectors; returns the number found.
 static void dense_eig_full(Ctx &c, double *A, int n, double *w);
 
-// The same for a TDA matrix of at most kSymEigMaxN CSFs on the engine's own
-// eigensolver (symeig_small.cuh): all eigenvalues, read back to count the window,
-// then the eigenvectors up to its upper end.  syevdx reduces such a matrix in
-// 1.0 ms and synchronises with the host several times (245 CSFs, 14 roots: 1.9 ms
-// against 0.46 here).  The vectors go to `out` (n x k), the window's roots to w.
+static int dense_eig(Ctx &c, double *A, int n, double vl, double vu, int kmax, double *w);
+
+// The same for a matrix of at most kSymEigMaxN CSFs on the engine's own
+// eigensolver (symeig_small.cuh), A intact afterwards: all eigenvalues, read back to
+// count the window, then all eigenvectors, and one refinement of the window's in that
+// basis (k_eig_refine): inverse iteration leaves them orthogonal to 1e-15 / gap only,
+// refined they are as exact as or more exact than syevdx's.  What the refinement finds also checks the
+// basis: a residual above 1e-12 ||A|| or an overlap above 1e-8 sends the matrix to
+// cuSOLVER, as do clusters of more than kCluster close eigenvalues, which one warp would
+// work off one after the other.
+// The vectors go to `out` (n x k), the window's roots to w.
 static int dense_window_small(Ctx &c, const double *A, int n, double vl, double vu, int kmax,
                               double *w, DBuf<double> &out, double *&X) {
+  constexpr int kCluster = 8;
   cudaStream_t s = c.stream;
-  const int kv = kmax > 0 ? std::min(kmax, n) : n;
-  double *all = c.w_dall.ensure(n), *work = c.w_work.ensure(symeig_work_doubles(n, kv));
-  int *info = c.w_info.ensure(1);
-  S2G_CUDA(cudaMemsetAsync(info, 0, sizeof(int), s));
-  symeig_small_values(s, A, n, n, kv, all, work);
-  int lo = 0, hi = kv;
+  auto library = [&]() {
+    X = out.ensure((size_t)n * n);
+    S2G_CUDA(cudaMemcpyAsync(X, A, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, s));
+    return dense_eig(c, X, n, vl, vu, kmax, w);
+  };
+  double *all = c.w_dall.ensure(n), *work = c.w_work.ensure(symeig_work_doubles(n, n));
+  symeig_small_values(s, A, n, n, n, all, work);
+  std::vector<double> h(n);
+  S2G_CUDA(cudaMemcpyAsync(h.data(), all, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+  S2G_CUDA(cudaStreamSynchronize(s));
+  const double norm = std::max(std::fabs(h[0]), std::fabs(h[n - 1]));
+  int run = 1, longest = 1;
+  for (int i = 0; i < n; ++i) {
+    if (!std::isfinite(h[i])) return library();
+    if (i > 0) run = h[i] - h[i - 1] <= 3e-5 * norm ? run + 1 : 1;
+    longest = std::max(longest, run);
+  }
+  if (longest > kCluster) return library();
+  int lo = 0, hi = std::min(kmax, n);
   if (kmax <= 0) {   // the eigenvalues in (vl, vu]
-    std::vector<double> h(n);
-    S2G_CUDA(cudaMemcpyAsync(h.data(), all, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    S2G_CUDA(cudaStreamSynchronize(s));
     lo = (int)(std::upper_bound(h.begin(), h.end(), vl) - h.begin());
     hi = (int)(std::upper_bound(h.begin(), h.end(), vu) - h.begin());
     if (hi <= lo) return 0;
   }
-  double *Z = out.ensure((size_t)n * hi);
-  symeig_small_vectors(s, n, hi, all, Z, n, work, info);
-  S2G_CUDA(cudaMemcpyAsync(w, all + lo, sizeof(double) * (hi - lo), cudaMemcpyDeviceToDevice, s));
-  int h_info = 0;
-  S2G_CUDA(cudaMemcpyAsync(&h_info, info, sizeof(int), cudaMemcpyDeviceToHost, s));
+  const int m = hi - lo;
+  const size_t nn = (size_t)n * n, nm = (size_t)n * m;
+  // Z, behind it the window's residuals R = A Z - Z w; G and Q; E; the maxima and the status
+  double *Z = c.w_zref.ensure(nn + 4 * nm + 3), *R = Z + nn, *G = R + nm, *E = G + 2 * nm;
+  double *Zw = Z + (size_t)n * lo;
+  auto *st = (unsigned long long *)(E + nm);
+  S2G_CUDA(cudaMemsetAsync(st, 0, 3 * sizeof(double), s));
+  symeig_small_vectors(s, n, n, all, Z, n, work, (int *)(st + 2));
+  S2G_LAUNCH(k_minus_scaled, dim3(2, (unsigned)m), 128, 0, s, R, Zw, all + lo, n);
+  gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, n, m, n, 1.0, A, n, Zw, n, 1.0, R, n);
+  gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, n, m, n, 1.0, Z, n, Zw, n, 0.0, G, n, 2, 0, R - Zw,
+       (int64_t)nm);
+  S2G_LAUNCH(k_eig_refine, m, 128, 0, s, G, G + nm, all, n, lo, E, w, st);
+  X = out.ensure(nm);
+  gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, n, m, n, 1.0, Z, n, E, n, 0.0, X, n);
+  double h_st[3];
+  S2G_CUDA(cudaMemcpyAsync(h_st, st, sizeof(h_st), cudaMemcpyDeviceToHost, s));
   S2G_CUDA(cudaStreamSynchronize(s));
-  if (h_info != 0) throw Error{STD2G_ECUDA, "eigensolve: non-finite result"};
-  X = Z + (size_t)n * lo;
-  return hi - lo;
+  int info;
+  std::memcpy(&info, h_st + 2, sizeof(int));
+  if (info != 0 || !(h_st[0] < 1e-8) || !(h_st[1] < 1e-12 * norm)) return library();
+  return m;
 }
 
 static int dense_eig(Ctx &c, double *A, int n, double vl, double vu, int kmax, double *w) {

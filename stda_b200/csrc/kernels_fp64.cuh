@@ -891,6 +891,66 @@ __global__ void k_properties(const double *__restrict__ TL, const double *__rest
   }
 }
 
+// R[:, j] = -w_j Z[:, j] (grid (any, columns)): what A Z is added to for the residuals
+__global__ void k_minus_scaled(double *__restrict__ R, const double *__restrict__ Z,
+                               const double *__restrict__ w, int n) {
+  const double f = -w[blockIdx.y];
+  const int64_t at = (int64_t)n * blockIdx.y;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    R[at + i] = f * Z[at + i];
+}
+
+// One refinement of the eigenvectors z_j, j = lo .. lo + m - 1 (m = gridDim.x), in the
+// basis of all n of them (T. Ogita, K. Aishima, Japan J. Indust. Appl. Math. 35, 1007
+// (2018)): from G[:, j] = Z^T z_j and Q[:, j] = Z^T (A z_j - w_j z_j) the coefficients
+//   E_ij = Q_ij / (l_j - l_i),  E_jj = (3 - G_jj) / 2,  z_j <- Z E[:, j],
+// l_j = w_j + Q_jj / G_jj, for which E_ij + E_ji = -G_ij: the result is orthonormal.
+// Q_ij is taken as the mean of what the columns i and j say about the pair (their
+// rounding over the gap would come back as overlap).  Pairs that the quotient would
+// turn by more than 1e-8 are closer than the rounding of Q can tell apart and are only
+// made orthogonal, E_ij = -G_ij / 2.  wout[j] = l_j, kept between the halfway points
+// to the neighbours of w_j, so that the order stays; st = {max |G - 1|, max |Q|}
+__global__ void k_eig_refine(const double *__restrict__ G, const double *__restrict__ Q,
+                             const double *__restrict__ w, int n, int lo, double *__restrict__ E,
+                             double *__restrict__ wout, unsigned long long *__restrict__ st) {
+  const int j = lo + blockIdx.x, m = gridDim.x;
+  const int64_t at = (int64_t)n * blockIdx.x;
+  const double gj = G[at + j], lj = w[j] + Q[at + j] / gj;
+  double dev = 0.0, res = 0.0;
+  auto top = [](double a, double b) { return b == b ? fmax(a, fabs(b)) : 1e300; };
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double g = G[at + i], q = Q[at + i];
+    res = top(res, q);
+    dev = top(dev, i == j ? 1.0 - gj : g);
+    if (i == j) {
+      E[at + i] = 0.5 * (3.0 - gj);
+      continue;
+    }
+    double li = w[i], qs = q;
+    if (i >= lo && i < lo + m) {   // Q_ji = Q_ij + (w_j - w_i) G_ij
+      const int64_t ati = (int64_t)n * (i - lo);
+      li += Q[ati + i] / G[ati + i];
+      qs = 0.5 * (q + fma(w[i] - w[j], g, Q[ati + j]));
+    }
+    const double gap = lj - li;
+    const bool turn = fmax(fabs(qs), fabs(fma(gap, g, qs))) <= 1e-8 * fabs(gap);
+    E[at + i] = turn && gap != 0.0 ? qs / gap : -0.5 * g;
+  }
+  if (threadIdx.x == 0) {
+    const double below = j > 0 ? 0.5 * (w[j - 1] + w[j]) : -1e300;
+    const double above = j + 1 < n ? 0.5 * (w[j] + w[j + 1]) : 1e300;
+    wout[blockIdx.x] = fmin(fmax(lj, below), above);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    dev = fmax(dev, __shfl_xor_sync(0xffffffffu, dev, o));
+    res = fmax(res, __shfl_xor_sync(0xffffffffu, res, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(st, (unsigned long long)__double_as_longlong(dev));
+    atomicMax(st + 1, (unsigned long long)__double_as_longlong(res));
+  }
+}
+
 // X[:, r] *= s[r]  (column scaling, e.g. 1/sqrt(w), 1/w)
 __global__ void k_scale_columns(double *__restrict__ X, int64_t n, int ncol,
                                 const double *__restrict__ s, int mode) {
