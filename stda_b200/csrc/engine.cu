@@ -255,6 +255,14 @@ static void sym_sqrt(Ctx &c, double *U, const double *w, int n, double *out, dou
   gemm(c, CUBLAS_OP_N, CUBLAS_OP_T, n, n, n, 1.0, tmp, n, U, n, 0.0, out, n);
 }
 
+// the products are split as usual (symmetric ones among them) while this is alive
+struct WaveSplitsOff {
+  Ctx &c;
+  const bool was;
+  explicit WaveSplitsOff(Ctx &ctx) : c(ctx), was(ctx.dg.wave_splits) { c.dg.wave_splits = false; }
+  ~WaveSplitsOff() { c.dg.wave_splits = was; }
+};
+
 // S^1/2 of the AO overlap (makel, stda.f:1615-1691) without an eigensolver:
 // with A = S / c (c = largest absolute row sum >= lambda_max, so the spectrum
 // of A lies in (0, 1]), the coupled Newton-Schulz iteration
@@ -335,19 +343,23 @@ static void sqrt_overlap_plain(Ctx &c, const double *S, int n, double *out) {
 // which the scaled steps of the plain form amplify (roots 20 times further off).
 // Converged when a step begins with max |I - Z Y| < kNsDone (it ends with the
 // square of that): then A = Y Z^-1 = Z^-2 to that accuracy, so a spectrum that is
-// not positive never gets there.  One host read after kFirst steps.
+// not positive never gets there.  The result is then held to max |Y Y - A| <
+// kNsMiss: rounding grows with the condition of S, and at this bound (largest row sum
+// over lambda_min around 5000) the Loewdin MOs of S are orthonormal to about 1e-9, as
+// far as the plain form goes with its 1e-10 (it gives up from 500 to 1000).  One host
+// read after kFirst steps.
 // Measured against the plain form: n = 220 0.83 -> 0.30 ms, 518 1.83 -> 0.76, 1584
 // 13.9 -> 5.1 ms, roots of 14 to 34 atoms 2 times closer to the dense FP64 ones.
 static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
   cudaStream_t s = c.stream;
   const size_t nn = (size_t)n * n;
-  auto fail = [&](double err) {
-    if (!(err < kNsDone))
+  auto verdict = [&](double err, double miss) {
+    if (!(err < kNsDone) || !(miss < kNsMiss))
       throw Error{STD2G_ES_NOT_PD, "S^1/2: overlap matrix not positive definite (Newton-Schulz "
                                    "did not converge)"};
   };
   if (n <= kNsSmallMax) {
-    double *stat = c.w_ns.ensure(2), h[2];
+    double *stat = c.w_ns.ensure(3), h[3];
     S2G_CUDA(cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns_small_smem(kNsSmallMax)));
     if (c.dg.timed) c.dg.mark(s);
@@ -355,18 +367,20 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
     if (c.dg.timed) c.dg.mark(s);
     S2G_CUDA(cudaMemcpyAsync(h, stat, sizeof(h), cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
-    c.ns_iters = (int)h[1];
-    // the products that the kernel formed: one, then three per step but the last's Z
-    const int products = 3 * (c.ns_iters - 1);
+    c.ns_iters = (int)h[2];
+    // the products that the kernel formed: one, then three per step but the last's Z,
+    // and the check's
+    const int products = 3 * (c.ns_iters - 1) + 1;
     c.dg.calls += products;
     c.dg.flop += 2.0 * n * (double)nn * products;
-    fail(h[0]);
+    verdict(h[0], h[1]);
     return;
   }
   double *Y = c.w_tmp.ensure(nn * 4), *Z = Y + nn, *P = Y + 2 * nn, *T = Y + 3 * nn;
   constexpr int kFirst = 8, kMax = 100;
-  auto *flags = (unsigned long long *)c.w_ns.ensure(1 + kMax);   // c, then the steps' errors
-  S2G_CUDA(cudaMemsetAsync(flags, 0, (1 + kMax) * sizeof(unsigned long long), s));
+  // c, max |Y Y - A|, then the steps' errors
+  auto *flags = (unsigned long long *)c.w_ns.ensure(2 + kMax);
+  S2G_CUDA(cudaMemsetAsync(flags, 0, (2 + kMax) * sizeof(unsigned long long), s));
   S2G_LAUNCH(k_row_abs_max, (int)div_up(n, 64), 64, 0, s, S, n, flags);
   const int sym = c.dg.lib ? 0 : -1;
   auto mult = [&](const double *L, const double *R, double *D) {
@@ -375,7 +389,7 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
   double l = kNsLow;
   S2G_LAUNCH(k_ns_first, grid_for((int64_t)nn), 256, 0, s, P, Z, S, n, ns_scale(l), flags);
   mult(P, Z, Y);
-  std::vector<unsigned long long> h(1 + kMax);
+  std::vector<unsigned long long> h(2 + kMax);
   double err = 1.0;
   int it = 0, until = kFirst;
   for (;;) {
@@ -387,26 +401,44 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
       }
       const double mu = l < 1.0 - 1e-6 ? ns_scale(l) : 1.0;
       mult(Z, Y, T);
-      S2G_LAUNCH(k_ns_scaled_step, grid_for((int64_t)nn), 256, 0, s, T, n, mu, flags + 1 + it);
+      S2G_LAUNCH(k_ns_scaled_step, grid_for((int64_t)nn), 256, 0, s, T, n, mu, flags + 2 + it);
       mult(Y, T, P);
       std::swap(Y, P);
     }
-    S2G_CUDA(cudaMemcpyAsync(h.data(), flags, sizeof(unsigned long long) * (1 + it),
+    // the check goes out with the steps, for the same host read
+    S2G_CUDA(cudaMemsetAsync(flags + 1, 0, sizeof(unsigned long long), s));
+    mult(Y, Y, P);
+    S2G_LAUNCH(k_ns_miss, grid_for((int64_t)nn), 256, 0, s, P, S, (int64_t)nn, flags, flags + 1);
+    S2G_CUDA(cudaMemcpyAsync(h.data(), flags, sizeof(unsigned long long) * (2 + it),
                              cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
     bool done = false;
     for (int q = first; q < it; ++q) {
-      std::memcpy(&err, &h[1 + q], sizeof(double));
+      std::memcpy(&err, &h[2 + q], sizeof(double));
       done = err < kNsDone || !(err < 1e6);
     }
     if (done || it >= kMax) break;
     until = std::min(kMax, it + (err < 1e-4 ? 1 : (err < 0.5 ? 2 : 3)));
   }
   c.ns_iters = 1 + it;
-  fail(err);
-  double cmax;
+  double cmax, miss;
   std::memcpy(&cmax, &h[0], sizeof(double));
+  std::memcpy(&miss, &h[1], sizeof(double));
+  verdict(err, miss);
   S2G_LAUNCH(k_scale_copy, grid_for((int64_t)nn), 256, 0, s, out, Y, (int64_t)nn, std::sqrt(cmax));
+}
+
+// The plain form for iterative sTD-DFT roots, and where it gives up the scaled one, so
+// that one overlap matrix is accepted or refused by every solve alike.
+static void sqrt_overlap_fixed(Ctx &c, const double *S, int n, double *out) {
+  try {
+    sqrt_overlap_plain(c, S, n, out);
+    return;
+  } catch (const Error &e) {
+    if (e.code != STD2G_ES_NOT_PD) throw;
+  }
+  WaveSplitsOff symmetric_products(c);
+  sqrt_overlap(c, S, n, out);
 }
 
 // (A-B)^1/2 of a dense sTD-DFT matrix of at most kSymEigMaxN CSFs by the same iteration
@@ -420,17 +452,14 @@ static bool sqrt_small(Ctx &c, const double *A, int n, double *out, double *R) {
   cudaStream_t s = c.stream;
   const size_t nn = (size_t)n * n;
   const int iters = c.ns_iters;
-  const bool waves = c.dg.wave_splits;
-  c.dg.wave_splits = false;   // symmetric products
   bool ok = true;
   try {
+    WaveSplitsOff symmetric_products(c);
     sqrt_overlap(c, A, n, out);
   } catch (const Error &e) {
-    c.dg.wave_splits = waves;
     if (e.code != STD2G_ES_NOT_PD) throw;
     ok = false;
   }
-  c.dg.wave_splits = waves;
   c.ns_iters = iters;
   if (!ok) return false;
   S2G_CUDA(cudaMemcpyAsync(R, A, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
@@ -1135,7 +1164,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
   if (c.sqrtS_kind < 1 || (sq_kind == 1 && c.sqrtS_kind == 2)) {
     double *sq = c.d_sqrtS.ensure((size_t)nao * nao);
     c.sqrtS_kind = 0;
-    if (sq_kind == 1) sqrt_overlap_plain(c, c.d_Sfull.get(), nao, sq);
+    if (sq_kind == 1) sqrt_overlap_fixed(c, c.d_Sfull.get(), nao, sq);
     else sqrt_overlap(c, c.d_Sfull.get(), nao, sq);
     c.sqrtS_kind = sq_kind;
   }

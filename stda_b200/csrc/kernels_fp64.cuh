@@ -99,9 +99,10 @@ __global__ void k_ns_scaled_step(double *__restrict__ QT, int n, double mu,
 // in shared memory (rows padded to ld = 4 or 12 mod 16 doubles: conflict-free
 // fragments), products by DMMA over the tiles on and below the diagonal (every
 // matrix here is a polynomial of A, so symmetric), each warp holding its tiles
-// in registers until all warps have read the operands.  out = sqrt(c) A Z; stat =
-// {last max |I - Z A Z|, steps}.  Latency-bound: 36 AOs 0.42 -> 0.07 ms, 72 AOs
-// 0.42 -> 0.11 ms against a launch per product and a host read every third step.
+// in registers until all warps have read the operands.  out = sqrt(c) Y with the last
+// Y = Y T; stat = {last max |I - Z Y|, max |Y Y - A|, steps}.  Latency-bound: 36 AOs
+// 0.42 -> 0.07 ms, 72 AOs 0.42 -> 0.11 ms against a launch per product and a host read
+// every third step.
 constexpr int kNsSmallMax = 96, kNsThreads = 512;
 __host__ __device__ inline int ns_small_ld(int n) {
   int ld = (n + 7) / 8 * 8;
@@ -122,6 +123,7 @@ __host__ __device__ inline double ns_scale(double &l) {
 }
 constexpr double kNsLow = 0.02;   // sqrt(smallest eigenvalue / largest row sum) expected
 constexpr double kNsDone = 1e-8;  // a step that begins below this ends at rounding
+constexpr double kNsMiss = 1e-11; // largest max |Y Y - A| of an accepted result
 
 __global__ void __launch_bounds__(kNsThreads, 1)
 k_ns_small(const double *__restrict__ S, int n, double *__restrict__ out,
@@ -229,10 +231,45 @@ k_ns_small(const double *__restrict__ S, int n, double *__restrict__ out,
       out[(int64_t)i * n + j] = out[(int64_t)j * n + i] = rc * acc[u][e];
     }
   }
-  if (tid == 0) {
-    stat[0] = err;
-    stat[1] = it;
+  // what the result misses A by (Z is not needed any more)
+  put(Z, same);
+  product(Z, Z);
+  double r = 0.0;
+#pragma unroll
+  for (int u = 0; u < MAXT; ++u) {
+    if (ti[u] >= nt) continue;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int i = 8 * ti[u] + g, j = 8 * tj[u] + 2 * t4 + e;
+      if (i < j || i >= n) continue;
+      const double d = acc[u][e] - S[(int64_t)i * n + j] / c;
+      r = fmax(r, d == d ? fabs(d) : 1e300);
+    }
   }
+  for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+  if (lane == 0) red[warp] = r;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 0; w < NW; ++w) r = fmax(r, red[w]);
+    stat[0] = err;
+    stat[1] = r;
+    stat[2] = it;
+  }
+}
+
+// *out = max |Y2 - S / c| (c = *cmax as stored by k_row_abs_max; *out zeroed before)
+__global__ void k_ns_miss(const double *__restrict__ Y2, const double *__restrict__ S, int64_t n,
+                          const unsigned long long *__restrict__ cmax,
+                          unsigned long long *__restrict__ out) {
+  const double inv = 1.0 / __longlong_as_double((long long)*cmax);
+  double e = 0.0;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const double d = Y2[t] - S[t] * inv;
+    e = fmax(e, d == d ? fabs(d) : 1e300);
+  }
+  for (int o = 16; o > 0; o >>= 1) e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(e));
 }
 
 // A = S / c (c = *cmax as stored by k_row_abs_max), Z = I
