@@ -208,6 +208,14 @@ __device__ __forceinline__ int warp_sums(double (&x)[NQ], int lane) {
   return q0;
 }
 
+// x, or 0 below 2^-485 (1e-146): the squares of what is left are exact to more than 53
+// bits.  (A column of entries about 1e-159 had squares of a few bits, and its
+// reflector was not orthogonal.)  A test of the column's norm instead, with a reflector
+// formed from scaled entries behind it, made the reduction 4 % slower.
+__device__ __forceinline__ double symeig_keep(double x) {
+  return (__double2hiint(x) & 0x7fffffff) < (1023 - 485) << 20 ? 0.0 : x;
+}
+
 template <class Shape>
 __device__ __forceinline__ void
 symeig_tridiag_body(const double *__restrict__ A, int lda, int n, double *__restrict__ work) {
@@ -229,7 +237,7 @@ symeig_tridiag_body(const double *__restrict__ A, int lda, int n, double *__rest
       a[q][t] = i < n && j < n ? A[max(i, j) + (size_t)lda * min(i, j)] : 0.0;
     }
   for (int i = tid; i < LD; i += kTridiagThreads) {
-    s_cur[0][i] = i < n ? A[i] : 0.0;   // column 0
+    s_cur[0][i] = i < n ? symeig_keep(A[i]) : 0.0;   // column 0
     s_cur[1][i] = 0.0;
     s_p[0][i] = s_p[1][i] = 0.0;
     s_col[0][i] = s_col[1][i] = 0.0;
@@ -254,25 +262,8 @@ symeig_tridiag_body(const double *__restrict__ A, int lda, int n, double *__rest
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
       double tc = 0.0, beta = alpha, scal = 0.0;
-      const double h2 = fma(alpha, alpha, xn2);
-      if (h2 < 1e-280) {
-        // a column below 1e-140, whose squares are lost in part or altogether (the
-        // reflector would not be orthogonal): formed from the column times 2^600;
-        // entries below 1e-300 count as zero
-        double x2 = 0.0;
-#pragma unroll
-        for (int t = 0; t < NT; ++t) x2 = fma(v[t] * 0x1p600, v[t] * 0x1p600, x2);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x2 += __shfl_xor_sync(0xffffffffu, x2, o);
-        const double as = alpha * 0x1p600;
-        if (x2 > 1e-239) {
-          const double bs = -copysign(sqrt(fma(as, as, x2)), as);
-          beta = bs * 0x1p-600;
-          tc = (bs - as) / bs;
-          scal = 0x1p600 / (as - bs);
-        }
-      } else if (xn2 != 0.0) {
-        beta = -copysign(sqrt(h2), alpha);
+      if (xn2 != 0.0) {
+        beta = -copysign(sqrt(fma(alpha, alpha, xn2)), alpha);
         tc = (beta - alpha) / beta;
         scal = 1.0 / (alpha - beta);
       }
@@ -349,7 +340,7 @@ symeig_tridiag_body(const double *__restrict__ A, int lda, int n, double *__rest
         const int i = tid + kTridiagThreads * k;
         if (i >= r0 && i < n) {
           const double vi = i == r0 ? 1.0 : cur[i] * scal;
-          s_cur[buf ^ 1][i] = rci[k] - fma(vi, p[r0] - K, p[i] - K * vi);
+          s_cur[buf ^ 1][i] = symeig_keep(rci[k] - fma(vi, p[r0] - K, p[i] - K * vi));
         }
       }
 #pragma unroll
