@@ -1156,12 +1156,12 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
   S2G_LAUNCH(k_gather_cols, grid_for((int64_t)nao * moci), 256, 0, s, Cact, c.d_C.get(),
              (int64_t)nao, c.w_act_idx.get(), (int64_t)moci, (int64_t)nao);
 
-  // ---- S^1/2 (makel stda.f:1615-1691), once per load ----
+  // ---- S^1/2 (makel stda.f:1615-1691), once per load and form ----
   record(c, PH_SQRTS);
-  // (a wavefunction that has been solved otherwise forms it anew, in the plain
-  // form, for iterative sTD-DFT roots)
+  // (anew where the wavefunction was last solved with the other form, so that a
+  // result does not depend on what was solved before)
   const int sq_kind = c.dg.wave_splits ? 1 : 2;
-  if (c.sqrtS_kind < 1 || (sq_kind == 1 && c.sqrtS_kind == 2)) {
+  if (c.sqrtS_kind != sq_kind) {
     double *sq = c.d_sqrtS.ensure((size_t)nao * nao);
     c.sqrtS_kind = 0;
     if (sq_kind == 1) sqrt_overlap_fixed(c, c.d_Sfull.get(), nao, sq);
