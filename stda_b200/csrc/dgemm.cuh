@@ -691,6 +691,8 @@ struct Dgemm {
            double *C, int64_t ldc, int64_t sC, int batch = 1, int tri = 0,
            DgSplitCols sc = DgSplitCols{}) {
     if (sc.len > 0 && tri != 0) throw Error{STD2G_EINVAL, "dgemm: split columns"};
+    // (its split sums in a second launch would take in tiles that are not formed)
+    if (tri < 0 && wave_splits) throw Error{STD2G_EINVAL, "dgemm: symmetric result"};
     if (m <= 0 || n <= 0 || batch <= 0) return;
     if (k < 0) throw Error{STD2G_EINVAL, "dgemm: negative k"};
     flop += 2.0 * m * n * (double)k * batch;
