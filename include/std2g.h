@@ -262,6 +262,11 @@ int std2g_kernel_stats(void *ctx, double *ms, int64_t *launches, double *flop);
    counts the products of the overlap's square root (formed once per load). */
 int std2g_set_gemm_timing(void *ctx, int on);
 int std2g_gemm_stats(void *ctx, double *ms, int64_t *calls, double *flop);
+/* What those numbers rest on: the event pairs recorded (with timing on, one per
+   counted product, a grouped launch counting as one; the square root of an
+   overlap of up to 96 AOs is one pair for all its products), and the launches of
+   the engine's own product kernels. */
+int std2g_gemm_launches(void *ctx, int64_t *timed, int64_t *own);
 
 /* Statistics of the last solve: Davidson iterations, sigma vectors formed
    with tensor-core (mixed) products and with FP64 products, and the number of

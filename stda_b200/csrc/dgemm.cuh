@@ -501,7 +501,22 @@ struct Dgemm {
     nev = 0;
     flop = 0;
     calls = 0;
+    launches = 0;
   }
+  // event pair around one product or grouped launch, where they are timed
+  struct Timed {
+    Dgemm &g;
+    cudaStream_t s;
+    Timed(Dgemm &dg, cudaStream_t stream) : g(dg), s(stream) {
+      if (g.timed) g.mark(s);
+    }
+    ~Timed() {
+      try {
+        if (g.timed) g.mark(s);
+      } catch (const Error &) {   // the launch's own error is the one to report
+      }
+    }
+  };
   // device time of the timed products since reset(); the stream must have
   // passed them (the caller synchronises first)
   double elapsed_ms() const {
@@ -559,6 +574,7 @@ struct Dgemm {
     }
     if (pr.empty()) return;
     ++calls;
+    Timed around(*this, s);
     const int np = (int)pr.size();
     double *wk = wtot > 0 ? gwork.ensure((size_t)wtot) : nullptr;
     DgProblem *d = gdesc.ensure(pr.size());
@@ -697,14 +713,7 @@ struct Dgemm {
     if (k < 0) throw Error{STD2G_EINVAL, "dgemm: negative k"};
     flop += 2.0 * m * n * (double)k * batch;
     ++calls;
-    if (timed) mark(s);
-    struct EndMark {
-      Dgemm &g;
-      cudaStream_t s;
-      ~EndMark() {
-        if (g.timed) g.mark(s);
-      }
-    } end_mark{*this, s};
+    Timed around(*this, s);
     if (lib && tri == 0 && sc.len == 0) {
       const cublasOperation_t oa = ta ? CUBLAS_OP_T : CUBLAS_OP_N, ob = tb ? CUBLAS_OP_T : CUBLAS_OP_N;
       S2G_CUBLAS(cublasSetStream(lib, s));

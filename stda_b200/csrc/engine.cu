@@ -362,9 +362,11 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
     double *stat = c.w_ns.ensure(3), h[3];
     S2G_CUDA(cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns_small_smem(kNsSmallMax)));
-    if (c.dg.timed) c.dg.mark(s);
-    S2G_LAUNCH(k_ns_small, 1, kNsThreads, ns_small_smem(n), s, S, n, out, stat);
-    if (c.dg.timed) c.dg.mark(s);
+    {
+      Dgemm::Timed around(c.dg, s);
+      S2G_LAUNCH(k_ns_small, 1, kNsThreads, ns_small_smem(n), s, S, n, out, stat);
+      ++c.dg.launches;
+    }
     S2G_CUDA(cudaMemcpyAsync(h, stat, sizeof(h), cudaMemcpyDeviceToHost, s));
     S2G_CUDA(cudaStreamSynchronize(s));
     c.ns_iters = (int)h[2];
@@ -2371,6 +2373,14 @@ int std2g_gemm_stats(void *ctx, double *ms, int64_t *calls, double *flop) {
     if (calls) *calls = c->dg.calls + c->mftc.side.dg.calls;
     if (flop) *flop = c->dg.flop + c->mftc.side.dg.flop;
   });
+}
+
+int std2g_gemm_launches(void *ctx, int64_t *timed, int64_t *own) {
+  if (!ctx) return STD2G_EINVAL;
+  auto *c = (Ctx *)ctx;
+  if (timed) *timed = (int64_t)(c->dg.nev / 2 + c->mftc.side.dg.nev / 2);
+  if (own) *own = c->dg.launches + c->mftc.side.dg.launches;
+  return STD2G_OK;
 }
 
 int std2g_solver_stats(void *ctx, int *iters, int64_t *matvecs, int64_t *matvecs_fp64,
