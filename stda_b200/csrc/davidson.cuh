@@ -559,12 +559,18 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
     }
     clk.tick(2);
     // Ritz vectors X = V Y_k, residuals R = W Y_k - X theta: the two products in
-    // one launch (members V, W at a fixed distance)
+    // one launch (members V, W at a fixed distance, which may be negative and leads from
+    // one allocation to another: two calls where they go to cuBLAS)
     const auto apart = [](const double *a, const double *b) {
       return (int64_t)((intptr_t)b - (intptr_t)a) / (int64_t)sizeof(double);
     };
-    dw.dg->run(s, false, false, n, k, m, 1.0, V, n, apart(V, W), Hs, m, 0, 0.0, X, n, apart(X, R),
-               2);
+    if (dw.dg->lib) {
+      dw.dg->run(s, false, false, n, k, m, 1.0, V, n, 0, Hs, m, 0, 0.0, X, n, 0);
+      dw.dg->run(s, false, false, n, k, m, 1.0, W, n, 0, Hs, m, 0, 0.0, R, n, 0);
+    } else {
+      dw.dg->run(s, false, false, n, k, m, 1.0, V, n, apart(V, W), Hs, m, 0, 0.0, X, n, apart(X, R),
+                 2);
+    }
     S2G_LAUNCH(k_dav_resid, dim3(kColSplit, (unsigned)k), 256, 0, s, R, X, theta, n, rpart);
     const size_t rbytes = sizeof(double) * ((size_t)k * kColSplit + 1);
     const double *h_part = (const double *)dw.pin.take(rbytes);
