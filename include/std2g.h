@@ -61,8 +61,10 @@ enum {
    size (by default they are used from ~2.5e8 PT couplings and 16384 CSFs, below
    which the solve is latency-bound and the FP64 GEMMs serve it). */
 #define STD2G_FLAG_TENSOR_ALWAYS 1
-/* FP64 matrix products through cuBLAS instead of the engine's own DMMA kernel
-   (the library baseline that the plain FP64 form is compared with). */
+/* FP64 matrix products through cuBLAS instead of the engine's own DMMA kernels
+   (the library baseline that the plain FP64 form is compared with): every product
+   of a context.  A batch of eigensolves shared by contexts (std2g_batch_create)
+   keeps the engine's. */
 #define STD2G_FLAG_LIBRARY_FP64 2
 /* Request server only (std2g_server_opts.flags): the slots' contexts share one
    batched eigensolver (std2g_batch_create / std2g_attach_batch). */

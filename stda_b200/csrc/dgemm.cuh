@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 #include <cublas_v2.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -699,9 +700,40 @@ struct Dgemm {
         ldc, 0, 1);
   }
 
+  // run() on cuBLAS: the whole product where `tri` asks for a part of it (the rest
+  // is what the caller would mirror), and with two-level columns one call per group,
+  // the members of the batch side by side.  With op(B) = B^T a group of C lies
+  // transposed: C^T = op(B)^T op(A)^T there.
+  void library(cudaStream_t s, bool ta, bool tb, int m, int n, int k, double alpha,
+               const double *A, int64_t lda, int64_t sA, const double *B, int64_t ldb, int64_t sB,
+               double beta, double *C, int64_t ldc, int64_t sC, int batch, DgSplitCols sc) {
+    S2G_CUBLAS(cublasSetStream(lib, s));
+    auto call = [&](bool tx, bool ty, int mm, int nn, const double *X, int64_t ldx, int64_t sX,
+                    const double *Y, int64_t ldy, int64_t sY, double *Z) {
+      const cublasOperation_t ox = tx ? CUBLAS_OP_T : CUBLAS_OP_N, oy = ty ? CUBLAS_OP_T : CUBLAS_OP_N;
+      if (batch == 1)
+        S2G_CUBLAS(cublasDgemm(lib, ox, oy, mm, nn, k, &alpha, X, (int)ldx, Y, (int)ldy, &beta, Z,
+                               (int)ldc));
+      else
+        S2G_CUBLAS(cublasDgemmStridedBatched(lib, ox, oy, mm, nn, k, &alpha, X, (int)ldx, sX, Y,
+                                             (int)ldy, sY, &beta, Z, (int)ldc, sC, batch));
+    };
+    if (sc.len <= 0) {
+      call(ta, tb, m, n, A, lda, sA, B, ldb, sB, C);
+      return;
+    }
+    for (int n0 = 0, g = 0; n0 < n; n0 += sc.len, ++g) {
+      const int len = std::min(sc.len, n - n0);
+      const double *Bg = B + g * sc.sB;
+      double *Cg = C + g * sc.sC;
+      if (tb) call(false, !ta, len, m, Bg, ldb, sB, A, lda, sA, Cg);
+      else call(ta, false, m, len, A, lda, sA, Bg, ldb, sB, Cg);
+    }
+  }
+
   // op(A) is m x k, op(B) is k x n; strides between batch members (0 for one).
   // tri > 0: see k_dgemm; tri < 0: a symmetric n x n result (not with wave_splits).
-  // sc: two-level columns (on this kernel also where `lib` is set).
+  // sc: two-level columns.
   void run(cudaStream_t s, bool ta, bool tb, int m, int n, int k, double alpha, const double *A,
            int64_t lda, int64_t sA, const double *B, int64_t ldb, int64_t sB, double beta,
            double *C, int64_t ldc, int64_t sC, int batch = 1, int tri = 0,
@@ -714,15 +746,8 @@ struct Dgemm {
     flop += 2.0 * m * n * (double)k * batch;
     ++calls;
     Timed around(*this, s);
-    if (lib && tri == 0 && sc.len == 0) {
-      const cublasOperation_t oa = ta ? CUBLAS_OP_T : CUBLAS_OP_N, ob = tb ? CUBLAS_OP_T : CUBLAS_OP_N;
-      S2G_CUBLAS(cublasSetStream(lib, s));
-      if (batch == 1)
-        S2G_CUBLAS(cublasDgemm(lib, oa, ob, m, n, k, &alpha, A, (int)lda, B, (int)ldb, &beta, C,
-                               (int)ldc));
-      else
-        S2G_CUBLAS(cublasDgemmStridedBatched(lib, oa, ob, m, n, k, &alpha, A, (int)lda, sA, B,
-                                             (int)ldb, sB, &beta, C, (int)ldc, sC, batch));
+    if (lib) {
+      library(s, ta, tb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, sc);
       return;
     }
     int bn = 64, ksplit = 1, cs = 1;

@@ -358,7 +358,7 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
       throw Error{STD2G_ES_NOT_PD, "S^1/2: overlap matrix not positive definite (Newton-Schulz "
                                    "did not converge)"};
   };
-  if (n <= kNsSmallMax) {
+  if (n <= kNsSmallMax && !c.dg.lib) {
     double *stat = c.w_ns.ensure(3), h[3];
     S2G_CUDA(cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns_small_smem(kNsSmallMax)));
@@ -384,9 +384,8 @@ static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
   auto *flags = (unsigned long long *)c.w_ns.ensure(2 + kMax);
   S2G_CUDA(cudaMemsetAsync(flags, 0, (2 + kMax) * sizeof(unsigned long long), s));
   S2G_LAUNCH(k_row_abs_max, (int)div_up(n, 64), 64, 0, s, S, n, flags);
-  const int sym = c.dg.lib ? 0 : -1;
   auto mult = [&](const double *L, const double *R, double *D) {
-    c.dg.run(s, false, false, n, n, n, 1.0, L, n, 0, R, n, 0, 0.0, D, n, 0, 1, sym);
+    c.dg.run(s, false, false, n, n, n, 1.0, L, n, 0, R, n, 0, 0.0, D, n, 0, 1, -1);
   };
   double l = kNsLow;
   S2G_LAUNCH(k_ns_first, grid_for((int64_t)nn), 256, 0, s, P, Z, S, n, ns_scale(l), flags);
@@ -1397,8 +1396,17 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
         // sum is rounded once, as a difference of the two couplings)
         gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, nv, nex, N, ak, Pia + (int64_t)i0 * nv * N, N, Qp, N, 0.0,
              X, nv, ni, (int64_t)nv * N, 0, (int64_t)nv * nex);
-        std::vector<DgProblem> jp(gb.size());
-        for (size_t g = 0; g < gb.size(); ++g) {
+        // (the library form: one strided batch over i per run of neighbouring j)
+        for (int q = 0; c.dg.lib && q < nex;) {
+          int e = q + 1;
+          while (e < nex && gq[e] == gq[q] && jq[e] == jq[e - 1] + 1) ++e;
+          gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, nv, e - q, N, -1.0, Qvv + (int64_t)gb[gq[q]] * nv * N, N,
+               Poo + ((int64_t)i0 * no + jq[q]) * N, N, 1.0, X + (int64_t)q * nv, nv, ni, 0,
+               (int64_t)no * N, (int64_t)nex * nv);
+          q = e;
+        }
+        std::vector<DgProblem> jp(c.dg.lib ? 0 : gb.size());
+        for (size_t g = 0; g < jp.size(); ++g) {
           DgProblem &d = jp[g];
           d.M = nv;
           d.N = nq[g] * ni;

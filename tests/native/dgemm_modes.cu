@@ -1,6 +1,7 @@
 // C entries to the forms of the FP64 product that std2g_dgemm_check does not reach
 // (symmetric results, two-level columns, grouped members with indexed columns), on
-// host arrays of na, nb, nc doubles.  Return an STD2G_* code.
+// host arrays of na, nb, nc doubles.  Return an STD2G_* code.  form: 0 as the engine
+// picks, 1 splits by wave counts, 2 cuBLAS.
 #include <atomic>
 
 #include "../../stda_b200/csrc/dgemm.cuh"
@@ -34,6 +35,13 @@ struct Arrays {
   }
 };
 
+struct Handle {
+  cublasHandle_t b = nullptr;
+  ~Handle() {
+    if (b) cublasDestroy(b);
+  }
+};
+
 template <class F>
 int code_of(F &&f) {
   try {
@@ -45,16 +53,22 @@ int code_of(F &&f) {
 }
 }  // namespace
 
-extern "C" int dg_run(int waves, int ta, int tb, int m, int n, int k, double alpha,
+extern "C" int dg_run(int form, int ta, int tb, int m, int n, int k, double alpha,
                       const double *A, int64_t na, int64_t lda, int64_t sA, const double *B,
                       int64_t nb, int64_t ldb, int64_t sB, double beta, double *C, int64_t nc,
                       int64_t ldc, int64_t sC, int batch, int tri, int len, int64_t colB,
                       int64_t colC) {
   return code_of([&] {
     Arrays x(A, na, B, nb, C, nc);
-    x.g.wave_splits = waves != 0;
+    x.g.wave_splits = form == 1;
+    Handle h;
+    if (form == 2) {
+      S2G_CUBLAS(cublasCreate(&h.b));
+      x.g.lib = h.b;
+    }
     x.g.run(x.s, ta != 0, tb != 0, m, n, k, alpha, x.A.get(), lda, sA, x.B.get(), ldb, sB, beta,
             x.C.get(), ldc, sC, batch, tri, DgSplitCols{len, colB, colC});
+    if (form == 2 && x.g.launches != 0) throw Error{STD2G_ESTATE, "own kernel"};
     x.get(C, nc);
   });
 }

@@ -1,6 +1,6 @@
-"""The FP64 product's symmetric results, two-level columns (both orders of op(B)) and
-grouped members with indexed columns, at the edges of their tiles, against numpy on
-the same addresses: |err| <= 4 eps (k + 8) |A| |B| summed, and everything that is not
+"""The FP64 product's symmetric results, two-level columns (both orders of op(B), the
+engine's kernel and cuBLAS) and grouped members with indexed columns, at the edges of
+their tiles, against numpy on the same addresses: |err| <= 4 eps (k + 8) |A| |B| summed, and everything that is not
 addressed is left as it was."""
 import ctypes as ct
 import os
@@ -28,10 +28,10 @@ def _d(a):
 
 
 def _run(lib, ta, tb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch=1, tri=0, len_=0,
-         colB=0, colC=0, waves=0):
+         colB=0, colC=0, form=0):
     out = C.copy()
     L, D = ct.c_int64, ct.c_double
-    code = lib.dg_run(waves, ta, tb, m, n, k, D(alpha), _d(A), L(A.size), L(lda), L(sA), _d(B), L(B.size),
+    code = lib.dg_run(form, ta, tb, m, n, k, D(alpha), _d(A), L(A.size), L(lda), L(sA), _d(B), L(B.size),
                       L(ldb), L(sB), D(beta), _d(out), L(C.size), L(ldc), L(sC), batch, tri, len_, L(colB),
                       L(colC))
     return code, out
@@ -41,9 +41,10 @@ def _close(got, ref, mag, k):
     return np.all(np.abs(got - ref) <= 4 * 2.2e-16 * (k + 8) * mag)
 
 
+@pytest.mark.parametrize("form", [0, 2])
 @pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0)])
 @pytest.mark.parametrize("n,k", [(1, 3), (31, 40), (64, 16), (65, 300), (220, 220), (518, 97)])
-def test_symmetric_result(lib, ta, tb, n, k):
+def test_symmetric_result(lib, form, ta, tb, n, k):
     rng = np.random.default_rng(n)
     G = rng.standard_normal((n, k))
     W = rng.standard_normal(k)
@@ -51,10 +52,11 @@ def test_symmetric_result(lib, ta, tb, n, k):
     A = np.ascontiguousarray(a if ta else a.T).ravel()    # column-major op(A)
     B = np.ascontiguousarray(b.T).ravel()
     code, out = _run(lib, ta, tb, n, n, k, 1.5, A, k if ta else n, 0, B, k, 0, 0.0,
-                     np.full(n * n, np.nan), n, 0, tri=-1)
+                     np.full(n * n, np.nan), n, 0, tri=-1, form=form)
     assert code == 0
     out = out.reshape(n, n)
-    assert np.array_equal(out, out.T)
+    if form == 0:
+        assert np.array_equal(out, out.T)
     assert _close(out, 1.5 * a @ b, 1.5 * np.abs(a) @ np.abs(b), k)
 
 
@@ -62,16 +64,16 @@ def test_symmetric_result_refused_with_wave_splits(lib):
     """Split sums in a second launch would add tiles that were never formed."""
     n = 300
     A = np.eye(n).ravel()
-    code, _ = _run(lib, 0, 0, n, n, n, 1.0, A, n, 0, A, n, 0, 0.0, A, n, 0, tri=-1, waves=1)
+    code, _ = _run(lib, 0, 0, n, n, n, 1.0, A, n, 0, A, n, 0, 0.0, A, n, 0, tri=-1, form=1)
     assert code == 1
 
 
 @pytest.mark.parametrize("tb", [0, 1])
-@pytest.mark.parametrize("waves", [0, 1])
+@pytest.mark.parametrize("form", [0, 1, 2])
 @pytest.mark.parametrize("m,k,len_,groups,batch", [(5, 3, 1, 1, 2), (64, 16, 4, 15, 3), (65, 130, 9, 8, 4),
                                                    (129, 700, 5, 26, 2), (90, 90, 9, 60, 7)])
 @pytest.mark.parametrize("beta", [0.0, 0.5])
-def test_two_level_columns(lib, tb, waves, m, k, len_, groups, batch, beta):
+def test_two_level_columns(lib, tb, form, m, k, len_, groups, batch, beta):
     rng = np.random.default_rng(m + k)
     lda, n = m + 3, len_ * groups
     sA = lda * k
@@ -88,7 +90,7 @@ def test_two_level_columns(lib, tb, waves, m, k, len_, groups, batch, beta):
     B = rng.standard_normal(colB * groups)
     C = rng.standard_normal(colC * groups)
     code, out = _run(lib, 0, tb, m, n, k, -1.5, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, 0, len_,
-                     colB, colC, waves)
+                     colB, colC, form)
     assert code == 0
     ref, mag = C.copy(), np.zeros_like(C)
     i, kk = np.arange(m), np.arange(k)
