@@ -417,6 +417,11 @@ int std2g_dgemm_check(int device, int ta, int tb, int m, int n, int k, double al
 int std2g_symeig_check(int device, int n, int k, const double *A, double *w, double *Z,
                        double *w_ref);
 
+/* Diagnostic: leaves a context as a call does that ended with another error after
+   one of its tensor-core waits had run out (the status word is set; nothing waits
+   on the device).  The calls that follow must not report it. */
+int std2g_leave_expired_wait(void *ctx);
+
 const char *std2g_error_string(int status);
 void std2g_destroy(void *ctx);
 

@@ -2069,6 +2069,24 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
   }
 }
 
+// solve() with the statuses of the tensor-core waits: what an earlier call left is
+// dropped, and where this one ends with another error after a wait ran out, the wait is
+// reported as the cause.
+static void run_solve(Ctx &c, const std2g_params &p, std2g_result *res, const RespReq *resp,
+                      const QuadReq *tpa = nullptr) {
+  c.mixed.tc.forget(c.stream);
+  c.mftc.tc.forget(c.stream);
+  try {
+    solve(c, p, res, resp, tpa);
+  } catch (const Error &e) {
+    if (e.code != STD2G_ETIMEOUT && e.code != STD2G_ECUDA) {
+      c.mixed.tc.check(c.stream);
+      c.mftc.tc.check(c.stream);
+    }
+    throw;
+  }
+}
+
 }  // namespace std2g
 
 // ============================ C boundary =================================
@@ -2205,7 +2223,7 @@ int std2g_solve(void *ctx, const std2g_params *par, std2g_result *res) {
   return guard([&] {
     S2G_CUDA(cudaSetDevice(c->opts.device));
     if (par->e_thr_ev <= 0) throw Error{STD2G_EINVAL, "e_thr_ev must be positive"};
-    std2g::solve(*c, *par, res, nullptr);
+    std2g::run_solve(*c, *par, res, nullptr);
   });
 }
 
@@ -2216,7 +2234,7 @@ int std2g_polarizability(void *ctx, const std2g_params *par, const double *omega
   return guard([&] {
     S2G_CUDA(cudaSetDevice(c->opts.device));
     std2g::RespReq rq{omega, nomega, alpha, resid};
-    std2g::solve(*c, *par, nullptr, &rq);
+    std2g::run_solve(*c, *par, nullptr, &rq);
   });
 }
 
@@ -2240,7 +2258,7 @@ int std2g_hyperpolarizability(void *ctx, const std2g_params *par, const double *
       q.nbeta = nk;
       std2g::RespReq rq{om.data(), 2 * nk, al.data(), rs.data()};
       rq.quad = &q;
-      std2g::solve(*c, *par, nullptr, &rq);
+      std2g::run_solve(*c, *par, nullptr, &rq);
     }
   });
 }
@@ -2258,7 +2276,7 @@ int std2g_two_photon(void *ctx, const std2g_params *par, int ntrans, double *row
     std2g::QuadReq q;
     q.tpa = rows;
     q.ntpa = ntrans;
-    std2g::solve(*c, p, nullptr, nullptr, &q);
+    std2g::run_solve(*c, p, nullptr, nullptr, &q);
   });
 }
 
@@ -2389,6 +2407,16 @@ int std2g_gemm_launches(void *ctx, int64_t *timed, int64_t *own) {
   if (timed) *timed = (int64_t)(c->dg.nev / 2 + c->mftc.side.dg.nev / 2);
   if (own) *own = c->dg.launches + c->mftc.side.dg.launches;
   return STD2G_OK;
+}
+
+int std2g_leave_expired_wait(void *ctx) {
+  if (!ctx) return STD2G_EINVAL;
+  auto *c = (Ctx *)ctx;
+  return guard([&] {
+    S2G_CUDA(cudaSetDevice(c->opts.device));
+    c->mixed.tc.leave_expired(c->stream);
+    c->mftc.tc.leave_expired(c->stream);
+  });
 }
 
 int std2g_solver_stats(void *ctx, int *iters, int64_t *matvecs, int64_t *matvecs_fp64,

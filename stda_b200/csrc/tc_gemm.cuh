@@ -645,7 +645,8 @@ struct TcGemm {
     throw Error{STD2G_ETIMEOUT, "tc_gemm: bounded wait expired (" + std::to_string(code) + ")"};
   }
   // between products of an iteration: reports an expired wait of an earlier one as soon
-  // as the host can see it; the caller ends with check()
+  // as the host can see it; the caller ends with check(), also where it ends with
+  // another error (an iteration on a product that was not finished may fail first)
   void poll(cudaStream_t s) {
     if (!armed) return;
     if (!h_err) {
@@ -654,6 +655,20 @@ struct TcGemm {
     }
     if (*(volatile int *)h_err) check(s);
     S2G_CUDA(cudaMemcpyAsync(h_err, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+  }
+
+  // drop what a call that ended early left behind (synchronises if there is any)
+  void forget(cudaStream_t s) {
+    if (!armed) return;
+    S2G_CUDA(cudaStreamSynchronize(s));
+    armed = false;
+    if (h_err) *h_err = 0;
+  }
+
+  // the state of a call that ended early after a wait of its products had run out
+  void leave_expired(cudaStream_t s) {
+    S2G_CUDA(cudaMemsetAsync(err.ensure(1), 1, sizeof(int), s));
+    armed = true;
   }
 
   // read the error flag of the launches since the last check (synchronises)

@@ -35,7 +35,8 @@ EXPORTS = [
     "std2g_symeig_check", "std2g_set_sm_limit", "std2g_hyperpolarizability", "std2g_two_photon",
     "std2g_ao_integrals", "std2g_load_prims", "std2g_dgemm_check", "std2g_set_spins",
     "std2g_set_gemm_timing", "std2g_gemm_stats", "std2g_gemm_launches", "std2g_batch_create",
-    "std2g_attach_batch", "std2g_batch_stats", "std2g_batch_destroy", "std2g_last_batched", "std2g_server_batch_stats",
+    "std2g_attach_batch", "std2g_batch_stats", "std2g_batch_destroy", "std2g_last_batched",
+    "std2g_server_batch_stats", "std2g_leave_expired_wait",
 ]
 
 
@@ -159,6 +160,7 @@ def library():
         lib.std2g_kernel_stats.argtypes = [C.c_void_p, dp, C.POINTER(C.c_int64), dp]
         lib.std2g_set_gemm_timing.argtypes = [C.c_void_p, C.c_int]
         lib.std2g_gemm_stats.argtypes = [C.c_void_p, dp, C.POINTER(C.c_int64), dp]
+        lib.std2g_leave_expired_wait.argtypes = [C.c_void_p]
         lib.std2g_gemm_launches.argtypes = [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
         lib.std2g_solver_stats.argtypes = [C.c_void_p, ip, C.POINTER(C.c_int64),
                                             C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
