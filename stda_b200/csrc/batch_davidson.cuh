@@ -210,7 +210,6 @@ __global__ void k_bd_unit(double *__restrict__ V, int n, const int *__restrict__
 struct BatchProblem {
   // inputs
   DavidsonWork *dw = nullptr;
-  cublasHandle_t blas = nullptr;
   cusolverDnHandle_t sol = nullptr;
   const double *A = nullptr, *diag = nullptr;   // dense A (n x n), diag(A)
   int n = 0, kwant = 0, max_iter = 300;
@@ -743,7 +742,7 @@ inline void BatchDavidson::iterate(std::vector<BatchProblem *> &act) {
         S2G_LAUNCH(k_colnorm_part, dim3(kColSplit, (unsigned)p->ncur), 256, 0, cs_, p->Tb, p->n,
                    dw.part.ensure((size_t)p->k * kColSplit));
         dw.pin.reset();
-        p->ncur = dav_orthonormalize(dw, p->blas, p->sol, cs_, dw.V.get(), p->n, p->m, p->Tb,
+        p->ncur = dav_orthonormalize(dw, p->sol, cs_, dw.V.get(), p->n, p->m, p->Tb,
                                      p->ncur, p->k, p->mmax - p->m);
         p->ortho_open = false;
       }

@@ -364,8 +364,7 @@ inline std::vector<int> lowest_indices(int n, int k, const Less &less) {
 // status (a failed factor only spoils buffers that the fallback writes anew): one
 // wait per block instead of two, each of which left the GPU idle for ~10 us.
 // fixed_order: the small factorisations by the kernels of symeig_seq.cuh.
-inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t sol,
-                              cudaStream_t s, double *V, int n, int m, double *T, int nc,
+inline int dav_orthonormalize(DavidsonWork &dw, cusolverDnHandle_t sol, cudaStream_t s, double *V, int n, int m, double *T, int nc,
                               int kcap, int room, bool fixed_order = false) {
   const int k = kcap;
   const int grid = 148 * 4;
@@ -479,8 +478,7 @@ inline int dav_orthonormalize(DavidsonWork &dw, cublasHandle_t blas, cusolverDnH
 // W = A V for nb column vectors (n x nb, column-major); `diag` is diag(A).
 // With `warm`, the first block is the k Ritz vectors left in dw.X by a
 // previous call on the same problem (orthonormal), instead of unit vectors.
-inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t sol,
-                    cudaStream_t s, const MatVec &mv, const double *diag, int n, int k,
+inline int davidson(DavidsonWork &dw, cusolverDnHandle_t sol, cudaStream_t s, const MatVec &mv, const double *diag, int n, int k,
                     double tol, int max_iter, double *omega_out, double *X_out,
                     bool warm = false, bool buffer_roots = true) {
   if (k > n) k = n;
@@ -613,7 +611,7 @@ inline int davidson(DavidsonWork &dw, cublasHandle_t blas, cusolverDnHandle_t so
       S2G_LAUNCH(k_diag_matrix, (int)div_up((int64_t)k * k, 256), 256, 0, s, H, mmax, k, theta);
     }
     // block orthogonalisation of the corrections, appended to V after column m
-    nb = dav_orthonormalize(dw, blas, sol, s, V, n, m, T, nc, k, mmax - m);
+    nb = dav_orthonormalize(dw, sol, s, V, n, m, T, nc, k, mmax - m);
     clk.tick(4);
     if (nb == 0) break;
   }

@@ -104,7 +104,7 @@ __global__ void k_rpa_precond(double *__restrict__ T, const double *__restrict__
 }
 
 struct DavidsonRpaWork {
-  DBuf<double> Q, Am, Amc, Ap2, S, T1, Mr, lam, ev, Z, Xp, Xm, Rp, Rm, C, Qc, tmpn, rn, part, om,
+  DBuf<double> Q, Am, Amc, Ap2, S, T1, Mr, lam, ev, Z, Xp, Xm, Rp, Rm, C, Qc, tmpn, part, om,
       wf, XpY, XmY;
   DBuf<int> cols;
   int iters = 0;
@@ -142,8 +142,8 @@ inline void rpa_small_eig(DavidsonWork &dw, DavidsonRpaWork &rw, cusolverDnHandl
 // Returns the number of converged wanted roots (== k on success).  mv_p /
 // mv_m form (A+B) V and (A-B) V for nb columns; dp, dm are diag(A+B),
 // diag(A-B).  On return omega_out [k], XpY_out, XmY_out (n x k).
-inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t blas,
-                        cusolverDnHandle_t sol, cudaStream_t s, const MatVec &mv_p,
+inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cusolverDnHandle_t sol,
+                        cudaStream_t s, const MatVec &mv_p,
                         const MatVec &mv_m, const double *dp, const double *dm, int n, int k,
                         double tol, int max_iter, double *omega_out, double *XpY_out,
                         double *XmY_out) {
@@ -301,7 +301,7 @@ inline int davidson_rpa(DavidsonWork &dw, DavidsonRpaWork &rw, cublasHandle_t bl
       }
       m = nkeep;
     }
-    nb = dav_orthonormalize(dw, blas, sol, s, B, n, m, T, 2 * nc, 2 * k, mmax - m, true);
+    nb = dav_orthonormalize(dw, sol, s, B, n, m, T, 2 * nc, 2 * k, mmax - m, true);
     if (nb == 0) break;
   }
   S2G_CUDA(cudaMemcpyAsync(omega_out, om, sizeof(double) * kwant, cudaMemcpyDeviceToDevice, s));

@@ -394,6 +394,32 @@ k_dgemm_reduce(int M, int N, int batch, int ksplit, double alpha, const double *
   }
 }
 
+// For products on cuBLAS: P[k + K (n + N q)] = element (k, n) of member q's op(B) with
+// two-level columns, or with column n at cols[n], and back: C = P + beta C on its columns
+__global__ void k_dgemm_pack(double *__restrict__ P, const double *__restrict__ B, int64_t ldb,
+                             int64_t sB, int N, int K, int batch, bool tb, DgSplitCols sc,
+                             const int *__restrict__ cols) {
+  const int64_t total = (int64_t)K * N * batch;
+  for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total;
+       x += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = x / K, q = c / N;
+    const int k = (int)(x - c * K), at = (int)(c - q * N), n = cols ? cols[at] : at;
+    P[x] = B[q * sB + (tb ? sc.b<true>(n, ldb) + k * ldb : sc.b<false>(n, ldb) + k)];
+  }
+}
+__global__ void k_dgemm_spread(double *__restrict__ C, int64_t ldc, int64_t sC,
+                               const double *__restrict__ P, int M, int N, int batch, bool tb,
+                               DgSplitCols sc, const int *__restrict__ cols, double beta) {
+  const int64_t total = (int64_t)M * N * batch;
+  for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total;
+       x += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = x / M, q = c / N;
+    const int i = (int)(x - c * M), at = (int)(c - q * N), n = cols ? cols[at] : at;
+    double *p = C + q * sC + sc.c(tb, i, n, ldc);
+    *p = beta == 0.0 ? P[x] : P[x] + beta * *p;
+  }
+}
+
 // One member of a grouped launch: C = alpha op(A) op(B) + beta C with op(A)
 // M x K and op(B) K x N (column-major; beta = 0: C is not read).
 struct DgProblem {
@@ -488,6 +514,7 @@ struct Dgemm {
   // set: the products go to cuBLAS on this handle instead (the library
   // baseline of the plain FP64 form, STD2G_FLAG_LIBRARY_FP64)
   cublasHandle_t lib = nullptr;
+  DBuf<double> packed;   // two-level columns and results of those products, contiguous
   // per-product device time (an event pair around each product) and the
   // algorithmic FLOPs 2 m n k of the products since the last reset()
   bool timed = false;
@@ -546,6 +573,7 @@ struct Dgemm {
   DBuf<double> gwork;   // partial tiles of the split members
   void grouped(cudaStream_t s, bool ta, bool tb, const std::vector<DgProblem> &in,
                PinnedArena *stage = nullptr) {
+    if (lib) return library_grouped(s, ta, tb, in);
     std::vector<DgProblem> pr;
     std::vector<int> t0(1, 0);
     int64_t wtot = 0;
@@ -701,33 +729,58 @@ struct Dgemm {
   }
 
   // run() on cuBLAS: the whole product where `tri` asks for a part of it (the rest
-  // is what the caller would mirror), and with two-level columns one call per group,
-  // the members of the batch side by side.  With op(B) = B^T a group of C lies
-  // transposed: C^T = op(B)^T op(A)^T there.
+  // is what the caller would mirror).  Two-level columns are packed into one block per
+  // member before, and the result is spread after it, outside the timed region (one
+  // strided batch per group of 4 columns halved the rate over C384H48's products).
   void library(cudaStream_t s, bool ta, bool tb, int m, int n, int k, double alpha,
                const double *A, int64_t lda, int64_t sA, const double *B, int64_t ldb, int64_t sB,
                double beta, double *C, int64_t ldc, int64_t sC, int batch, DgSplitCols sc) {
     S2G_CUBLAS(cublasSetStream(lib, s));
-    auto call = [&](bool tx, bool ty, int mm, int nn, const double *X, int64_t ldx, int64_t sX,
-                    const double *Y, int64_t ldy, int64_t sY, double *Z) {
-      const cublasOperation_t ox = tx ? CUBLAS_OP_T : CUBLAS_OP_N, oy = ty ? CUBLAS_OP_T : CUBLAS_OP_N;
+    auto product = [&](cublasOperation_t ob, const double *Y, int64_t ldy, int64_t sY, double bt,
+                       double *Z, int64_t ldz, int64_t sZ) {
+      Timed around(*this, s);
+      const cublasOperation_t oa = ta ? CUBLAS_OP_T : CUBLAS_OP_N;
       if (batch == 1)
-        S2G_CUBLAS(cublasDgemm(lib, ox, oy, mm, nn, k, &alpha, X, (int)ldx, Y, (int)ldy, &beta, Z,
-                               (int)ldc));
+        S2G_CUBLAS(cublasDgemm(lib, oa, ob, m, n, k, &alpha, A, (int)lda, Y, (int)ldy, &bt, Z,
+                               (int)ldz));
       else
-        S2G_CUBLAS(cublasDgemmStridedBatched(lib, ox, oy, mm, nn, k, &alpha, X, (int)ldx, sX, Y,
-                                             (int)ldy, sY, &beta, Z, (int)ldc, sC, batch));
+        S2G_CUBLAS(cublasDgemmStridedBatched(lib, oa, ob, m, n, k, &alpha, A, (int)lda, sA, Y,
+                                             (int)ldy, sY, &bt, Z, (int)ldz, sZ, batch));
     };
     if (sc.len <= 0) {
-      call(ta, tb, m, n, A, lda, sA, B, ldb, sB, C);
+      product(tb ? CUBLAS_OP_T : CUBLAS_OP_N, B, ldb, sB, beta, C, ldc, sC);
       return;
     }
-    for (int n0 = 0, g = 0; n0 < n; n0 += sc.len, ++g) {
-      const int len = std::min(sc.len, n - n0);
-      const double *Bg = B + g * sc.sB;
-      double *Cg = C + g * sc.sC;
-      if (tb) call(false, !ta, len, m, Bg, ldb, sB, A, lda, sA, Cg);
-      else call(ta, false, m, len, A, lda, sA, Bg, ldb, sB, Cg);
+    const int64_t kn = (int64_t)k * n, mn = (int64_t)m * n;
+    double *Bp = packed.ensure((size_t)batch * (kn + mn)), *Cp = Bp + batch * kn;
+    const int g = nsm * 16;
+    S2G_LAUNCH(k_dgemm_pack, g, 256, 0, s, Bp, B, ldb, sB, n, k, batch, tb, sc, nullptr);
+    product(CUBLAS_OP_N, Bp, k, kn, 0.0, Cp, m, mn);
+    S2G_LAUNCH(k_dgemm_spread, g, 256, 0, s, C, ldc, sC, Cp, m, n, batch, tb, sc, nullptr, beta);
+  }
+
+  // grouped() on cuBLAS: one call per member, indexed columns packed and spread
+  void library_grouped(cudaStream_t s, bool ta, bool tb, const std::vector<DgProblem> &in) {
+    const int g = nsm * 16;
+    for (const DgProblem &q : in) {
+      if (q.M <= 0 || q.N <= 0) continue;
+      flop += 2.0 * q.M * q.N * (double)q.K;
+      ++calls;
+      const int64_t kn = (int64_t)q.K * q.N, mn = (int64_t)q.M * q.N;
+      double *Bp = q.bcol || q.ccol ? packed.ensure((size_t)(kn + mn)) : nullptr, *Cp = Bp + kn;
+      const double *B = q.B;
+      int64_t ldb = q.ldb;
+      if (q.bcol) {   // op(B) = B
+        S2G_LAUNCH(k_dgemm_pack, g, 256, 0, s, Bp, q.B, q.ldb, (int64_t)0, q.N, q.K, 1, false,
+                   DgSplitCols{}, q.bcol);
+        B = Bp;
+        ldb = q.K;
+      }
+      library(s, ta, tb, q.M, q.N, q.K, q.alpha, q.A, q.lda, 0, B, ldb, 0, q.ccol ? 0.0 : q.beta,
+              q.ccol ? Cp : q.C, q.ccol ? q.M : q.ldc, 0, 1, DgSplitCols{});
+      if (q.ccol)
+        S2G_LAUNCH(k_dgemm_spread, g, 256, 0, s, q.C, q.ldc, (int64_t)0, Cp, q.M, q.N, 1, false,
+                   DgSplitCols{}, q.ccol, q.beta);
     }
   }
 
@@ -745,11 +798,11 @@ struct Dgemm {
     if (k < 0) throw Error{STD2G_EINVAL, "dgemm: negative k"};
     flop += 2.0 * m * n * (double)k * batch;
     ++calls;
-    Timed around(*this, s);
     if (lib) {
       library(s, ta, tb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, sc);
       return;
     }
+    Timed around(*this, s);
     int bn = 64, ksplit = 1, cs = 1;
     pick_split(m, n, k, batch, tri < 0, bn, ksplit, cs);
     const int tiles = (int)(div_up(m, dg::BM) * div_up(n, bn));

@@ -73,9 +73,9 @@ struct Ctx {
   // work buffers
   DBuf<double> w_Cact, w_Clow, w_T, w_mu_ov, w_gj, w_gk, w_Qii, w_Qaa, w_Pii, w_uci;
   DBuf<double> w_Qia, w_Pia, w_Qoo, w_Poo, w_Qvv, w_de, w_ek;
-  DBuf<int> w_flag, w_act_idx, w_pk, w_ck, w_tmpi, w_pj, w_pb, w_omap, w_vmap, w_OP, w_VP, w_ci,
+  DBuf<int> w_flag, w_act_idx, w_pk, w_ck, w_tmpi, w_pj, w_pgroup, w_gstart, w_gsize, w_bcol, w_ccol, w_ci,
       w_ca, w_allk, w_status;
-  DBuf<double> w_ed, w_edsorted, w_Qp, w_W, w_Kbuf, w_pert, w_colpart,
+  DBuf<double> w_ed, w_edsorted, w_Qp, w_rowpart, w_coup, w_pert, w_colpart,
       w_pt2, w_edp;
   DBuf<unsigned char> w_sel;
   DBuf<double> w_Qs, w_Ps, w_K, w_J, w_Kx, w_A, w_Apb, w_Amb, w_Bh, w_Ambh, w_M, w_eval, w_X,
@@ -867,13 +867,13 @@ static void response_matfree(Ctx &c, int n, const double *musel, const RespReq &
   const bool amb_diag = std::fabs(ax) < 1e-6;
   auto products = [&](const double *U, const double *V, double *PU, double *MV, bool tc) {
     if (tc)
-      mftc_apply(c.mftc, c.blas, s, U, ncol, PU, 2.0 * ak, -1.0, -ax, d);
+      mftc_apply(c.mftc, s, U, ncol, PU, 2.0 * ak, -1.0, -ax, d);
     else
       mf_apply(c.mf, s, U, ncol, PU, 2.0 * ak, -1.0, -ax, d);
     if (amb_diag)
       S2G_LAUNCH(k_diag_mul, grid_for((int64_t)n * ncol), 256, 0, s, MV, dmd, V, n, ncol);
     else if (tc)
-      mftc_apply(c.mftc, c.blas, s, V, ncol, MV, 0.0, -1.0, ax, d);
+      mftc_apply(c.mftc, s, V, ncol, MV, 0.0, -1.0, ax, d);
     else
       mf_apply(c.mf, s, V, ncol, MV, 0.0, -1.0, ax, d);
   };
@@ -1350,7 +1350,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
         return d;
       };
       int *d_pk = up(c.w_pk, pko), *d_ck = up(c.w_ck, ck), *d_jq = up(c.w_pj, jq),
-          *d_gq = up(c.w_pb, gq), *d_qs = up(c.w_omap, qs), *d_nq = up(c.w_vmap, nq);
+          *d_gq = up(c.w_pgroup, gq), *d_qs = up(c.w_gstart, qs), *d_nq = up(c.w_gsize, nq);
       double *d_ed = c.w_edsorted.ensure(nex);
       S2G_CUDA(cudaMemcpyAsync(d_ed, edo.data(), sizeof(double) * nex, cudaMemcpyHostToDevice, s));
       double *Qp = c.w_Qp.ensure((size_t)N * nex);   // the primaries' charges
@@ -1388,25 +1388,16 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
         const int i0 = q * occ_chunk, i1 = std::min(no, i0 + occ_chunk), ni = i1 - i0;
         const int r0 = first_of_occ[i0], r1 = first_of_occ[i1], nr = r1 - r0;
         if (nr == 0) continue;
-        double *X = c.w_Kbuf.ensure((size_t)nex * nv * ni);
-        int *bcol = c.w_OP.ensure((size_t)nex * ni), *ccol = c.w_VP.ensure((size_t)nex * ni);
+        double *X = c.w_coup.ensure((size_t)nex * nv * ni);
+        int *bcol = c.w_bcol.ensure((size_t)nex * ni), *ccol = c.w_ccol.ensure((size_t)nex * ni);
         S2G_LAUNCH(k_pt_columns, grid_for((int64_t)nex * ni), 256, 0, s, d_jq, d_gq, d_qs, d_nq, nex,
                    ni, i0, no, bcol, ccol);
         // ak (ia|jb), then -(ij|ab) group by group (ak = 0, 1, 2: exact, so that the
         // sum is rounded once, as a difference of the two couplings)
         gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, nv, nex, N, ak, Pia + (int64_t)i0 * nv * N, N, Qp, N, 0.0,
              X, nv, ni, (int64_t)nv * N, 0, (int64_t)nv * nex);
-        // (the library form: one strided batch over i per run of neighbouring j)
-        for (int q = 0; c.dg.lib && q < nex;) {
-          int e = q + 1;
-          while (e < nex && gq[e] == gq[q] && jq[e] == jq[e - 1] + 1) ++e;
-          gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, nv, e - q, N, -1.0, Qvv + (int64_t)gb[gq[q]] * nv * N, N,
-               Poo + ((int64_t)i0 * no + jq[q]) * N, N, 1.0, X + (int64_t)q * nv, nv, ni, 0,
-               (int64_t)no * N, (int64_t)nex * nv);
-          q = e;
-        }
-        std::vector<DgProblem> jp(c.dg.lib ? 0 : gb.size());
-        for (size_t g = 0; g < jp.size(); ++g) {
+        std::vector<DgProblem> jp(gb.size());
+        for (size_t g = 0; g < gb.size(); ++g) {
           DgProblem &d = jp[g];
           d.M = nv;
           d.N = nq[g] * ni;
@@ -1426,7 +1417,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
         const int nz = (int)std::max<int64_t>(
             1, std::min<int64_t>(div_up(nex, 8), div_up(8 * (int64_t)c.dev_sms, (int64_t)ni * nab)));
         const int qlen = (int)div_up(nex, nz);
-        double *part = c.w_W.ensure((size_t)nz * ni * nv);
+        double *part = c.w_rowpart.ensure((size_t)nz * ni * nv);
         S2G_LAUNCH(k_pt_rows, dim3((unsigned)nab, (unsigned)ni, (unsigned)nz), kPtRowThreads, 0, s, X,
                    nv, nex, qlen, i0, de, d_ed, part);
         S2G_LAUNCH(k_pt_rows_finish, grid_for(nr, 128), 128, 0, s, part, nz, ni, nv, i0, d_ck + r0,
@@ -1654,7 +1645,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
     nroot = std::min(p.nroots, nci);
     X = c.w_X.ensure((size_t)nci * nroot);
     Yv = c.w_Y.ensure((size_t)nci * nroot);
-    const int conv = davidson_rpa(c.dav, c.davr, c.blas, c.solver, s, mv_p, mv_m, dpd, dmd, nci,
+    const int conv = davidson_rpa(c.dav, c.davr, c.solver, s, mv_p, mv_m, dpd, dmd, nci,
                                   p.nroots, tol, 300, om, X, Yv);
     c.dav_iters = c.davr.iters;
     c.dav_matvecs = 0;
@@ -1680,11 +1671,11 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       // stage 1: tensor-core (split-BF16 FP32) products; stage 2: FP64 products
       // from those Ritz vectors until the FP64 residuals meet tol
       MatVec mv_tc = [&](const double *V, int nb, double *W) {
-        mftc_apply(c.mftc, c.blas, s, V, nb, W, ak, -1.0, 0.0, c.mf.dA.get());
+        mftc_apply(c.mftc, s, V, nb, W, ak, -1.0, 0.0, c.mf.dA.get());
       };
       c.dav.profile = c.opts.verbose >= 2;
       for (double &v : c.dav.sec_ms) v = 0;
-      davidson(c.dav, c.blas, c.solver, s, mv_tc, d_edall, nci, p.nroots, tol1, 300, om, Xd);
+      davidson(c.dav, c.solver, s, mv_tc, d_edall, nci, p.nroots, tol1, 300, om, Xd);
       c.mftc.tc.check(s);
       c.dav_iters = c.dav.iters;
       c.dav_matvecs = c.dav.matvecs;
@@ -1702,7 +1693,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       sc.tick(0);
       if (c.dav.profile) std::fprintf(stderr, "FP64 operator setup %.2f ms\n", c.dav.sec_ms[0]);
       for (double &v : c.dav.sec_ms) v = 0;
-      conv = davidson(c.dav, c.blas, c.solver, s, mv, d_edall, nci, p.nroots, tol, 100, om, Xd,
+      conv = davidson(c.dav, c.solver, s, mv, d_edall, nci, p.nroots, tol, 100, om, Xd,
                       true, false);
       c.dav_iters += c.dav.iters;
       c.dav_fp64_matvecs = c.dav.matvecs;   // B X of the velocity correction also in FP64
@@ -1713,7 +1704,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
                      c.dav.iters, c.dav.sec_ms[0], c.dav.sec_ms[1], c.dav.sec_ms[2],
                      c.dav.sec_ms[3], c.dav.sec_ms[4]);
     } else {
-      conv = davidson(c.dav, c.blas, c.solver, s, mv, d_edall, nci, p.nroots, tol, 300, om, Xd);
+      conv = davidson(c.dav, c.solver, s, mv, d_edall, nci, p.nroots, tol, 300, om, Xd);
       c.dav_iters = c.dav.iters;
       c.dav_matvecs = 0;
       c.dav_fp64_matvecs = c.dav.matvecs;
@@ -1741,7 +1732,6 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       // solve gives them, from the shared batch
       BatchProblem bp;
       bp.dw = &c.dav;
-      bp.blas = c.blas;
       bp.sol = c.solver;
       bp.A = A;
       bp.diag = d_edall;
@@ -1966,7 +1956,7 @@ static void solve(Ctx &c, const std2g_params &p_in, std2g_result *res, const Res
       // X_new = (B/2) X / w (apbtrafo.f:51-65)
       double *Xn = c.w_Y.ensure((size_t)nci * nroot);
       if (use_mf && tc_dav) {   // mixed form: tensor-core exchange products
-        mftc_apply(c.mftc, c.blas, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);
+        mftc_apply(c.mftc, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);
         c.mftc.tc.check(s);
       } else if (use_mf)
         mf_apply(c.mf, s, X, nroot, Xn, 0.5 * ak, 0.0, -0.5 * p.ax, nullptr);

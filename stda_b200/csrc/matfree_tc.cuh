@@ -231,7 +231,7 @@ inline void mftc_setup(MatFreeTc &w, cudaStream_t s, const double *Clow, int nao
 
 // out (nci x m, FP64) = cK (K X) + cJ (J X) + cX (K_x X) + diag o X
 // (cX != 0 needs the exchange operands of mftc_setup(..., Pia))
-inline void mftc_apply(MatFreeTc &w, cublasHandle_t h, cudaStream_t s, const double *X, int m,
+inline void mftc_apply(MatFreeTc &w, cudaStream_t s, const double *X, int m,
                        double *out, double cK, double cJ, double cX, const double *diag) {
   const int N = w.N, no = w.no, nv = w.nv, nci = w.nci, rows = w.rows, maxa = w.maxa;
   const int g = 148 * 8;
@@ -252,7 +252,6 @@ inline void mftc_apply(MatFreeTc &w, cublasHandle_t h, cudaStream_t s, const dou
   } else {
     S2G_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * nci * m, s));
   }
-  (void)h;
   if (cJ != 0.0 || cX != 0.0) {
     const int64_t mo = (int64_t)no * m, mz = (int64_t)maxa * m;
     const int ldo = ld4(no), ldv = ld4(nv), Zo = ld8(no), Zv = ld8(nv);

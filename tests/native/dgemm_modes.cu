@@ -75,7 +75,7 @@ extern "C" int dg_run(int form, int ta, int tb, int m, int n, int k, double alph
 
 // members p: C[at C0[p]] = alpha op(A[at A0[p]]) op(B) + beta C, columns named by
 // bcol / ccol from col0[p] on (col0[p] < 0: plain columns)
-extern "C" int dg_grouped(int ta, int tb, int np, const int *M, const int *N, const int *K,
+extern "C" int dg_grouped(int form, int ta, int tb, int np, const int *M, const int *N, const int *K,
                           double alpha, double beta, const double *A, int64_t na,
                           const int64_t *A0, int64_t lda, const double *B, int64_t nb,
                           const int64_t *B0, int64_t ldb, double *C, int64_t nc,
@@ -83,6 +83,11 @@ extern "C" int dg_grouped(int ta, int tb, int np, const int *M, const int *N, co
                           int ncol, const int64_t *col0) {
   return code_of([&] {
     Arrays x(A, na, B, nb, C, nc);
+    Handle h;
+    if (form == 2) {
+      S2G_CUBLAS(cublasCreate(&h.b));
+      x.g.lib = h.b;
+    }
     DBuf<int> db, dc;
     S2G_CUDA(cudaMemcpyAsync(db.ensure(ncol), bcol, sizeof(int) * ncol, cudaMemcpyHostToDevice, x.s));
     S2G_CUDA(cudaMemcpyAsync(dc.ensure(ncol), ccol, sizeof(int) * ncol, cudaMemcpyHostToDevice, x.s));
@@ -106,6 +111,7 @@ extern "C" int dg_grouped(int ta, int tb, int np, const int *M, const int *N, co
       }
     }
     x.g.grouped(x.s, ta != 0, tb != 0, pr);
+    if (form == 2 && x.g.launches != 0) throw Error{STD2G_ESTATE, "own kernel"};
     x.get(C, nc);
   });
 }

@@ -105,9 +105,10 @@ def test_two_level_columns(lib, tb, form, m, k, len_, groups, batch, beta):
     assert _close(out, ref, mag, k)
 
 
+@pytest.mark.parametrize("form", [0, 2])
 @pytest.mark.parametrize("M,N,K", [([7, 70], [3, 33], [5, 20]), ([64] * 9, [1, 2, 31, 32, 33, 63, 64, 65, 7], [141] * 9),
                                    ([588] * 45, [64] * 45, [48] * 45)])
-def test_grouped_indexed_columns(lib, M, N, K):
+def test_grouped_indexed_columns(lib, form, M, N, K):
     """Each member adds to the columns that its list names; one launch, 32- and
     64-wide tiles."""
     rng = np.random.default_rng(len(M))
@@ -126,7 +127,7 @@ def test_grouped_indexed_columns(lib, M, N, K):
     p = lambda v, t: v.ctypes.data_as(ct.POINTER(t))  # noqa: E731
     Mi, Ni, Ki = i32(M), i32(N), i32(K)
     out, L, D = C.copy(), ct.c_int64, ct.c_double
-    code = lib.dg_grouped(1, 0, np_, p(Mi, ct.c_int), p(Ni, ct.c_int), p(Ki, ct.c_int), D(-1.0), D(1.0), _d(A),
+    code = lib.dg_grouped(form, 1, 0, np_, p(Mi, ct.c_int), p(Ni, ct.c_int), p(Ki, ct.c_int), D(-1.0), D(1.0), _d(A),
                           L(A.size), p(A0, L), L(kmax), _d(B), L(B.size), p(zero, L), L(kmax), _d(out),
                           L(C.size), p(zero, L), L(ld), p(bcol, ct.c_int), p(ccol, ct.c_int), ncol, p(col0, L))
     assert code == 0
