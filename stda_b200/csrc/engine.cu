@@ -73,10 +73,11 @@ struct Ctx {
   // work buffers
   DBuf<double> w_Cact, w_Clow, w_T, w_mu_ov, w_gj, w_gk, w_Qii, w_Qaa, w_Pii, w_uci;
   DBuf<double> w_Qia, w_Pia, w_Qoo, w_Poo, w_Qvv, w_de, w_ek;
-  DBuf<int> w_flag, w_act_idx, w_pk, w_ck, w_tmpi, w_pj, w_pgroup, w_gstart, w_gsize, w_bcol, w_ccol, w_ci,
-      w_ca, w_allk, w_status;
-  DBuf<double> w_ed, w_edsorted, w_Qp, w_rowpart, w_coup, w_pert, w_colpart,
-      w_pt2, w_edp;
+  // PT selection: primaries' occupied indices and groups (one per virtual index), the
+  // groups' first primaries and sizes, columns of the (ij|ab) products
+  DBuf<int> w_flag, w_act_idx, w_pk, w_ck, w_tmpi, w_pj, w_pgroup, w_gstart, w_gsize, w_bcol,
+      w_ccol, w_ci, w_ca, w_allk, w_status;
+  DBuf<double> w_ed, w_edsorted, w_Qp, w_rowpart, w_coup, w_pert, w_colpart, w_pt2, w_edp;
   DBuf<unsigned char> w_sel;
   DBuf<double> w_Qs, w_Ps, w_K, w_J, w_Kx, w_A, w_Apb, w_Amb, w_Bh, w_Ambh, w_M, w_eval, w_X,
       w_Y, w_tmp, w_musel, w_TL, w_TVM, w_T2, w_props, w_work;
@@ -146,11 +147,15 @@ static int dense_eig(Ctx &c, double *A, int n, double vl, double vu, int kmax, d
 // The same for a matrix of at most kSymEigMaxN CSFs on the engine's own
 // eigensolver (symeig_small.cuh), A intact afterwards: all eigenvalues, read back to
 // count the window, then all eigenvectors, and one refinement of the window's in that
-// basis (k_eig_refine): inverse iteration leaves them orthogonal to 1e-15 / gap only,
-// refined they are as exact as or more exact than syevdx's.  What the refinement finds also checks the
-// basis: a residual above 1e-12 ||A|| or an overlap above 1e-8 sends the matrix to
-// cuSOLVER, as do clusters of more than kCluster close eigenvalues, which one warp would
-// work off one after the other.
+// basis (k_eig_refine): inverse iteration leaves them orthogonal to 1e-15 / gap only;
+// refined they are orthonormal to 1e-15, and strengths of 30 benzene windows 0.7 to 1.0
+// as far off as with syevdx.  What the refinement finds also checks the basis: a
+// residual above 1e-12 ||A|| or an overlap above 1e-8 sends the matrix to cuSOLVER, as do
+// clusters of more than kCluster close eigenvalues, which one warp would work off one
+// after the other.  syevdx reduces such a matrix in 1.0 ms and synchronises with the
+// host several times: load and solve of benzene (212 CSFs) 1.31 ms here, of 10 roots of
+// a 12-atom sTD-DFT problem (276 CSFs) 2.35, of 8 roots of 283 UKS CSFs 1.53 ms; with
+// syevdx, and before the other changes of these paths, 3.23, 6.93 and 4.08 ms.
 // The vectors go to `out` (n x k), the window's roots to w.
 static int dense_window_small(Ctx &c, const double *A, int n, double vl, double vu, int kmax,
                               double *w, DBuf<double> &out, double *&X) {
@@ -348,8 +353,8 @@ static void sqrt_overlap_plain(Ctx &c, const double *S, int n, double *out) {
 // over lambda_min around 5000) the Loewdin MOs of S are orthonormal to about 1e-9, as
 // far as the plain form goes with its 1e-10 (it gives up from 500 to 1000).  One host
 // read after kFirst steps.
-// Measured against the plain form: n = 220 0.83 -> 0.30 ms, 518 1.83 -> 0.76, 1584
-// 13.9 -> 5.1 ms, roots of 14 to 34 atoms 2 times closer to the dense FP64 ones.
+// Measured against the plain form: n = 220 0.81 -> 0.31 ms, 517 1.80 -> 0.79, 1584
+// 13.8 -> 5.3 ms, roots of 14 to 34 atoms 2 times closer to the dense FP64 ones.
 static void sqrt_overlap(Ctx &c, const double *S, int n, double *out) {
   cudaStream_t s = c.stream;
   const size_t nn = (size_t)n * n;
@@ -444,10 +449,11 @@ static void sqrt_overlap_fixed(Ctx &c, const double *S, int n, double *out) {
 
 // (A-B)^1/2 of a dense sTD-DFT matrix of at most kSymEigMaxN CSFs by the same iteration
 // as S^1/2, instead of all eigenpairs through syevd: with the roots on the engine's
-// eigensolver too, 10 roots of a 12-atom cluster 6.27 -> 2.13 ms per load and solve.  False, with `out` undefined, when the iteration does not converge or Y Y
-// misses A by more than rounding (64 eps of the largest element; this form leaves 4 to 27
-// eps for n = 30 to 320, an eigen-decomposition 8 to 20): near-singular and indefinite
-// matrices, which the caller's eigen-decomposition decides.
+// eigensolver too, 10 roots of a 12-atom cluster 6.9 -> 2.35 ms per load and solve.
+// False, with `out` undefined, when the iteration does not converge or Y Y misses A by
+// more than rounding (64 eps of the largest element; this form leaves 4 to 27 eps for
+// n = 30 to 320, an eigen-decomposition 8 to 20): near-singular and indefinite matrices,
+// which the caller's eigen-decomposition decides.
 // R: n x n scratch.
 static bool sqrt_small(Ctx &c, const double *A, int n, double *out, double *R) {
   cudaStream_t s = c.stream;

@@ -101,7 +101,7 @@ __global__ void k_ns_scaled_step(double *__restrict__ QT, int n, double mu,
 // matrix here is a polynomial of A, so symmetric), each warp holding its tiles
 // in registers until all warps have read the operands.  out = sqrt(c) Y with the last
 // Y = Y T; stat = {last max |I - Z Y|, max |Y Y - A|, steps}.  Latency-bound: 36 AOs
-// 0.42 -> 0.07 ms, 72 AOs 0.42 -> 0.11 ms against a launch per product and a host read
+// 0.41 -> 0.07 ms, 72 AOs 0.41 -> 0.12 ms against a launch per product and a host read
 // every third step.
 constexpr int kNsSmallMax = 96, kNsThreads = 512;
 __host__ __device__ inline int ns_small_ld(int n) {

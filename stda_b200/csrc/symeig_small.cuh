@@ -1,6 +1,6 @@
-// Lowest k eigenpairs of a small dense symmetric matrix (n <= kSymEigMaxN),
-// for the Rayleigh-Ritz step of the Davidson solver, in four kernels with no
-// host synchronisation:
+// Lowest k eigenpairs of a small dense symmetric matrix (n <= kSymEigMaxN), for the
+// Rayleigh-Ritz step of the Davidson solver and for dense windows, in four kernels
+// with no host synchronisation:
 //   1. k_symeig_tridiag: Householder reduction to tridiagonal form
 //      T = Q^T A Q (LAPACK dsytd2, lower, restated) by one CTA or a cluster of
 //      4 or 8, the matrix in registers (the scheme is described at the
@@ -17,9 +17,10 @@
 //      component by ~1/eps); the cluster threshold is
 //      1e-5 ||T||, tighter than dstein's 1e-3, so that the dense Rayleigh-Ritz
 //      spectra do not collapse into one serial cluster), vectors in T's basis;
-//   4. k_symeig_backtransform (one warp per eigenvector, held in registers):
-//      z = Q y with the reflectors staged through shared memory in blocks
-//      that all warps of the CTA apply.
+//   4. k_symeig_backtransform (one CTA of 128 threads per eigenvector, held in
+//      registers): z = Q y, the reflectors applied 8 at a time through the
+//      triangular factors that phase 2 forms beside the eigenvalues.
+// The vectors are orthogonal to 1e-15 ||A|| / gap (dense windows refine them).
 // cuSOLVER's syevd takes 1-3 ms at n = 75-300, most of it launch and host
 // synchronisation latency.
 // Eigenvalues ascending in w[0..k), eigenvectors in the columns of Z (ld ldz).
@@ -39,7 +40,7 @@
 namespace std2g {
 
 constexpr int kTridiagThreads = 256;
-constexpr int kSymEigMaxN = 320;       // 3 columns per warp in a cluster of 8 CTAs
+constexpr int kSymEigMaxN = 320;       // 5 columns per warp in a cluster of 8 CTAs
 
 constexpr int kBtBlock = 8;   // reflectors applied together by the back-transformation
 __host__ __device__ inline int symeig_bt_blocks(int n) {

@@ -4,7 +4,10 @@
 //   D[m, n] (FP32, row-major, ldd) = sum_k A[m, k] * B[n, k]
 //
 // A and B are given as BF16 pairs (hi, lo) with x ~= hi + lo, stored K-major
-// (row-major with K contiguous, K padded to a multiple of 64 with zeros).
+// (row-major with K contiguous).  run(): rows of any pitch that is a multiple of 8; what
+// lies behind the K elements is never read (the tensor maps end at K and fill in zeros),
+// so K is the true length and not a padded one.  run_direct(): K padded to a multiple
+// of 64 with zeros.
 // Three MMAs per K step (hi*hi + hi*lo + lo*hi) into one FP32 TMEM
 // accumulator recover ~16 mantissa bits of each operand, i.e. products close
 // to FP32 accuracy at BF16 tensor-core rate.
