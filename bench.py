@@ -724,7 +724,8 @@ def main():
             "same_products_cublas_tflops": gst["cublas"]["flop"] / (gst["cublas"]["ms"] / 1e3) / 1e12,
             "same_products_cublas_ms": gst["cublas"]["ms"],
             "note": "each product bracketed by an event pair (std2g_set_gemm_timing); "
-                    "FLOP = 2 m n k per product"}
+                    "FLOP = 2 m n k per product; strided and indexed columns are packed for "
+                    "cuBLAS outside its event pairs"}
 
     if rank == 0 and world == 1 and not args.no_serve:
         # the benchmark solve's context holds tens of GB that the servers'
